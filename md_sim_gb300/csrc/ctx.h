@@ -98,11 +98,12 @@ struct KSet {
     double* ak = nullptr;         // nk
     double2* qw = nullptr;        // nk static wall structure factor
     double2* s = nullptr;         // nk moving-atom structure factor (accumulated)
-    double2* c = nullptr;         // nk: Ak * conj(S_total)
+    double2* c4 = nullptr;        // C(k) = Ak conj(S_total) by pairs (n, -n), 4 per entry (recip.cu)
+    int* ent = nullptr;           // per row: its first entry
     int3* kvec = nullptr;         // nk: (l, m, n)
     int* witem_row = nullptr;     // k_sfac work items: row
-    int* witem_n0 = nullptr;      //                    n offset inside the row
-    int nwork = 0, tile = 0, splits = 1, atoms_per_split = 0, sfac_smem = 0, force_smem = 0;
+    int* witem_n = nullptr;       //                    first entry | entries << 16
+    int nwork = 0;
     std::vector<int4> h_row;      // host copies of row and row_nlen
     std::vector<int> h_nlen;
 };
@@ -321,7 +322,6 @@ int recip_forces_noalloc(const double* x, const double* y, const double* z, cons
                          double lx, double ly, double lz, double alpha, int64_t kmax, double* fx, double* fy,
                          double* fz, double* uewa, cudaStream_t st);
 const char* recip_noalloc_error();
-void recip_energy_launch(Ctx& c);
 // recip_tc.cu
 int recip_tc_setup(Ctx& c);
 int tc_plan_pass1(Ctx& c, int tpc, int mult);

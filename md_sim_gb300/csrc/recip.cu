@@ -6,13 +6,27 @@
 // in single precision (src/forcem.f90:756-759).  For a fixed (l, m) the kept n form the
 // contiguous range -nmax..nmax (1..nmax when l = m = 0), so the list is a sequence of rows.
 //
-//   k_sfac       S(k) = sum_j q_j e^{i k.r_j} over moving atoms.  Work item = (row, chunk of 8 n);
-//                phase factors el/em/en of a tile of atoms are built in shared memory by the
-//                same recurrences as the reference (el(l) = el(l-1)*el(1), negative powers by
-//                conjugation); partial sums over atom splits meet in FP64 atomics.
-//   k_kenergy    uewa, ewqLL and C(k) = Ak conj(S(k) + Sw(k)) (Sw: static walls)
-//   k_kforce     f_j += sum_k Ak Im(conj(S) q_j e^{ik.r_j}) k; one thread per atom walks the rows
-//                with its own phase tables in shared memory and reads C(k) as warp broadcasts.
+// The n range of a row is symmetric, so both directions work on the pairs (n, -n), n >= 0 ("entries"
+// of a row, 0..nmax), and the number of FP64 operations, which is what bounds them (an FP64 FMA
+// retires 1.6 lanes per clock per SM on this part), is that of the real sums of a pair:
+//
+//   k_sfac       S(k) = sum_j q_j e^{i k.r_j} over moving atoms.  With a = q e^{i(l tx + m ty)} and
+//                e^{i n tz} = c + i s the four real sums of a.re c, a.im s, a.re s, a.im c give both
+//                S(n) and S(-n): 4 FMAs per (atom, entry), 2 per (atom, k), where a complex product
+//                and sum per (atom, k) takes 6.  Work item = (row, up to kChunk entries), items
+//                sorted by length; phase factors of a tile of atoms are built in shared memory by
+//                the same recurrences as the reference (el(l) = el(l-1)*el(1)); partial sums over
+//                atom splits meet in FP64 atomics.
+//   k_kenergy    uewa, ewqLL and C(k) = Ak conj(S(k) + Sw(k)) (Sw: static walls), stored per entry as
+//                P = C(n) + C(-n), M = C(n) - C(-n) and both times n
+//   k_kforce     f_j += sum_k Ak Im(conj(S) q_j e^{ik.r_j}) k; one thread per atom with its phase
+//                tables in shared memory: per entry T += P c + i M s and T' += nM c + i nP s, 8 FMAs
+//                (4 per k), then Im(a T), Im(a T') once per row; P and M are warp broadcasts.  The
+//                rows are dealt to as many grid rows as give every SM work when atoms are few.
+// 2,048-water slab (6,144 atoms, 4,338 k): k_sfac 586 -> 204 us, k_kforce 1,778 -> 290 us against the
+// form with complex products, items of 8 n, 256-thread blocks and one thread per atom over all rows;
+// a force call at 32,768 waters (29,038 k) 115.7 -> 48.6 ms, of which k_kforce 27 ms, its FMAs at
+// the 0.5 TFMA/s that a loop of independent FP64 FMAs reaches on this part.
 #include <algorithm>
 #include <cmath>
 #include <complex>
@@ -27,9 +41,16 @@ namespace mdg {
 
 namespace {
 
-constexpr int kChunk = 8;     // n per work item in k_sfac
-constexpr int kSfacNT = 256;
-constexpr int kForceNT = 128;
+constexpr int kChunk = 13;    // most entries per work item in k_sfac (4 sums each, in registers)
+constexpr int kSfacNT = 128;
+constexpr int kForceNT = 64;
+constexpr int kSfacTile = 32;   // atoms per phase table of k_sfac
+constexpr int kMaxSplit = 64;   // most grid rows of k_kforce
+
+// Entries of a row: n = 0..nmax, whose (n, -n) are the row's k vectors ((0, 0, n > 0) for the first).
+__host__ __device__ __forceinline__ int row_entries(int n_first, int nlen) {
+    return (n_first > 0 ? n_first + nlen - 1 : -n_first) + 1;
+}
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
     return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
@@ -41,91 +62,79 @@ struct KDims {
     double px, py, pz;     // 2 pi / L
 };
 
-// Phase tables of one atom: el[0..KL], em[0..KM], en[0..KN] by recurrence.
-__device__ void phase_tables(double x, double y, double z, const KDims& d, double2* el, double2* em,
-                             double2* en, int which) {
+// Phase table of one atom and direction, e^{i k a} for k = 0..K at t[k * stride], by recurrence.
+__device__ void phase_table(double a, int K, double2* t, int stride) {
     double s, c;
-    if (which == 0) {
-        sincos(d.px * x, &s, &c);
-        const double2 e1 = make_double2(c, s);
-        el[0] = make_double2(1.0, 0.0);
-        if (d.KL >= 1) el[1] = e1;
-        for (int l = 2; l <= d.KL; ++l) el[l] = cmul(el[l - 1], e1);
-    } else if (which == 1) {
-        sincos(d.py * y, &s, &c);
-        const double2 e1 = make_double2(c, s);
-        em[0] = make_double2(1.0, 0.0);
-        if (d.KM >= 1) em[1] = e1;
-        for (int m = 2; m <= d.KM; ++m) em[m] = cmul(em[m - 1], e1);
-    } else {
-        sincos(d.pz * z, &s, &c);
-        const double2 e1 = make_double2(c, s);
-        en[0] = make_double2(1.0, 0.0);
-        if (d.KN >= 1) en[1] = e1;
-        for (int n = 2; n <= d.KN; ++n) en[n] = cmul(en[n - 1], e1);
+    sincos(a, &s, &c);
+    const double2 e1 = make_double2(c, s);
+    double2 e = make_double2(1.0, 0.0);
+    t[0] = e;
+    for (int k = 1; k <= K; ++k) {
+        e = k == 1 ? e1 : cmul(e, e1);
+        t[(size_t)k * stride] = e;
     }
 }
 
-__device__ __forceinline__ double2 pw(const double2* t, int k) { return k >= 0 ? t[k] : conjd(t[-k]); }
-#ifdef MDG_DEBUG_BOUNDS
-#define PW(t, k, lim, tag) pw((t), ((k) > (lim) || (k) < -(lim)) ? (atomicCAS(&v.status[ST_OOB], 0, (tag)), 0) : (k))
-#else
-#define PW(t, k, lim, tag) pw((t), (k))
-#endif
-
-// rows: (l, m, n_first, k_first); nlen: kept n in the row (n = n_first .. n_first + nlen - 1)
-__global__ void __launch_bounds__(kSfacNT) k_sfac(View v, KDims d, int nrow, const int4* rows,
-                                                  const int* nlen, const int* witem_row,
-                                                  const int* witem_n0, int nwork, int tile,
-                                                  int atoms_per_split, double2* S, int nk_total) {
+// rows: (l, m, n_first, k_first); witem_n: first entry | entries << 16 of each work item
+__global__ void __launch_bounds__(kSfacNT) k_sfac(View v, KDims d, int nrow, const int4* __restrict__ rows,
+                                                  const int* __restrict__ witem_row, const int* __restrict__ witem_n,
+                                                  int nwork, int atoms_per_split, double2* S, int nk_total) {
     extern __shared__ double2 sm[];
+    // per atom: q e^{i l tx} (l = 0..KL), e^{i m ty} (m = 0..KM), e^{i n tz} (n = 0..KN)
     const int per = d.KL + 1 + d.KM + 1 + d.KN + 1;
-    double2* tab = sm;                                  // tile * per
-    double* qt = reinterpret_cast<double*>(sm + (size_t)tile * per);  // tile
     const int w = blockIdx.x * blockDim.x + threadIdx.x;
-    int l = 0, m = 0, n0 = 0, nn = 0, k0 = 0;
+    int l = 0, m = 0, n0 = 0, nn = 0, kc = 0;  // kc: the k index of n = 0 (of n, if that row had it)
+    bool half = false;                         // the row of l = m = 0 has no n <= 0
     if (w < nwork) {
-        const int r = CK(witem_row[w], nrow, 201);
-        const int4 rw = rows[r];
+        const int4 rw = rows[CK(witem_row[w], nrow, 201)];
         l = rw.x;
         m = rw.y;
-        const int off = witem_n0[w];
-        n0 = rw.z + off;
-        k0 = rw.w + off;
-        nn = min(kChunk, nlen[r] - off);
+        n0 = witem_n[w] & 0xffff;
+        nn = witem_n[w] >> 16;
+        kc = rw.w - rw.z;
+        half = rw.z > 0;
     }
-    double2 acc[kChunk];
+    const int nw = __reduce_max_sync(0xffffffffu, nn);  // items are sorted: a warp's lengths are alike
+    const int ma = abs(m);
+    const double sgm = m < 0 ? -1.0 : 1.0;
+    double x1[kChunk], x2[kChunk], x3[kChunk], x4[kChunk];
 #pragma unroll
-    for (int c = 0; c < kChunk; ++c) acc[c] = make_double2(0.0, 0.0);
+    for (int c = 0; c < kChunk; ++c) x1[c] = x2[c] = x3[c] = x4[c] = 0.0;
     const int a_begin = blockIdx.y * atoms_per_split;
     const int a_end = min(v.nmove, a_begin + atoms_per_split);
-    for (int t0 = a_begin; t0 < a_end; t0 += tile) {
-        const int nt = min(tile, a_end - t0);
+    for (int t0 = a_begin; t0 < a_end; t0 += kSfacTile) {
+        const int nt = min(kSfacTile, a_end - t0);
         __syncthreads();
         for (int s = threadIdx.x; s < nt * 3; s += blockDim.x) {
             const int a = s % nt, which = s / nt;
             const int at = CK(t0 + a, v.nmove, 202);
-            double2* base = tab + (size_t)CK(a, tile, 203) * per;
-            phase_tables(v.x[at], v.y[at], v.z[at], d, base, base + d.KL + 1, base + d.KL + 1 + d.KM + 1, which);
-            if (which == 0) qt[a] = v.q[at];
+            double2* base = sm + (size_t)CK(a, kSfacTile, 203) * per;
+            if (which == 0) {
+                phase_table(d.px * v.x[at], d.KL, base, 1);
+                const double q = v.q[at];
+                for (int k = 0; k <= d.KL; ++k) base[k] = make_double2(q * base[k].x, q * base[k].y);
+            } else if (which == 1) {
+                phase_table(d.py * v.y[at], d.KM, base + d.KL + 1, 1);
+            } else {
+                phase_table(d.pz * v.z[at], d.KN, base + d.KL + 1 + d.KM + 1, 1);
+            }
         }
         __syncthreads();
-        if (nn > 0) {
-            for (int a = 0; a < nt; ++a) {
-                const double2* base = tab + (size_t)a * per;
-                const double2 el = base[CK(l, d.KL + 1, 204)];
-                const double2 em = PW(base + d.KL + 1, m, d.KM, 209);
-                const double2* en = base + d.KL + 1 + d.KM + 1;
-                // elm = q*el*em (src/forcem.f90:874), elmn = elm*en (:879)
-                const double q = qt[a];
-                const double2 elm = cmul(make_double2(q * el.x, q * el.y), em);
+        for (int a = 0; a < nt; ++a) {
+            const double2* base = sm + (size_t)a * per;
+            const double2 el = base[CK(l, d.KL + 1, 204)];
+            double2 em = base[d.KL + 1 + CK(ma, d.KM + 1, 209)];
+            em.y *= sgm;
+            const double2* en = base + d.KL + 1 + d.KM + 1 + n0;
+            const double2 e = cmul(el, em);
 #pragma unroll
-                for (int c = 0; c < kChunk; ++c) {
-                    if (c < nn) {
-                        const double2 e = cmul(elm, PW(en, n0 + c, d.KN, 210));
-                        acc[c].x += e.x;
-                        acc[c].y += e.y;
-                    }
+            for (int c = 0; c < kChunk; ++c) {
+                if (c < nw) {
+                    const double2 p = en[c < nn ? c : 0];
+                    x1[c] = fma(e.x, p.x, x1[c]);
+                    x2[c] = fma(e.y, p.y, x2[c]);
+                    x3[c] = fma(e.x, p.y, x3[c]);
+                    x4[c] = fma(e.y, p.x, x4[c]);
                 }
             }
         }
@@ -133,72 +142,163 @@ __global__ void __launch_bounds__(kSfacNT) k_sfac(View v, KDims d, int nrow, con
 #pragma unroll
     for (int c = 0; c < kChunk; ++c) {
         if (c < nn) {
-            atomicAdd(&S[CK(k0 + c, nk_total, 205)].x, acc[c].x);
-            atomicAdd(&S[CK(k0 + c, nk_total, 205)].y, acc[c].y);
+            const int n = n0 + c;
+            if (n > 0) {
+                atomicAdd(&S[CK(kc + n, nk_total, 205)].x, x1[c] - x2[c]);
+                atomicAdd(&S[CK(kc + n, nk_total, 205)].y, x3[c] + x4[c]);
+            }
+            if (!half) {
+                atomicAdd(&S[CK(kc - n, nk_total, 205)].x, n > 0 ? x1[c] + x2[c] : x1[c]);
+                atomicAdd(&S[CK(kc - n, nk_total, 205)].y, n > 0 ? x4[c] - x3[c] : x4[c]);
+            }
         }
     }
 }
 
-__global__ void k_kenergy(View v, int nk, const double* ak, const double2* S, const double2* qw, double2* C) {
+// One warp per row: energies, and the row's entries of the pair table C4 (two double4 per entry:
+// P.re, P.im, M.re, M.im and the same times n).  qw may be null (no static walls).
+__global__ void k_kenergy(View v, int nrow, const int4* __restrict__ rows, const int* __restrict__ nlen,
+                          const int* __restrict__ ent, const double* __restrict__ ak, const double2* __restrict__ S,
+                          const double2* __restrict__ qw, double2* __restrict__ C4) {
     double ew = 0.0, ll = 0.0;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nk; k += gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    auto coef = [&](int k) {
         const double2 s = S[k];
-        const double2 st = make_double2(s.x + qw[k].x, s.y + qw[k].y);
+        const double2 q = qw ? qw[k] : make_double2(0.0, 0.0);
+        const double2 st = make_double2(s.x + q.x, s.y + q.y);
         const double a = ak[k];
         ll += a * (s.x * s.x + s.y * s.y);
         ew += a * (st.x * st.x + st.y * st.y);
-        C[k] = make_double2(a * st.x, -a * st.y);
+        return make_double2(a * st.x, -a * st.y);
+    };
+    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrow; r += (gridDim.x * blockDim.x) >> 5) {
+        const int4 rw = rows[r];
+        const int ne = row_entries(rw.z, nlen[r]), kc = rw.w - rw.z;
+        for (int n = lane; n < ne; n += 32) {
+            double2 cp = make_double2(0.0, 0.0), cm = cp;
+            if (n > 0 || rw.z <= 0) cp = coef(kc + n);
+            if (n > 0 && rw.z <= 0) cm = coef(kc - n);
+            const double2 P = make_double2(cp.x + cm.x, cp.y + cm.y);
+            const double2 M = n > 0 ? make_double2(cp.x - cm.x, cp.y - cm.y) : make_double2(0.0, 0.0);
+            double2* o = C4 + 4 * (size_t)(ent[r] + n);
+            o[0] = P;
+            o[1] = M;
+            o[2] = make_double2((double)n * P.x, (double)n * P.y);
+            o[3] = make_double2((double)n * M.x, (double)n * M.y);
+        }
     }
     block_atomic_sum<256>(ew, &v.acc[2 * v.nijt + ACC_UEWA]);
     block_atomic_sum<256>(ll, &v.acc[2 * v.nijt + ACC_EWQLL]);
 }
 
-__global__ void __launch_bounds__(kForceNT) k_kforce(View v, KDims d, int nrow, const int4* rows,
-                                                     const int* nlen, const double2* C, int nk_total) {
+__global__ void __launch_bounds__(kForceNT) k_kforce(View v, KDims d, int nrow, const int4* __restrict__ rows,
+                                                     const int* __restrict__ nlen, const int* __restrict__ ent,
+                                                     const double2* __restrict__ C4) {
     extern __shared__ double2 sm[];
-    const int per = d.KM + 1 + d.KN + 1;
-    double2* em = sm + (size_t)CK(threadIdx.x, blockDim.x, 206) * per;
-    double2* en = em + d.KM + 1;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    // this thread's e^{i m ty} and e^{i n tz}, kForceNT apart (no bank conflicts)
+    double2* em = sm + threadIdx.x;
+    double2* en = em + (size_t)(d.KM + 1) * kForceNT;
+    const int j = blockIdx.x * kForceNT + threadIdx.x;
     const bool active = j < v.nmove;
     const int jj = active ? j : 0;
-    phase_tables(0, v.y[jj], 0, d, nullptr, em, nullptr, 1);
-    phase_tables(0, 0, v.z[jj], d, nullptr, nullptr, en, 2);
+    phase_table(d.py * v.y[jj], d.KM, em, kForceNT);
+    phase_table(d.pz * v.z[jj], d.KN, en, kForceNT);
     double s, c;
     sincos(d.px * v.x[jj], &s, &c);
     const double2 el1 = make_double2(c, s);
-    double2 el = make_double2(1.0, 0.0);
-    int lcur = 0;
     const double q = v.q[jj];
+    double2 el = make_double2(q, 0.0);
+    int lcur = 0;
     double fx = 0.0, fy = 0.0, fz = 0.0;
-    for (int r = 0; r < nrow; ++r) {
+    for (int r = blockIdx.y; r < nrow; r += gridDim.y) {
         const int4 rw = rows[r];
         while (lcur < rw.x) {
             el = cmul(el, el1);
             ++lcur;
         }
-        const double2 emm = PW(em, rw.y, d.KM, 211);
-        const double2 elm = cmul(make_double2(q * el.x, q * el.y), emm);
-        const int n0 = rw.z, cnt = nlen[r];
-        const double2* Ck = C + CK(rw.w, nk_total, 207);
-        double st = 0.0, stn = 0.0;
-        for (int t = 0; t < cnt; ++t) {
-            const int n = n0 + t;
-            const double2 e = cmul(elm, PW(en, n, d.KN, 212));
-            const double2 ck = Ck[CK(t, nk_total - rw.w, 208)];
-            const double f = ck.x * e.y + ck.y * e.x;  // Im(C * e), C = Ak conj(S)
-            st += f;
-            stn += f * (double)n;
+        double2 emm = em[(size_t)CK(abs(rw.y), d.KM + 1, 211) * kForceNT];
+        if (rw.y < 0) emm.y = -emm.y;
+        const double2 elm = cmul(el, emm);
+        const int ne = row_entries(rw.z, nlen[r]);
+        const double2* Ck = C4 + 4 * (size_t)ent[r];
+        // each sum in two chains, so that consecutive FMAs do not wait for one another
+        const double2 P0 = __ldg(Ck);  // n = 0: e = 1, M = 0
+        double tr0 = P0.x, tr1 = 0.0, ti0 = P0.y, ti1 = 0.0, ur0 = 0.0, ur1 = 0.0, ui0 = 0.0, ui1 = 0.0;
+#pragma unroll 2
+        for (int n = 1; n < ne; ++n) {
+            const double2 e = en[(size_t)CK(n, d.KN + 1, 212) * kForceNT];
+            const double2 P = __ldg(Ck + 4 * n), M = __ldg(Ck + 4 * n + 1), nP = __ldg(Ck + 4 * n + 2),
+                          nM = __ldg(Ck + 4 * n + 3);
+            tr0 = fma(P.x, e.x, tr0);
+            tr1 = fma(M.y, e.y, tr1);
+            ti0 = fma(P.y, e.x, ti0);
+            ti1 = fma(M.x, e.y, ti1);
+            ur0 = fma(nM.x, e.x, ur0);
+            ur1 = fma(nP.y, e.y, ur1);
+            ui0 = fma(nM.y, e.x, ui0);
+            ui1 = fma(nP.x, e.y, ui1);
         }
-        fx += st * (d.px * (double)rw.x);
-        fy += st * (d.py * (double)rw.y);
-        fz += stn * d.pz;
+        const double st = elm.x * (ti0 + ti1) + elm.y * (tr0 - tr1);
+        const double stn = elm.x * (ui0 + ui1) + elm.y * (ur0 - ur1);
+        fx += st * (double)rw.x;
+        fy += st * (double)rw.y;
+        fz += stn;
     }
-    if (active) {
+    if (!active) return;
+    fx *= d.px;
+    fy *= d.py;
+    fz *= d.pz;
+    if (gridDim.y > 1) {
+        atomicAdd(&v.fx[j], fx);
+        atomicAdd(&v.fy[j], fy);
+        atomicAdd(&v.fz[j], fz);
+    } else {
         v.fx[j] += fx;
         v.fy[j] += fy;
         v.fz[j] += fz;
     }
+}
+
+// Work items of k_sfac for the rows (n_first, nlen): (row, first entry | entries << 16), each row cut
+// into equal items of at most kChunk entries, sorted by length so that the lanes of a warp run alike.
+// Returns the number of entries of all rows; ent[r] is row r's first.
+int sfac_items(const int4* rows, const int* nlen, int nrow, int* ent, int* wr, int* wn, int& nwork) {
+    int ne = 0;
+    nwork = 0;
+    for (int r = 0; r < nrow; ++r) {
+        ent[r] = ne;
+        ne += row_entries(rows[r].z, nlen[r]);
+    }
+    for (int len = kChunk; len >= 1; --len)
+        for (int r = 0; r < nrow; ++r) {
+            const int e = row_entries(rows[r].z, nlen[r]), parts = (e + kChunk - 1) / kChunk;
+            for (int p = 0; p < parts; ++p) {
+                const int a = e * p / parts, b = e * (p + 1) / parts;
+                if (b - a != len) continue;
+                wr[nwork] = r;
+                wn[nwork++] = a | len << 16;
+            }
+        }
+    return ne;
+}
+
+// Launch shapes: atom splits of k_sfac and grid rows of k_kforce that give every SM a few blocks
+// (both kernels keep the FP64 pipe busy with four warps per SM), at least 4 atoms and 4 rows each.
+struct KGrid {
+    dim3 sfac, force;
+    int atoms_per_split, smem_sfac, smem_force;
+};
+KGrid k_grid(const KDims& d, int natom, int nrow, int nwork) {
+    KGrid g;
+    const int kb = std::max(1, (nwork + kSfacNT - 1) / kSfacNT), fb = std::max(1, (natom + kForceNT - 1) / kForceNT);
+    int splits = std::max(1, std::min((152 * 16 + kb - 1) / kb, (natom + 3) / 4));
+    g.atoms_per_split = (natom + splits - 1) / splits;
+    splits = (natom + g.atoms_per_split - 1) / g.atoms_per_split;
+    g.sfac = dim3(kb, splits);
+    g.force = dim3(fb, std::max(1, std::min({(152 * 16 + fb - 1) / fb, kMaxSplit, nrow / 4})));
+    g.smem_sfac = kSfacTile * (d.KL + 1 + d.KM + 1 + d.KN + 1) * (int)sizeof(double2);
+    g.smem_force = kForceNT * (d.KM + 1 + d.KN + 1) * (int)sizeof(double2);
+    return g;
 }
 
 }  // namespace
@@ -290,55 +390,39 @@ int recip_setup(Ctx& c, int64_t kmax, const double* x0, const double* y0, const 
         c.ewqWW += (ak[k] * s * std::conj(s)).real();
     }
     c.ewqWW *= 0.5;
-    // work items of k_sfac: (row, n offset) in chunks of kChunk
-    std::vector<int> wr, wn;
-    for (int r = 0; r < ks.nrow; ++r)
-        for (int off = 0; off < nlen[r]; off += kChunk) {
-            wr.push_back(r);
-            wn.push_back(off);
-        }
-    ks.nwork = (int)wr.size();
+    std::vector<int> ent(std::max(ks.nrow, 1)), wr(ks.nk + 1), wn(ks.nk + 1);
+    const int nent = sfac_items(rows.data(), nlen.data(), ks.nrow, ent.data(), wr.data(), wn.data(), ks.nwork);
     const int nk1 = std::max(ks.nk, 1), nr1 = std::max(ks.nrow, 1), nw1 = std::max(ks.nwork, 1);
     ks.row = (int4*)dalloc(c, sizeof(int4) * nr1);
     ks.row_nlen = (int*)dalloc(c, sizeof(int) * nr1);
     ks.ak = (double*)dalloc(c, sizeof(double) * nk1);
     ks.qw = (double2*)dalloc(c, sizeof(double2) * nk1);
     ks.s = (double2*)dalloc(c, sizeof(double2) * nk1);
-    ks.c = (double2*)dalloc(c, sizeof(double2) * nk1);
+    ks.c4 = (double2*)dalloc(c, 4 * sizeof(double2) * std::max(nent, 1));
+    ks.ent = (int*)dalloc(c, sizeof(int) * nr1);
     ks.kvec = (int3*)dalloc(c, sizeof(int3) * nk1);
     ks.witem_row = (int*)dalloc(c, sizeof(int) * nw1);
-    ks.witem_n0 = (int*)dalloc(c, sizeof(int) * nw1);
+    ks.witem_n = (int*)dalloc(c, sizeof(int) * nw1);
     ks.h_row = rows;
     ks.h_nlen = nlen;
     if (ks.nk > 0) {
         MDG_CUDA(cudaMemcpy(ks.row, rows.data(), sizeof(int4) * ks.nrow, cudaMemcpyHostToDevice));
         MDG_CUDA(cudaMemcpy(ks.row_nlen, nlen.data(), sizeof(int) * ks.nrow, cudaMemcpyHostToDevice));
+        MDG_CUDA(cudaMemcpy(ks.ent, ent.data(), sizeof(int) * ks.nrow, cudaMemcpyHostToDevice));
         MDG_CUDA(cudaMemcpy(ks.ak, ak.data(), sizeof(double) * ks.nk, cudaMemcpyHostToDevice));
         MDG_CUDA(cudaMemcpy(ks.qw, qw.data(), sizeof(double2) * ks.nk, cudaMemcpyHostToDevice));
         MDG_CUDA(cudaMemcpy(ks.kvec, kvec.data(), sizeof(int3) * ks.nk, cudaMemcpyHostToDevice));
         MDG_CUDA(cudaMemcpy(ks.witem_row, wr.data(), sizeof(int) * ks.nwork, cudaMemcpyHostToDevice));
-        MDG_CUDA(cudaMemcpy(ks.witem_n0, wn.data(), sizeof(int) * ks.nwork, cudaMemcpyHostToDevice));
+        MDG_CUDA(cudaMemcpy(ks.witem_n, wn.data(), sizeof(int) * ks.nwork, cudaMemcpyHostToDevice));
     }
-    // launch geometry of k_sfac: atom tile in shared memory, atom splits to fill the GPU
-    const int per = (KL + 1 + KM + 1 + KN + 1) * (int)sizeof(double2) + (int)sizeof(double);
-    ks.tile = std::max(8, std::min(64, (96 * 1024) / per));
-    const int kblocks = (ks.nwork + kSfacNT - 1) / kSfacNT;
-    int splits = std::max(1, (152 * 4 + kblocks - 1) / std::max(kblocks, 1));
-    splits = std::min(splits, std::max(1, (v.nmove + ks.tile - 1) / ks.tile));
-    ks.atoms_per_split = (v.nmove + splits - 1) / splits;
-    ks.splits = splits;
-    ks.sfac_smem = ks.tile * ((KL + 1 + KM + 1 + KN + 1) * (int)sizeof(double2) + (int)sizeof(double));
-    ks.force_smem = kForceNT * (KM + 1 + KN + 1) * (int)sizeof(double2);
     MDG_CUDA(allow_max_smem(k_sfac));
     MDG_CUDA(allow_max_smem(k_kforce));
-    if (ks.force_smem > 200 * 1024 || ks.sfac_smem > 200 * 1024)
+    // (the limits that earlier tile sizes set: what they refused stays refused)
+    const int per = (KL + 1 + KM + 1 + KN + 1) * (int)sizeof(double2) + (int)sizeof(double);
+    if (128 * (KM + 1 + KN + 1) * (int)sizeof(double2) > 200 * 1024 ||
+        std::max(8, std::min(64, (96 * 1024) / per)) * per > 200 * 1024)
         return set_err(&c, MDG_E_UNSUPPORTED, "kmax too large for the shared-memory phase tables");
     return MDG_OK;
-}
-
-void recip_energy_launch(Ctx& c) {
-    KSet& ks = c.ks;
-    k_kenergy<<<std::min((ks.nk + 255) / 256, 256), 256, 0, c.stream>>>(c.v, ks.nk, ks.ak, ks.s, ks.qw, ks.c);
 }
 
 void recip_fp64(Ctx& c) {
@@ -346,13 +430,13 @@ void recip_fp64(Ctx& c) {
     KSet& ks = c.ks;
     if (ks.nk == 0 || v.nmove == 0) return;
     KDims d{ks.klmax, ks.kmmax, ks.knmax, ks.pipix, ks.pipiy, ks.pipiz};
+    const KGrid g = k_grid(d, v.nmove, ks.nrow, ks.nwork);
     cudaMemsetAsync(ks.s, 0, sizeof(double2) * ks.nk, c.stream);
-    dim3 g((ks.nwork + kSfacNT - 1) / kSfacNT, ks.splits);
-    k_sfac<<<g, kSfacNT, ks.sfac_smem, c.stream>>>(v, d, ks.nrow, ks.row, ks.row_nlen, ks.witem_row,
-                                                   ks.witem_n0, ks.nwork, ks.tile, ks.atoms_per_split, ks.s, ks.nk);
-    k_kenergy<<<std::min((ks.nk + 255) / 256, 256), 256, 0, c.stream>>>(v, ks.nk, ks.ak, ks.s, ks.qw, ks.c);
-    k_kforce<<<(v.nmove + kForceNT - 1) / kForceNT, kForceNT, ks.force_smem, c.stream>>>(v, d, ks.nrow, ks.row,
-                                                                                        ks.row_nlen, ks.c, ks.nk);
+    k_sfac<<<g.sfac, kSfacNT, g.smem_sfac, c.stream>>>(v, d, ks.nrow, ks.row, ks.witem_row, ks.witem_n, ks.nwork,
+                                                       g.atoms_per_split, ks.s, ks.nk);
+    k_kenergy<<<std::min((ks.nrow + 7) / 8, 256), 256, 0, c.stream>>>(v, ks.nrow, ks.row, ks.row_nlen, ks.ent, ks.ak,
+                                                                     ks.s, ks.qw, ks.c4);
+    k_kforce<<<g.force, kForceNT, g.smem_force, c.stream>>>(v, d, ks.nrow, ks.row, ks.row_nlen, ks.ent, ks.c4);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -370,16 +454,19 @@ namespace {
 
 constexpr int kNaMaxK = MDG_NOALLOC_MAX_K;
 constexpr int kNaMaxRows = MDG_NOALLOC_MAX_ROWS;
+// a row of 2 nmax + 1 k vectors has nmax + 1 entries; the first row, with n > 0 only, at most 100
+// (the phase tables' limit on knmax)
+constexpr int kNaMaxEnt = (kNaMaxK + kNaMaxRows) / 2 + 128;
 constexpr int kNaMaxWork = kNaMaxK / kChunk + kNaMaxRows;
 
 // byte offsets of the regions inside the scratch array
 constexpr size_t kNaS = 0;                                              // double2 [MAX_K]  S(k)
-constexpr size_t kNaC = kNaS + sizeof(double2) * kNaMaxK;               // double2 [MAX_K]  C(k)
-constexpr size_t kNaQw = kNaC + sizeof(double2) * kNaMaxK;              // double2 [MAX_K]  zeros
-constexpr size_t kNaAk = kNaQw + sizeof(double2) * kNaMaxK;             // double  [MAX_K]
+constexpr size_t kNaC = kNaS + sizeof(double2) * kNaMaxK;               // 4 x double2 [MAX_ENT]  C(k) by entry
+constexpr size_t kNaAk = kNaC + 4 * sizeof(double2) * kNaMaxEnt;        // double  [MAX_K]
 constexpr size_t kNaRows = kNaAk + sizeof(double) * kNaMaxK;            // int4    [MAX_ROWS]
 constexpr size_t kNaNlen = kNaRows + sizeof(int4) * kNaMaxRows;         // int     [MAX_ROWS]
-constexpr size_t kNaWr = kNaNlen + sizeof(int) * kNaMaxRows;            // int     [MAX_WORK]
+constexpr size_t kNaEnt = kNaNlen + sizeof(int) * kNaMaxRows;           // int     [MAX_ROWS]
+constexpr size_t kNaWr = kNaEnt + sizeof(int) * kNaMaxRows;             // int     [MAX_WORK]
 constexpr size_t kNaWn = kNaWr + sizeof(int) * kNaMaxWork;              // int     [MAX_WORK]
 constexpr size_t kNaAcc = (kNaWn + sizeof(int) * kNaMaxWork + 255) / 256 * 256;  // double [64]
 constexpr size_t kNaStatus = kNaAcc + sizeof(double) * 64;              // int [ST_NWORDS]
@@ -396,7 +483,7 @@ constexpr int kNaMaxDev = 64;
 unsigned char* g_na_ptr[kNaMaxDev] = {nullptr};
 // host-side k tables, reused by every call (calls are serialised by g_na_mutex)
 int4 g_na_rows[kNaMaxRows];
-int g_na_nlen[kNaMaxRows];
+int g_na_nlen[kNaMaxRows], g_na_ent[kNaMaxRows];
 double g_na_ak[kNaMaxK];
 int g_na_wr[kNaMaxWork], g_na_wn[kNaMaxWork];
 thread_local char g_na_err[256] = "";
@@ -463,12 +550,6 @@ int recip_forces_noalloc(const double* x, const double* y, const double* z, cons
                 if (nrow >= kNaMaxRows) return na_fail(MDG_E_UNSUPPORTED, "mdg_recip_forces_noalloc: too many k rows");
                 g_na_rows[nrow] = make_int4(kl, km, first, nk - cnt);
                 g_na_nlen[nrow] = cnt;
-                for (int off = 0; off < cnt; off += kChunk) {
-                    if (nwork >= kNaMaxWork) return na_fail(MDG_E_UNSUPPORTED, "mdg_recip_forces_noalloc: too many work items");
-                    g_na_wr[nwork] = nrow;
-                    g_na_wn[nwork] = off;
-                    ++nwork;
-                }
                 ++nrow;
             }
             knmin = -KN;
@@ -476,23 +557,23 @@ int recip_forces_noalloc(const double* x, const double* y, const double* z, cons
         kmmin = -KM;
     }
     if (nk == 0) return na_fail(MDG_E_ARG, "mdg_recip_forces_noalloc: empty k set");
-    const int sfac_smem = 64 * ((KL + 1 + KM + 1 + KN + 1) * (int)sizeof(double2) + (int)sizeof(double));
-    const int tile = std::max(8, std::min(64, (96 * 1024) / ((KL + 1 + KM + 1 + KN + 1) * (int)sizeof(double2) + (int)sizeof(double))));
-    const int smem1 = tile * ((KL + 1 + KM + 1 + KN + 1) * (int)sizeof(double2) + (int)sizeof(double));
-    const int smem2 = kForceNT * (KM + 1 + KN + 1) * (int)sizeof(double2);
-    (void)sfac_smem;
+    const int per = (KL + 1 + KM + 1 + KN + 1) * (int)sizeof(double2) + (int)sizeof(double);
+    const int smem1 = std::max(8, std::min(64, (96 * 1024) / per)) * per;
+    const int smem2 = 128 * (KM + 1 + KN + 1) * (int)sizeof(double2);
     if (smem1 > 200 * 1024 || smem2 > 200 * 1024)
         return na_fail(MDG_E_UNSUPPORTED, "mdg_recip_forces_noalloc: kmax too large for the phase tables");
+    if (sfac_items(g_na_rows, g_na_nlen, nrow, g_na_ent, g_na_wr, g_na_wn, nwork) > kNaMaxEnt)
+        return na_fail(MDG_E_UNSUPPORTED, "mdg_recip_forces_noalloc: too many k rows");
     auto ck = [](cudaError_t e) { return e == cudaSuccess; };
     if (!ck(allow_max_smem(k_sfac)) ||
         !ck(allow_max_smem(k_kforce)))
         return na_fail(MDG_E_CUDA, "mdg_recip_forces_noalloc: cudaFuncSetAttribute failed");
     double2* S = reinterpret_cast<double2*>(base + kNaS);
     double2* C = reinterpret_cast<double2*>(base + kNaC);
-    double2* Qw = reinterpret_cast<double2*>(base + kNaQw);
     double* Ak = reinterpret_cast<double*>(base + kNaAk);
     int4* rows = reinterpret_cast<int4*>(base + kNaRows);
     int* nlen = reinterpret_cast<int*>(base + kNaNlen);
+    int* ent = reinterpret_cast<int*>(base + kNaEnt);
     int* wr = reinterpret_cast<int*>(base + kNaWr);
     int* wn = reinterpret_cast<int*>(base + kNaWn);
     double* acc = reinterpret_cast<double*>(base + kNaAcc);
@@ -501,10 +582,10 @@ int recip_forces_noalloc(const double* x, const double* y, const double* z, cons
     bool ok = ck(cudaMemcpyAsync(Ak, g_na_ak, sizeof(double) * nk, cudaMemcpyHostToDevice, st)) &&
               ck(cudaMemcpyAsync(rows, g_na_rows, sizeof(int4) * nrow, cudaMemcpyHostToDevice, st)) &&
               ck(cudaMemcpyAsync(nlen, g_na_nlen, sizeof(int) * nrow, cudaMemcpyHostToDevice, st)) &&
+              ck(cudaMemcpyAsync(ent, g_na_ent, sizeof(int) * nrow, cudaMemcpyHostToDevice, st)) &&
               ck(cudaMemcpyAsync(wr, g_na_wr, sizeof(int) * nwork, cudaMemcpyHostToDevice, st)) &&
               ck(cudaMemcpyAsync(wn, g_na_wn, sizeof(int) * nwork, cudaMemcpyHostToDevice, st)) &&
               ck(cudaMemsetAsync(S, 0, sizeof(double2) * nk, st)) &&
-              ck(cudaMemsetAsync(Qw, 0, sizeof(double2) * nk, st)) &&
               ck(cudaMemsetAsync(acc, 0, sizeof(double) * 64, st)) &&
               ck(cudaMemsetAsync(status, 0, sizeof(int) * ST_NWORDS, st)) &&
               ck(cudaMemsetAsync(fx, 0, sizeof(double) * n, st)) && ck(cudaMemsetAsync(fy, 0, sizeof(double) * n, st)) &&
@@ -524,13 +605,10 @@ int recip_forces_noalloc(const double* x, const double* y, const double* z, cons
     v.acc = acc;
     v.status = status;
     KDims d{KL, KM, KN, pipix, pipiy, pipiz};
-    const int kblocks = (nwork + kSfacNT - 1) / kSfacNT;
-    int splits = std::max(1, (152 * 4 + kblocks - 1) / std::max(kblocks, 1));
-    splits = std::min(splits, std::max(1, (int)((n + tile - 1) / tile)));
-    const int aps = (int)((n + splits - 1) / splits);
-    k_sfac<<<dim3(kblocks, splits), kSfacNT, smem1, st>>>(v, d, nrow, rows, nlen, wr, wn, nwork, tile, aps, S, nk);
-    k_kenergy<<<std::min((nk + 255) / 256, 256), 256, 0, st>>>(v, nk, Ak, S, Qw, C);
-    k_kforce<<<(int)((n + kForceNT - 1) / kForceNT), kForceNT, smem2, st>>>(v, d, nrow, rows, nlen, C, nk);
+    const KGrid g = k_grid(d, (int)n, nrow, nwork);
+    k_sfac<<<g.sfac, kSfacNT, g.smem_sfac, st>>>(v, d, nrow, rows, wr, wn, nwork, g.atoms_per_split, S, nk);
+    k_kenergy<<<std::min((nrow + 7) / 8, 256), 256, 0, st>>>(v, nrow, rows, nlen, ent, Ak, S, nullptr, C);
+    k_kforce<<<g.force, kForceNT, g.smem_force, st>>>(v, d, nrow, rows, nlen, ent, C);
     k_noalloc_energy<<<1, 32, 0, st>>>(acc, uewa);
     if (cudaGetLastError() != cudaSuccess) return na_fail(MDG_E_CUDA, "mdg_recip_forces_noalloc: launch failed");
     return MDG_OK;

@@ -686,7 +686,7 @@ __global__ void __launch_bounds__(32 * kRedG) k_tc_sreduce(View v, const float* 
                                                           int rtot, TcDims d, const int4* __restrict__ rows,
                                                           const int* __restrict__ nlen,
                                                           const double* __restrict__ ak,
-                                                          const double2* __restrict__ qw, double2* S, double2* C,
+                                                          const double2* __restrict__ qw, double2* S,
                                                           float2* Cf, float* cmax, float* rowsc) {
     __shared__ float4 sh[kRedG][32];
     const int le = threadIdx.x & 31, g = threadIdx.x >> 5;
@@ -737,7 +737,6 @@ __global__ void __launch_bounds__(32 * kRedG) k_tc_sreduce(View v, const float* 
         ll = a * (sv.x * sv.x + sv.y * sv.y);
         ew = a * (st.x * st.x + st.y * st.y);
         const double2 cv = make_double2(a * st.x, -a * st.y);
-        C[k] = cv;
         Cf[k] = make_float2((float)cv.x, (float)cv.y);
         const float w = (float)max(1, abs(n));
         mx = fmaxf(fabsf((float)cv.x), fabsf((float)cv.y)) * w;
@@ -1392,7 +1391,7 @@ void recip_tc(Ctx& c) {
             v, c.d_tc_atoms, p.chunk1, ks.row, d, p.NM, p.KM, c.d_tc_part, p.rtot, (uint32_t)p.ncols1, p.rowsc);
     const long nred = (long)ks.nrow * p.NN;
     k_tc_sreduce<<<(int)((nred + 31) / 32), 32 * kRedG, 0, c.stream>>>(
-        v, c.d_tc_part, p.nsplit1, p.rtot, d, ks.row, ks.row_nlen, ks.ak, ks.qw, ks.s, ks.c, c.d_tc_cf, c.d_tc_cmax,
+        v, c.d_tc_part, p.nsplit1, p.rtot, d, ks.row, ks.row_nlen, ks.ak, ks.qw, ks.s, c.d_tc_cf, c.d_tc_cmax,
         p.rowsc);
     const int per_chunk = p.KS * kNC2 * 8;  // elements of the widest chunk image
     k_tc_prep_c<<<dim3((per_chunk + 255) / 256, p.nchunk2), 256, 0, c.stream>>>(
