@@ -106,8 +106,9 @@ __global__ void __launch_bounds__(kNT) k_pair_fp64(View v) {
             const int jt = v.type[CK(j, v.ntota, 110)];
             const int ijt = CK(v.ijt[CK(it * v.nit + jt, v.nit * v.nit, 111)], v.nijt, 112);
             const int nsi_j = v.nsi[CK(jt, v.nit, 113)];
-            const double rsqi = 1.0 / rsq;
-            const double rij = sqrt(rsq);
+            const double rinv = rsqrt(rsq);
+            const double rsqi = rinv * rinv;
+            const double rij = rsq * rinv;
             double fij = 0.0, elj = 0.0;
             const int vk = v.vdw[ijt];
             if (vk == 1) {
@@ -118,10 +119,10 @@ __global__ void __launch_bounds__(kNT) k_pair_fp64(View v) {
                 const double r6 = v.cc[ijt] * (rsqi * rsqi * rsqi);
                 const double aux = v.aa[ijt] * exp(-rij * v.rhoi[ijt]);
                 elj = aux - r6;
-                fij = aux * v.rhoi[ijt] / rij - 6.0 * rsqi * r6;
+                fij = aux * v.rhoi[ijt] * rinv - 6.0 * rsqi * r6;
             }
             double ff;
-            const double auxq = v.facq * qi[0] * v.q[CK(j, v.ntota, 114)] / rij;
+            const double auxq = v.facq * qi[0] * v.q[CK(j, v.ntota, 114)] * rinv;
             const double erfx = ewald_erfc(v.alfa * rij, &ff, v.spii);
             double eqq = erfx * auxq;
             fij = fij + ff * auxq * rsqi;
@@ -152,13 +153,12 @@ __global__ void __launch_bounds__(kNT) k_pair_fp64(View v) {
                     if (a == 0 && b == 0) continue;
                     const double xd = xa - rjx[b], yd = ya - rjy[b], zd = za - rjz[b];
                     const double r2 = xd * xd + yd * yd + zd * zd;
-                    const double r2i = 1.0 / r2;
-                    const double rr = sqrt(r2);
-                    const double au = qx * qj[b] / rr;
+                    const double ri = rsqrt(r2);
+                    const double au = qx * qj[b] * ri;
                     double fq;
-                    const double ef = ewald_erfc(v.alfa * rr, &fq, v.spii);
+                    const double ef = ewald_erfc(v.alfa * (r2 * ri), &fq, v.spii);
                     eqq += ef * au;
-                    const double fs = fq * au * r2i;
+                    const double fs = fq * au * (ri * ri);
                     fix[a] += xd * fs; fiy[a] += yd * fs; fiz[a] += zd * fs;
                     fjx[b] -= xd * fs; fjy[b] -= yd * fs; fjz[b] -= zd * fs;
                 }
@@ -230,18 +230,17 @@ __global__ void __launch_bounds__(kNT) k_wall_fp64(View v) {
             const int ijt = v.ijt[it * v.nit + v.type[j]];
             double fij = 0.0, elj = 0.0;
             const int vk = v.vdw[ijt];
+            const double rinv = rsqrt(rsq);
+            const double rsqi = rinv * rinv;
             if (vk == 1) {
-                const double rsqi = 1.0 / rsq;
                 const double r6 = v.sig[ijt] * (rsqi * rsqi * rsqi);
                 elj = v.eps[ijt] * r6 * (r6 - 1.0);
                 fij = 6.0 * rsqi * v.eps[ijt] * r6 * (2.0 * r6 - 1.0);
             } else if (vk == 2) {
-                const double rsqi = 1.0 / rsq;
-                const double rij = sqrt(rsq);
                 const double r6 = v.cc[ijt] * (rsqi * rsqi * rsqi);
-                const double aux = v.aa[ijt] * exp(-rij * v.rhoi[ijt]);
+                const double aux = v.aa[ijt] * exp(-(rsq * rinv) * v.rhoi[ijt]);
                 elj = aux - r6;
-                fij = aux * v.rhoi[ijt] / rij - 6.0 * rsqi * r6;
+                fij = aux * v.rhoi[ijt] * rinv - 6.0 * rsqi * r6;
             }
             const double qx = v.facq * v.q[j];
             double eqq = 0.0;
@@ -250,13 +249,12 @@ __global__ void __launch_bounds__(kNT) k_wall_fp64(View v) {
                 if (a >= nsi_i) break;
                 const double xd = xi + rix[a], yd = yi + riy[a], zd = zi + riz[a];
                 const double r2 = xd * xd + yd * yd + zd * zd;
-                const double rr = sqrt(r2);
-                const double r2i = 1.0 / r2;
-                const double au = qx * qi[a] / rr;
+                const double ri = rsqrt(r2);
+                const double au = qx * qi[a] * ri;
                 double fq;
-                const double ef = ewald_erfc(v.alfa * rr, &fq, v.spii);
+                const double ef = ewald_erfc(v.alfa * (r2 * ri), &fq, v.spii);
                 eqq += ef * au;
-                fij = fij + fq * au * r2i;
+                fij = fij + fq * au * (ri * ri);
                 fix[a] += xd * fij; fiy[a] += yd * fij; fiz[a] += zd * fij;
                 if (book) {
                     ws[so] -= xd * fij; ws[so + 1] -= yd * fij; ws[so + 2] -= zd * fij;
