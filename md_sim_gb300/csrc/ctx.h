@@ -108,6 +108,33 @@ struct KSet {
     std::vector<int> h_nlen;
 };
 
+// Device arrays and sizes of the gridded reciprocal sum (recip_nu.cu), passed to kernels by value.
+struct NuView {
+    int M[3], K[3];          // grid points and largest frequency per direction
+    int n8[3], nblk;         // blocks of 8 x 8 x 8 cells
+    int cap, split, ngrp, mgrp, ygrp, yrows;
+    float scale[3];          // d(grid coordinate)/d(position), with the reference's pi
+    int* cnt = nullptr;      // atoms per block (beyond cap: in ovf), then those in ovf; 0 between evaluations
+    int* cntf = nullptr;     // the same counts for the force kernel
+    int* bucket = nullptr;   // their indices, cap per block
+    int* novf = nullptr;     // cnt + nblk: atoms that found their bucket full
+    int* ovf = nullptr;      // their indices
+    float* grid = nullptr;   // charges [x][y][z], zero between evaluations
+    float* pot = nullptr;    // potential [x][y][z]
+    float2* H = nullptr;     // [n][x][m + KM]
+    float2 *tw[3], *twt[3];  // twiddles by (point, frequency) and by (frequency, point)
+    double* dec[3];          // 1 / transform of the spreading window, then of the force window
+    int* kmap = nullptr;     // [n][m + KM][l + KL]: 2 k + (conjugate), or -1
+    double2* S = nullptr;    // the k set's arrays (KSet)
+    const double2* qw = nullptr;
+    const double* ak = nullptr;
+};
+struct NuPlan {
+    bool ready = false;
+    NuView g{};
+    int smem_zy = 0, smem_x = 0, smem_yz = 0;
+};
+
 // Per-step packed atom records of the mixed-precision real-space kernels (pair_mx.cu).
 struct Pk {
     uint4* P = nullptr;     // fixed-point x, y (z if periodic) | FP32 z hi; w = type | sign(z) << 31
@@ -115,6 +142,9 @@ struct Pk {
     float* zlo = nullptr;   // z - z_hi when z is not periodic
     float4* F = nullptr;    // j-side force accumulator (moving atoms)
     uint4* tc = nullptr;    // reciprocal-sum records (moving atoms), or nullptr
+    // buckets of the gridded reciprocal sum (NuView), or nullptr
+    int *nu_cnt = nullptr, *nu_bucket = nullptr, *nu_novf = nullptr, *nu_ovf = nullptr;
+    int nu_M[3] = {0, 0, 0}, nu_n8[3] = {0, 0, 0}, nu_cap = 0;
     float* cmax = nullptr;  // scale of the reciprocal sum's pass-2 operand, cleared here for it
     double* part = nullptr; // per-block slab dipole shares of the packing kernel
     float sx = 0, sy = 0, sz = 0;  // box edge / 2^32
@@ -149,10 +179,10 @@ struct Meas {
 // Launch plan of the tensor-core reciprocal sum (recip_tc.cu).
 struct TcPlan {
     bool ready = false;
-    int KN = 0, NN = 0, NP = 0, KS = 0, KM = 0, NM = 0;
-    int ncols1 = 0, mtiles = 0, nchunk2 = 0, chunk1 = 0, nsplit1 = 0, grid1x = 0, rtot = 0, tpc1 = 0, smem1 = 0, smem2 = 0;
+    int KN = 0, NN = 0, NP = 0, KS = 0;
+    int mtiles = 0, nchunk2 = 0, chunk1 = 0, nsplit1 = 0, grid1x = 0, rtot = 0, smem1 = 0, smem2 = 0;
     int ntile2 = 0, nparts2 = 0, cper2 = 0, grid2 = 0, nlist2 = 0, mult1 = 2, nst2 = 2;
-    int G1 = 4;  // n-side pass 1: groups of 16 atoms per TMEM accumulation chain
+    int G1 = 4;  // pass 1: groups of 16 atoms per TMEM accumulation chain
     int4* row2 = nullptr;    // pass-2 rows, sorted by their K-step range (nchunk2 x kRC, padded)
     int* rorig2 = nullptr;   // pass-2 row -> row of the k set (-1: padding)
     float* rowsc = nullptr;  // per row of the k set: max |C| max(1, |n|) of this evaluation
@@ -176,6 +206,7 @@ struct Ctx {
     Grid grid{}, wgrid{};
     KSet ks;
     TcPlan tcp;
+    NuPlan nu;
     Pk pk;
     uint4* d_tc_atoms = nullptr;        // fixed-point phases + charge per moving atom
     unsigned char* d_tc_img = nullptr;  // packed C(k) operand chunks
@@ -324,12 +355,15 @@ int recip_forces_noalloc(const double* x, const double* y, const double* z, cons
 const char* recip_noalloc_error();
 // recip_tc.cu
 int recip_tc_setup(Ctx& c);
-int tc_plan_pass1(Ctx& c, int tpc, int mult);
+void tc_plan_pass1(Ctx& c, int mult);
 // on: the fewest CTAs per pass (pass 1 in chunks of about 1024 atoms, pass 2 whole tiles), for a
 // system stepped among many in one graph; off: back to the plan for the system alone.  Drops the
 // context's captured graphs.
 int recip_tc_throughput(Ctx& c, bool on);
-void recip_tc(Ctx& c);
+void recip_tc(Ctx& c);  // (or the gridded sum, by the size of the system)
+// recip_nu.cu
+int recip_nu_setup(Ctx& c);
+void recip_nu(Ctx& c);
 int umma_selftest(int n, int k, const float* a, const float* b, float* d, std::string& err);
 // mlp.cu
 int mlp_nw();

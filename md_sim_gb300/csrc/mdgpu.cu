@@ -577,6 +577,18 @@ int mdg_create(const mdg_sysdesc* s, const mdg_params* p, const double* x0, cons
         rc = recip_tc_setup(c);
         if (rc) return bail(rc);
         pack_setup(c);
+        if (c.nu.ready) {
+            const NuView& g = c.nu.g;
+            c.pk.nu_cnt = g.cnt;
+            c.pk.nu_bucket = g.bucket;
+            c.pk.nu_novf = g.novf;
+            c.pk.nu_ovf = g.ovf;
+            c.pk.nu_cap = g.cap;
+            for (int d = 0; d < 3; ++d) {
+                c.pk.nu_M[d] = g.M[d];
+                c.pk.nu_n8[d] = g.n8[d];
+            }
+        }
         c.pk.tc = c.d_tc_atoms;
         c.pk.cmax = c.d_tc_cmax;
         std::vector<float> parf(6 * (size_t)std::max<int64_t>(nijt, 1), 0.f);
@@ -1774,28 +1786,23 @@ int mdg_autotune(mdg_ctx* cp, int32_t reps, mdg_tuning* out) {
         }
     }
     c.pair_blocks = best_pb;
-    // structure-factor split: row tiles per CTA x atom splits
+    // atom splits of the structure factor (tensor-core form)
     if (c.precision == MDG_MIXED && c.tcp.ready) {
         const int trc = recip_tc_throughput(c, false);  // tune the plan for the system alone
         if (trc) return trc;
     }
-    int best_tpc = c.tcp.tpc1, best_mult = c.tcp.mult1;
     if (c.precision == MDG_MIXED && c.tcp.ready) {
         best = time_force(c, reps);
-        // the n-side form when it applies (its accumulation chains are short), its atom split tuned
-        const bool nside = c.tcp.tpc1 == 1;
-        for (int tpc : {1, 4, 2})
-            for (int m : {1, 2, 4}) {
-                if ((tpc == 1) != nside) continue;
-                if (tc_plan_pass1(c, tpc, m)) continue;
-                const float t = time_force(c, reps);
-                if (t < best * kTuneGain) {
-                    best = t;
-                    best_tpc = tpc;
-                    best_mult = m;
-                }
+        int best_mult = c.tcp.mult1;
+        for (int m : {1, 2, 4}) {
+            tc_plan_pass1(c, m);
+            const float t = time_force(c, reps);
+            if (t < best * kTuneGain) {
+                best = t;
+                best_mult = m;
             }
-        tc_plan_pass1(c, best_tpc, best_mult);
+        }
+        tc_plan_pass1(c, best_mult);
     }
     drop_graphs(c);
     const float t1 = time_force(c, reps);
@@ -1804,8 +1811,8 @@ int mdg_autotune(mdg_ctx* cp, int32_t reps, mdg_tuning* out) {
     if (rc) return rc;
     if (out) {
         out->pair_blocks = best_pb;
-        out->tc_rows_per_cta = best_tpc == 1 ? 256 : 128 * best_tpc;
-        out->tc_atom_splits = c.tcp.nsplit1;
+        out->tc_rows_per_cta = 256;
+        out->tc_atom_splits = std::max(c.tcp.nsplit1, 1);  // 1: the gridded sum has no such split
         out->ms_before = t0;
         out->ms_after = t1;
     }

@@ -51,6 +51,13 @@ __device__ __forceinline__ double pack_atom(const View& v, const Pk& pk, int a, 
         v.fz[a] = 0.0;
         mz = qa * z;
         if (pk.tc) pk.tc[a] = make_uint4(p.x, p.y, uz, __float_as_uint(q.w));
+        if (pk.nu_cnt) {  // the block of 8 x 8 x 8 grid cells that holds the atom
+            const int bx = __umulhi(p.x, pk.nu_M[0]) >> 3, by = __umulhi(p.y, pk.nu_M[1]) >> 3, bz = __umulhi(uz, pk.nu_M[2]) >> 3;
+            const int b = (bx * pk.nu_n8[1] + by) * pk.nu_n8[2] + bz;
+            const int k = atomicAdd(&pk.nu_cnt[b], 1);
+            if (k < pk.nu_cap) pk.nu_bucket[(size_t)b * pk.nu_cap + k] = a;
+            else pk.nu_ovf[atomicAdd(pk.nu_novf, 1)] = a;
+        }
     }
     pk.Q[a] = q;
     return mz;

@@ -6,11 +6,9 @@
 //              q_j kz sum_{l,m} Im( e^{i(l tx_j + m ty_j)} T'_j(l,m) ) with
 //   T_j(l,m) = sum_n C(l,m,n) e^{i n tz_j},  T'_j(l,m) = sum_n n C(l,m,n) e^{i n tz_j}   (pass 2)
 // with C = Ak conj(S + S_wall).  Both are complex matrix products written as real ones:
-//   pass 1: the structure factor over K = atoms, split-K over atom chunks, in one of two forms:
-//           n-side (k_tc_sfac2, used when 2 (2 KN + 1) <= 128): D[(re|im, n) lane, (l, m) row],
-//           A = q e^{i n tz} in the 2x2 real block form, B = e^{i(l tx + m ty)}, N = 256 rows per
-//           CTA; row-side (k_tc_sfac): D[(l, m) row, (re|im, n)], A = [Re | Im] of the row factor,
-//           B = the 2x2 block form of e^{i n tz}, M = 128 rows per tile;
+//   pass 1: the structure factor over K = atoms, split-K over atom chunks (k_tc_sfac2, for
+//           2 (2 KN + 1) <= 128): D[(re|im, n) lane, (l, m) row], A = q e^{i n tz} in the 2x2 real
+//           block form, B = e^{i(l tx + m ty)}, N = 256 rows per CTA;
 //   pass 2: D[atom, (row, T|T', re|im)] over K = (n, re|im), A = e^{i n tz} per atom (built once
 //           per CTA), B = packed C chunks streamed with cp.async.bulk through a ring of K-step
 //           slots, two TMEM accumulators double-buffered against the epilogue that forms
@@ -51,65 +49,7 @@ __device__ __forceinline__ void phase(uint32_t u, float& c, float& s) {
 }
 
 
-// ---------------------------------------------------------------------------------------------
-// pass 1: structure factor
-//
-// One CTA owns TPC row tiles (TPC * 128 (l, m) rows; TPC = 4 when the accumulators fit TMEM) and a
-// contiguous chunk of atoms, walked in groups of kGA = 16 atoms (one K step) through a 2-3 deep
-// shared-memory ring:
-//   producer warps (one thread per row): per group, phase tables e^{i m ty_j} (all m) and q_j e^{i l tx_j}
-//       (the l values of the CTA's rows) by __sincosf of exact fixed-point phases, the B tiles
-//       e^{i n tz_j} in the 2x2 real block form, then each thread its row's A entries
-//       q_j e^{i l tx_j} e^{i m ty_j} = table products, split hi/lo and stored in the UMMA
-//       canonical layout; arrive on full[s];
-//   last warp, lane 0 (issuer): waits full[s], issues 3 (hi/lo) x 2 (re/im part) MMAs per tile,
-//       commits to empty[s], which frees the stage for the producers.
-// The accumulators (one per tile, N = NP columns) are written once, as FP32 partial sums per
-// atom chunk, to part[split][col][row]; k_tc_sreduce adds the chunks in compensated FP32 and
-// forms S(k), the energy terms, C(k) and the scale of the pass-2 operand (src/forcem.f90:879-917).
-// ---------------------------------------------------------------------------------------------
 constexpr int kGA = 16;                  // atoms per group (one K step)
-constexpr int kMaxNL = 64;               // l values per CTA (table width; the last slot stays 0)
-constexpr int kMaxItems = 4;             // table entries per producer thread and group
-
-template <int TPC>
-struct P1 {
-    static constexpr int kProd = 128 * TPC;      // producer threads: one per CTA row
-    static constexpr int kThreads = kProd + 32;  // + issuer warp
-    static constexpr int kS = TPC >= 4 ? 2 : 3;  // ring depth
-};
-
-struct P1Layout {
-    uint32_t a_bytes, b_tile, stage, tab_m, tab_l, off_stage, off_tab, total;
-};
-
-// tables: e^{i m ty} as float2 [atom][NM + 1] (slot NM = 0), q e^{i l tx} as float2 [atom][kMaxNL]
-__host__ __device__ inline P1Layout p1_layout(int tpc, int stages, int NP, int NM) {
-    P1Layout L;
-    L.a_bytes = tpc * 4 * 4096;                         // [tile][p][h] 128 x 16 halves
-    L.b_tile = (uint32_t)NP * 32;                       // NP x 16 halves
-    L.stage = L.a_bytes + 4 * L.b_tile;                 // + [p][h] B tiles
-    L.tab_m = (uint32_t)kGA * (NM + 1) * 8;
-    L.tab_l = (uint32_t)kGA * kMaxNL * 8;
-    L.off_stage = 1024;
-    L.off_tab = L.off_stage + stages * L.stage;
-    L.total = L.off_tab + 2 * (L.tab_m + L.tab_l);
-    return L;
-}
-
-// Named barrier 1 over the producer warps with an AND of their flags (every producer reaches it on
-// every group, so a timeout seen by one producer stops all of them together).
-template <int NPROD>
-__device__ __forceinline__ bool producers_all(bool ok) {
-    uint32_t res;
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.u32 q, %1, 0;\n\tbar.red.and.pred p, 1, %2, q;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}\n"
-        : "=r"(res)
-        : "r"((uint32_t)ok), "n"(NPROD)
-        : "memory");
-    return res != 0;
-}
 
 __device__ __forceinline__ uint32_t pack_h2(float a, float b) {
     const __half2 h = __floats2half2_rn(a, b);
@@ -124,236 +64,8 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
     lo = pack_h2(a - hf.x, b - hf.y);
 }
 
-template <int TPC>
-__global__ void __launch_bounds__(P1<TPC>::kThreads, 1)
-    k_tc_sfac(View v, const uint4* __restrict__ atoms, int chunk, const int4* __restrict__ rows, TcDims d, int NM,
-              int KM, float* __restrict__ part, int rtot, uint32_t ncols, float* __restrict__ rowsc) {
-    constexpr int kProd = P1<TPC>::kProd, kS = P1<TPC>::kS;
-    extern __shared__ __align__(1024) unsigned char sm[];
-    const P1Layout L = p1_layout(TPC, kS, d.NP, NM);
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    uint64_t* full = reinterpret_cast<uint64_t*>(sm);
-    uint64_t* empty = full + kS;
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(sm + 512);
-    int* err = &v.status[ST_TC_TIMEOUT];
-    const int a0 = blockIdx.y * chunk, a1 = min(v.nmove, a0 + chunk);
-    const int ngroup = a1 > a0 ? (a1 - a0 + kGA - 1) / kGA : 0;
-    const int row0 = blockIdx.x * (TPC * 128);
-    const int rlast = min(row0 + TPC * 128, d.nrow) - 1;
-    const int l_lo = rows[row0].x, nl = min(rows[rlast].x - l_lo + 1, kMaxNL - 1);
-    const int NM1 = NM + 1;
-    if (t == 0) {
-        for (int i = 0; i < kS; ++i) {
-            tc::mbar_init(tc::smem_u32(&full[i]), kProd);
-            tc::mbar_init(tc::smem_u32(&empty[i]), 1);
-        }
-        tc::mbar_fence_init();
-    }
-    // zero the ring (B rows beyond 2 NN stay zero) and both table buffers (padding slots stay zero)
-    for (uint32_t o = t * 16; o < L.total - L.off_stage; o += P1<TPC>::kThreads * 16)
-        *reinterpret_cast<uint4*>(sm + L.off_stage + o) = make_uint4(0, 0, 0, 0);
-    if (warp == 0) tc::tmem_alloc(tc::smem_u32(tslot), ncols);
-    tc::fence_before();
-    __syncthreads();
-    tc::fence_after();
-    const uint32_t tmem = *tslot;
-    const uint32_t tcols = ncols / TPC;
-    bool alive = true;
-    if (warp == kProd / 32) {
-        // ---------------- issuer
-        if (lane == 0) {
-            const uint32_t idesc = idesc_e(128, d.NP);
-            const uint64_t dS0 = tc::desc(tc::smem_u32(sm + L.off_stage));
-            int committed = -1;
-            for (int g = 0; g < ngroup && alive; ++g) {
-                const int s = g % kS;
-                alive = tc::mbar_wait(tc::smem_u32(&full[s]), (g / kS) & 1, err, 11);
-                if (!alive) break;
-                tc::fence_after();
-                const uint64_t ds = dS0 + (uint64_t)((s * L.stage) >> 4);
-                const uint64_t db = ds + (uint64_t)(L.a_bytes >> 4);
-                // all products of one accumulator back to back: switching the accumulator between
-                // consecutive MMAs roughly halves the issue rate
-#pragma unroll
-                for (int tile = 0; tile < TPC; ++tile) {
-                    const uint32_t dcol = tmem + tile * tcols;
-#pragma unroll
-                    for (int p = 0; p < 2; ++p) {
-                        const uint64_t bh = db + (uint64_t)(((p * 2 + 0) * L.b_tile) >> 4);
-                        const uint64_t bl = db + (uint64_t)(((p * 2 + 1) * L.b_tile) >> 4);
-                        const uint64_t ah = ds + (uint64_t)(((tile * 2 + p) * 2 + 0) * 256);
-                        const uint64_t al = ds + (uint64_t)(((tile * 2 + p) * 2 + 1) * 256);
-                        tc::mma_bf16(dcol, ah, bh, idesc, (g > 0 || p > 0) ? 1u : 0u);
-                        tc::mma_bf16(dcol, ah, bl, idesc, 1u);
-                        tc::mma_bf16(dcol, al, bh, idesc, 1u);
-                    }
-                }
-                tc::commit(tc::smem_u32(&empty[s]));
-                committed = g;
-            }
-            // on a timeout, let the issued MMAs drain (bounded) before the block frees its TMEM
-            if (!alive && committed >= 0)
-                tc::mbar_wait(tc::smem_u32(&empty[committed % kS]), (committed / kS) & 1, nullptr, 0);
-        }
-    } else {
-        // ---------------- producers
-        const int r = t;                                 // CTA row (tile = r / 128)
-        const int row = row0 + r;
-        if (blockIdx.y == 0 && row < d.nrow) rowsc[row] = 0.f;  // k_tc_sreduce takes the maximum
-        int li = kMaxNL - 1, mi = NM;                    // zero slots for padding rows
-        if (row < d.nrow) {
-            const int4 rw = rows[row];
-            li = min(rw.x - l_lo, kMaxNL - 2);
-            mi = rw.y + KM;
-        }
-        const int tile = r >> 7, rr = r & 127;
-        // this thread's table entries (the same every group): e^{i m ty} items, q e^{i l tx} items,
-        // and B items (n, atom pair)
-        const int nm_items = kGA * NM, nl_items = kGA * nl, nb_items = d.NN * (kGA / 2);
-        // items packed as (atom << 16) | index, -1 when the thread has no such item
-        int im_i[kMaxItems], il_i[kMaxItems], ib_i[kMaxItems];
-#pragma unroll
-        for (int k = 0; k < kMaxItems; ++k) {
-            const int e = t + k * kProd;
-            im_i[k] = e < nm_items ? ((e / NM) << 16) | (e % NM) : -1;
-            il_i[k] = e < nl_items ? ((e / nl) << 16) | (e % nl) : -1;
-            ib_i[k] = e < nb_items ? (((e / d.NN) * 2) << 16) | (e % d.NN) : -1;
-        }
-#define IM_J(k) (im_i[k] >> 16)
-#define IM_M(k) (im_i[k] & 0xffff)
-#define IL_J(k) (il_i[k] >> 16)
-#define IL_L(k) (il_i[k] & 0xffff)
-#define IB_J(k) (ib_i[k] >> 16)
-#define IB_N(k) (ib_i[k] & 0xffff)
-        // the atom fractions this thread's items need, loaded one group ahead so that the global
-        // load latency overlaps the barrier and the A fill of the current group
-        uint32_t pm[kMaxItems], plx[kMaxItems], plq[kMaxItems], pb0[kMaxItems], pb1[kMaxItems];
-        auto prefetch = [&](int gb) {
-#pragma unroll
-            for (int k = 0; k < kMaxItems; ++k) {
-                pm[k] = (im_i[k] >= 0 && gb + IM_J(k) < a1) ? __ldg(&atoms[gb + IM_J(k)].y) : 0u;
-                plx[k] = plq[k] = 0u;
-                if (il_i[k] >= 0 && gb + IL_J(k) < a1) {
-                    const uint4 rec = __ldg(&atoms[gb + IL_J(k)]);
-                    plx[k] = rec.x;
-                    plq[k] = rec.w;
-                }
-                pb0[k] = (ib_i[k] >= 0 && gb + IB_J(k) < a1) ? __ldg(&atoms[gb + IB_J(k)].z) : 0u;
-                pb1[k] = (ib_i[k] >= 0 && gb + IB_J(k) + 1 < a1) ? __ldg(&atoms[gb + IB_J(k) + 1].z) : 0u;
-            }
-        };
-        if (ngroup > 0) prefetch(a0);
-        for (int g = 0; g < ngroup; ++g) {
-            const int s = g % kS;
-            const int gb = a0 + g * kGA;
-            float2* tm = reinterpret_cast<float2*>(sm + L.off_tab + (g & 1) * (L.tab_m + L.tab_l));
-            float2* tl = reinterpret_cast<float2*>(reinterpret_cast<unsigned char*>(tm) + L.tab_m);
-            bool ok = true;
-            if (g >= kS) ok = tc::mbar_wait_warp(tc::smem_u32(&empty[s]), ((g / kS) - 1) & 1, err, 12);
-            unsigned char* st = sm + L.off_stage + s * L.stage;
-            unsigned char* bb = st + L.a_bytes;
-            if (ok) {
-#pragma unroll
-                for (int k = 0; k < kMaxItems; ++k) {
-                    if (im_i[k] >= 0) {
-                        const int at = gb + IM_J(k);
-                        float c = 0.f, sn = 0.f;
-                        if (at < a1) phase((uint32_t)(IM_M(k) - KM) * pm[k], c, sn);
-                        tm[IM_J(k) * NM1 + IM_M(k)] = make_float2(c, sn);
-                    }
-                    if (il_i[k] >= 0) {
-                        const int at = gb + IL_J(k);
-                        float c = 0.f, sn = 0.f;
-                        if (at < a1) {
-                            phase((uint32_t)(IL_L(k) + l_lo) * plx[k], c, sn);
-                            const float q = __uint_as_float(plq[k]);
-                            c *= q;
-                            sn *= q;
-                        }
-                        tl[IL_J(k) * kMaxNL + IL_L(k)] = make_float2(c, sn);
-                    }
-                    if (ib_i[k] >= 0) {
-                        const int jp = IB_J(k), ni = IB_N(k);
-                        const uint32_t n = (uint32_t)(ni - d.KN);
-                        float c0 = 0.f, s0 = 0.f, c1 = 0.f, s1 = 0.f;
-                        if (gb + jp < a1) phase(n * pb0[k], c0, s0);
-                        if (gb + jp + 1 < a1) phase(n * pb1[k], c1, s1);
-                        uint32_t ch, cl, sh, sl;
-                        split2(c0, c1, ch, cl);
-                        split2(s0, s1, sh, sl);
-                        const uint32_t ore = tc::tile_off(ni, jp), oim = tc::tile_off(d.NN + ni, jp);
-                        // part 0: re row <- cos, im row <- sin ; part 1: re row <- -sin, im row <- cos
-                        *reinterpret_cast<uint32_t*>(bb + 0 * L.b_tile + ore) = ch;
-                        *reinterpret_cast<uint32_t*>(bb + 1 * L.b_tile + ore) = cl;
-                        *reinterpret_cast<uint32_t*>(bb + 0 * L.b_tile + oim) = sh;
-                        *reinterpret_cast<uint32_t*>(bb + 1 * L.b_tile + oim) = sl;
-                        *reinterpret_cast<uint32_t*>(bb + 2 * L.b_tile + ore) = sh ^ 0x80008000u;
-                        *reinterpret_cast<uint32_t*>(bb + 3 * L.b_tile + ore) = sl ^ 0x80008000u;
-                        *reinterpret_cast<uint32_t*>(bb + 2 * L.b_tile + oim) = ch;
-                        *reinterpret_cast<uint32_t*>(bb + 3 * L.b_tile + oim) = cl;
-                    }
-                }
-            }
-            if (g + 1 < ngroup) prefetch(gb + kGA);
-            if (!producers_all<kProd>(ok)) {
-                alive = false;
-                break;
-            }
-            // A: this row's 16 entries q e^{i l tx} e^{i m ty} (zero for padding rows)
-            uint32_t wrh[8], wrl[8], wih[8], wil[8];
-#pragma unroll
-            for (int j = 0; j < kGA; j += 2) {
-                const float2 el0 = tl[j * kMaxNL + li], em0 = tm[j * NM1 + mi];
-                const float2 el1 = tl[(j + 1) * kMaxNL + li], em1 = tm[(j + 1) * NM1 + mi];
-                const float re0 = el0.x * em0.x - el0.y * em0.y, im0 = el0.x * em0.y + el0.y * em0.x;
-                const float re1 = el1.x * em1.x - el1.y * em1.y, im1 = el1.x * em1.y + el1.y * em1.x;
-                split2(re0, re1, wrh[j >> 1], wrl[j >> 1]);
-                split2(im0, im1, wih[j >> 1], wil[j >> 1]);
-            }
-            unsigned char* ta = st + (tile * 2) * 2 * 4096;   // [tile][p][h]
-            const uint32_t o0 = tc::tile_off(rr, 0), o8 = tc::tile_off(rr, 8);
-            *reinterpret_cast<uint4*>(ta + 0 * 4096 + o0) = make_uint4(wrh[0], wrh[1], wrh[2], wrh[3]);
-            *reinterpret_cast<uint4*>(ta + 0 * 4096 + o8) = make_uint4(wrh[4], wrh[5], wrh[6], wrh[7]);
-            *reinterpret_cast<uint4*>(ta + 1 * 4096 + o0) = make_uint4(wrl[0], wrl[1], wrl[2], wrl[3]);
-            *reinterpret_cast<uint4*>(ta + 1 * 4096 + o8) = make_uint4(wrl[4], wrl[5], wrl[6], wrl[7]);
-            *reinterpret_cast<uint4*>(ta + 2 * 4096 + o0) = make_uint4(wih[0], wih[1], wih[2], wih[3]);
-            *reinterpret_cast<uint4*>(ta + 2 * 4096 + o8) = make_uint4(wih[4], wih[5], wih[6], wih[7]);
-            *reinterpret_cast<uint4*>(ta + 3 * 4096 + o0) = make_uint4(wil[0], wil[1], wil[2], wil[3]);
-            *reinterpret_cast<uint4*>(ta + 3 * 4096 + o8) = make_uint4(wil[4], wil[5], wil[6], wil[7]);
-            tc::fence_async_smem();
-            tc::mbar_arrive(tc::smem_u32(&full[s]));
-        }
-#undef IM_J
-#undef IM_M
-#undef IL_J
-#undef IL_L
-#undef IB_J
-#undef IB_N
-        // all MMAs done -> accumulators to the partial-sum buffer
-        if (ngroup > 0 && alive)
-            alive = tc::mbar_wait_warp(tc::smem_u32(&empty[(ngroup - 1) % kS]), ((ngroup - 1) / kS) & 1, err, 13);
-        tc::fence_after();
-        const uint32_t tbase = tmem + ((uint32_t)((warp & 3) * 32) << 16) + tile * tcols;
-        float* dst = part + (size_t)blockIdx.y * d.NP * rtot;
-        for (int cc = 0; cc < d.NP / 16; ++cc) {
-            float val[16];
-            tc::tmem_ld16(tbase + cc * 16, val);
-            if (!alive) continue;
-#pragma unroll
-            for (int c = 0; c < 16; ++c) dst[(size_t)(cc * 16 + c) * rtot + row] = ngroup > 0 ? val[c] : 0.f;
-        }
-        tc::fence_before();
-    }
-    __syncthreads();
-    if (warp == 0) {
-        tc::fence_after();
-        tc::tmem_dealloc(tmem, ncols);
-    }
-}
-
 // ---------------------------------------------------------------------------------------------
-// pass 1, n-side form (2 NN <= 128): the same structure factor with the roles of the operands
-// swapped, D[(re|im, n) lane, (l, m) row] over K = atoms:
+// pass 1: the structure factor as D[(re|im, n) lane, (l, m) row] over K = atoms:
 //   A (M = 128 lanes): q e^{i n tz} in the 2x2 real block form (part 0: cos / sin, part 1: -sin /
 //     cos), lanes n (re) and NN + n (im), zero beyond 2 NN;
 //   B (N = 256 rows): the real (part 0) and imaginary (part 1) parts of e^{i(l tx + m ty)}.
@@ -1156,58 +868,28 @@ __global__ void __launch_bounds__(128, 1) k_umma_selftest(const float* A, const 
 
 }  // namespace
 
-// Pass-1 launch plan: tpc row tiles per CTA (2 or 4) and mult x (152 / row-tile groups) atom
-// splits (mult 2 is the default; the autotuner tries the others).  Returns nonzero when the
-// combination does not fit (TMEM columns or table capacity).
-// mult: CTAs about 76 mult per launch (one system alone: fill the GPU), or 0 for the fewest
-// CTAs of about kThroughputChunk atoms each (a system among many in one graph, where the GPU is
-// full anyway and each CTA's set-up is paid in SM time).
+// Pass-1 launch plan: at most kMaxChunk1b atoms per CTA (their records in shared memory), 256 rows.
+// mult: CTAs about 76 mult per launch (one system alone: fill the GPU; 2 is the default, the
+// autotuner tries the others), or 0 for the fewest CTAs of about kThroughputChunk atoms each (a
+// system among many in one graph, where the GPU is full anyway and each CTA's set-up is paid in SM
+// time).
 constexpr int kThroughputChunk = 1024;
 
-int tc_plan_pass1(Ctx& c, int tpc, int mult) {
+void tc_plan_pass1(Ctx& c, int mult) {
     View& v = c.v;
     KSet& ks = c.ks;
     TcPlan& p = c.tcp;
-    const int nthr = std::max(1, (v.nmove + kThroughputChunk - 1) / kThroughputChunk);
-    if (tpc == 1) {
-        // n-side form: 2 NN lanes in one 128-lane accumulator, 256 rows per CTA, at most
-        // kMaxChunk1b atoms per CTA (their records in shared memory)
-        if (2 * p.NN > 128) return 1;
-        const size_t smem = p1b_layout().total;
-        if (smem > 227 * 1024) return 1;
-        p.smem1 = (int)smem;
-        p.tpc1 = 1;
-        p.ncols1 = 512;
-        p.grid1x = (ks.nrow + 255) / 256;
-        p.rtot = p.grid1x * 256;
-        p.nsplit1 = mult > 0 ? std::max(1, std::min(std::max(1, 76 * mult / p.grid1x), (v.nmove + kGA - 1) / kGA))
-                             : nthr;
-        p.nsplit1 = std::max(p.nsplit1, (v.nmove + kMaxChunk1b - 1) / kMaxChunk1b);
-        p.chunk1 = (v.nmove + p.nsplit1 - 1) / p.nsplit1;
-        p.chunk1 = std::max(kGA, (p.chunk1 + kGA - 1) / kGA * kGA);
-        if (p.chunk1 > kMaxChunk1b) return 1;
-        p.nsplit1 = std::max(1, (v.nmove + p.chunk1 - 1) / p.chunk1);
-        p.mult1 = mult;
-        p.G1 = 8;
-        return 0;
-    }
-    if (tpc == 4 && p.NP > 128) return 1;
-    if (kGA * p.NM > kMaxItems * 128 * tpc || kGA * (kMaxNL - 1) > kMaxItems * 128 * tpc ||
-        p.NN * (kGA / 2) > kMaxItems * 128 * tpc)
-        return 1;
-    const size_t smem = tpc == 4 ? p1_layout(4, P1<4>::kS, p.NP, p.NM).total : p1_layout(2, P1<2>::kS, p.NP, p.NM).total;
-    if (smem > 227 * 1024) return 1;
-    p.smem1 = (int)smem;
-    p.tpc1 = tpc;
-    p.ncols1 = tpc * (p.NP <= 128 ? 128 : 256);
-    p.grid1x = (ks.nrow + tpc * 128 - 1) / (tpc * 128);
-    p.rtot = p.grid1x * tpc * 128;
-    p.nsplit1 = mult > 0 ? std::max(1, std::min(std::max(1, 76 * mult / p.grid1x), (v.nmove + 127) / 128)) : nthr;
+    p.smem1 = (int)p1b_layout().total;
+    p.grid1x = (ks.nrow + 255) / 256;
+    p.rtot = p.grid1x * 256;
+    p.nsplit1 = mult > 0 ? std::max(1, std::min(std::max(1, 76 * mult / p.grid1x), (v.nmove + kGA - 1) / kGA))
+                         : std::max(1, (v.nmove + kThroughputChunk - 1) / kThroughputChunk);
+    p.nsplit1 = std::max(p.nsplit1, (v.nmove + kMaxChunk1b - 1) / kMaxChunk1b);
     p.chunk1 = (v.nmove + p.nsplit1 - 1) / p.nsplit1;
     p.chunk1 = std::max(kGA, (p.chunk1 + kGA - 1) / kGA * kGA);
     p.nsplit1 = std::max(1, (v.nmove + p.chunk1 - 1) / p.chunk1);
     p.mult1 = mult;
-    return 0;
+    p.G1 = 8;
 }
 
 // Work items of pass 2 (one CTA each): whole atom tiles; with pieces, the tiles of the last,
@@ -1266,8 +948,7 @@ int recip_tc_throughput(Ctx& c, bool on) {
     TcPlan& p = c.tcp;
     if (!p.ready || on == p.throughput) return MDG_OK;
     if (on) p.mult_alone = p.mult1;
-    if (tc_plan_pass1(c, p.tpc1, on ? 0 : p.mult_alone))
-        return set_err(&c, MDG_E_UNSUPPORTED, "tensor-core plan");
+    tc_plan_pass1(c, on ? 0 : p.mult_alone);
     const int k = on ? 1 : 0;
     p.items2 = p.items2_k[k];
     p.nitems2 = p.nitems2_k[k];
@@ -1277,6 +958,12 @@ int recip_tc_throughput(Ctx& c, bool on) {
     return MDG_OK;
 }
 
+// (atom, k) products from which the gridded sum (recip_nu.cu) is taken.  Resident step, alone on the
+// GPU, tensor cores against grid: 17,496 atoms x 5,876 k (1.0e8) 98.9 and 93.6 us, 9,000 x 7,404
+// with walls (6.7e7) 116.7 and 99.0, 14,739 x 4,717 (7.0e7) 89.0 and 98.6, 12,288 x 3,720 (4.6e7)
+// 80.7 and 81.0, 6,144 x 4,338 (2.7e7) 84.8 and 89.2; 98,304 x 29,038 (2.9e9) 462 and 240.
+constexpr double kGridWork = 8e7;
+
 int recip_tc_setup(Ctx& c) {
     View& v = c.v;
     KSet& ks = c.ks;
@@ -1285,20 +972,12 @@ int recip_tc_setup(Ctx& c) {
     p.NN = 2 * ks.knmax + 1;
     p.NP = (2 * p.NN + 15) / 16 * 16;
     p.KS = (2 * p.NN + 15) / 16;
-    p.KM = ks.kmmax;
-    p.NM = 2 * ks.kmmax + 1;
+    // limits of the operand tables and tiles, for either form of the sum (what was refused by the
+    // forms before stays refused)
     if (p.NP > 256) return set_err(&c, MDG_E_UNSUPPORTED, "knmax too large for the tensor-core reciprocal sum");
-    if (ks.klmax + 1 > kMaxNL - 1) return set_err(&c, MDG_E_UNSUPPORTED, "klmax too large for the tensor-core reciprocal sum");
-    // the n-side form where it applies, else the row-side form with 4 or 2 row tiles per CTA
-    const int tpc0 = !tc_plan_pass1(c, 1, 2) ? 1 : p.NP <= 128 ? 4 : 2;
-    if (tc_plan_pass1(c, tpc0, 2) && tc_plan_pass1(c, 2, 2))
+    if (ks.klmax > 62) return set_err(&c, MDG_E_UNSUPPORTED, "klmax too large for the tensor-core reciprocal sum");
+    if (2 * p.NN > 128 && 2 * ks.kmmax + 1 > 64)
         return set_err(&c, MDG_E_UNSUPPORTED, "k range too large for the tensor-core table fill");
-    // the partial-sum buffer is sized for the largest split the autotuner may choose
-    size_t part_max = 0;
-    for (int tpc : {1, 2, 4})
-        for (int m : {0, 1, 2, 4})
-            if (!tc_plan_pass1(c, tpc, m)) part_max = std::max(part_max, (size_t)p.nsplit1 * p.NP * p.rtot);
-    if (tc_plan_pass1(c, tpc0, 2) && tc_plan_pass1(c, 2, 2)) return set_err(&c, MDG_E_UNSUPPORTED, "tensor-core plan");
     p.mtiles = (ks.nrow + 127) / 128;
     p.nchunk2 = (ks.nrow + kRC - 1) / kRC;
     p.nst2 = kMaxSlot2;  // slot groups of the pass-2 ring: as many as fit
@@ -1306,6 +985,17 @@ int recip_tc_setup(Ctx& c) {
     p.smem2 = (int)p2_layout(p.KS, p.nchunk2 * kRC, p.nst2).total;
     if (p.smem2 > 227 * 1024)
         return set_err(&c, MDG_E_UNSUPPORTED, "k range too large for the tensor-core shared-memory tiles");
+    c.d_tc_atoms = (uint4*)dalloc(c, sizeof(uint4) * std::max(v.nmove, 1));
+    c.d_frc = (double*)dalloc(c, sizeof(double) * 3 * std::max(v.nmove, 1));
+    if (c.alloc_failed) return set_err(&c, MDG_E_CUDA, "out of device memory for the tensor-core reciprocal sum");
+    if (2 * p.NN > 128 || (double)v.nmove * ks.nk >= kGridWork) return recip_nu_setup(c);
+    tc_plan_pass1(c, 2);
+    // the partial-sum buffer is sized for the largest split the autotuner may choose
+    size_t part_max = 0;
+    for (int m : {0, 1, 4, 2}) {
+        tc_plan_pass1(c, m);
+        part_max = std::max(part_max, (size_t)p.nsplit1 * p.NP * p.rtot);
+    }
     // pass-2 row order: rows sorted by the K steps of their n range, so that a chunk of kRC rows
     // runs only the K steps its rows need (the n range shrinks towards the edge of the k sphere)
     {
@@ -1358,16 +1048,12 @@ int recip_tc_setup(Ctx& c) {
             MDG_CUDA(cudaMemset(p.rsc2, 0, sizeof(float) * nrp));
         }
     }
-    c.d_tc_atoms = (uint4*)dalloc(c, sizeof(uint4) * std::max(v.nmove, 1));
     c.d_tc_img = (unsigned char*)dalloc(c, std::max<size_t>(p.img_bytes, 16));
     c.d_tc_cmax = (float*)dalloc(c, sizeof(float) * 4);
     c.d_tc_part = (float*)dalloc(c, sizeof(float) * std::max<size_t>(part_max, 1));
     c.d_tc_cf = (float2*)dalloc(c, sizeof(float2) * std::max(ks.nk, 1));
-    c.d_frc = (double*)dalloc(c, sizeof(double) * 3 * std::max(v.nmove, 1));
     if (c.alloc_failed) return set_err(&c, MDG_E_CUDA, "out of device memory for the tensor-core reciprocal sum");
     MDG_CUDA(allow_max_smem(k_tc_sfac2));
-    MDG_CUDA(allow_max_smem(k_tc_sfac<4>));
-    MDG_CUDA(allow_max_smem(k_tc_sfac<2>));
     MDG_CUDA(allow_max_smem(k_tc_force));
     p.ready = true;
     return MDG_OK;
@@ -1378,17 +1064,14 @@ void recip_tc(Ctx& c) {
     KSet& ks = c.ks;
     const TcPlan& p = c.tcp;
     if (ks.nk == 0 || v.nmove == 0) return;
+    if (c.nu.ready) {
+        recip_nu(c);
+        return;
+    }
     TcDims d{p.KN, p.NN, p.NP, p.KS, ks.nrow, p.nchunk2, (float)ks.pipix, (float)ks.pipiy, (float)ks.pipiz, p.nst2};
     // c.d_tc_atoms was filled, and c.d_tc_cmax cleared, by the packing kernel of this evaluation
-    if (p.tpc1 == 1)
-        k_tc_sfac2<<<dim3(p.grid1x, p.nsplit1), kT1b, p.smem1, c.stream>>>(
-            v, c.d_tc_atoms, p.chunk1, ks.row, d, c.d_tc_part, p.rtot, p.G1, p.rowsc);
-    else if (p.tpc1 == 4)
-        k_tc_sfac<4><<<dim3(p.grid1x, p.nsplit1), P1<4>::kThreads, p.smem1, c.stream>>>(
-            v, c.d_tc_atoms, p.chunk1, ks.row, d, p.NM, p.KM, c.d_tc_part, p.rtot, (uint32_t)p.ncols1, p.rowsc);
-    else
-        k_tc_sfac<2><<<dim3(p.grid1x, p.nsplit1), P1<2>::kThreads, p.smem1, c.stream>>>(
-            v, c.d_tc_atoms, p.chunk1, ks.row, d, p.NM, p.KM, c.d_tc_part, p.rtot, (uint32_t)p.ncols1, p.rowsc);
+    k_tc_sfac2<<<dim3(p.grid1x, p.nsplit1), kT1b, p.smem1, c.stream>>>(v, c.d_tc_atoms, p.chunk1, ks.row, d,
+                                                                       c.d_tc_part, p.rtot, p.G1, p.rowsc);
     const long nred = (long)ks.nrow * p.NN;
     k_tc_sreduce<<<(int)((nred + 31) / 32), 32 * kRedG, 0, c.stream>>>(
         v, c.d_tc_part, p.nsplit1, p.rtot, d, ks.row, ks.row_nlen, ks.ak, ks.qw, ks.s, c.d_tc_cf, c.d_tc_cmax,
