@@ -263,7 +263,7 @@ int launch_force(Ctx& c, bool force_rebuild, bool reset_status, bool acc_clear =
         // the packing's close (dipole, rebuild decision) runs here, ahead of the list it decides
         if (packed) step_close_launch(c);
         else pack_close_launch(c);
-        const bool conc = v.nliqa == v.nmove && v.nwall > 0 && v.nheads > 0;
+        const bool conc = v.nliqa == v.nmove && v.nheads > 0;
         if (conc) {
             // third branch: the wall tail (positions only) while the list is checked and rebuilt,
             // then the head-wall loop once the list is there

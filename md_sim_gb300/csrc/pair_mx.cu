@@ -11,15 +11,24 @@
 //   F[a]   float4 j-side force accumulator, zeroed here
 //   tc[a]  uint4  fixed-point fractions of x, y, z and the charge, for the tensor-core reciprocal
 //                 sum of the same evaluation (recip_tc.cu)
-// k_pair_mx walks the same per-head half lists as the FP64 kernel (one warp per head): i-side
-// site forces in FP32 sums per lane (a lane holds ~n/32 partners), warp-reduced once per head;
-// j-side site forces per pair; both leave as one vector FP32 reduction (red.global.add.v4.f32)
-// per site into F, which k_merge_f adds into the FP64 forces (and clears) after the loops.
-// Energies per lane are compensated FP32 sums.  k_wall_mx does the head-wall loop
-// (src/forcem.f90:418-498) the same way over (head, segment) work items, with the wall reaction
-// sums of each item added into FP64 per lane.  The pair loops issue no FP64 instructions (the
-// FP64 pipe of GB300 is narrow).  k_pair_mx_batch and k_wall_mx_batch run the same loop bodies
-// over the heads of many systems at once (replica batches), one persistent launch each.
+// k_pair_mx walks the same per-head half lists as the FP64 kernel (one warp per head).  The lists hold
+// the skin's partners (28 % beyond the cutoff): a warp tests 32 at a time, appends those inside the
+// cutoff to a queue in shared memory, and evaluates the queue 32 at a time, so that no lane idles
+// through the nine site pairs.  i-side site forces are FP32 sums per lane (a lane holds ~n/32
+// partners), reduced once per head; j-side site forces per pair; both leave as one vector FP32
+// reduction (red.global.add.v4.f32) per site into F, which k_merge_f adds into the FP64 forces (and
+// clears) after the loops.  Energies per lane are compensated FP32 sums, kept apart for partners of
+// the first and of other site types: alternating partner types (the O and H heads of constrained
+// waters) would otherwise flush a lane's sums to shared memory at nearly every pair.  Two resident
+// blocks per SM walk all heads and load the next head's first partners ahead.  32,768 waters: 105 ->
+// 73 us (issue slots: 70.8 -> 58 M instructions; without the partners' reductions 70 us, so those are
+// not what bounds it; full lists, which need none, took 129 us); 14,739 constrained sites: 278 -> 52.
+// k_wall_mx does the head-wall loop (src/forcem.f90:418-498) the same way over (head, segment) work
+// items, with the wall reaction sums of each item added into FP64 per lane (14,739 constrained sites
+// between walls: 191 -> 37 us).  The pair loops issue no
+// FP64 instructions (the FP64 pipe of GB300 is narrow).  k_pair_mx_batch and k_wall_mx_batch run the
+// same loop bodies over the heads of many systems at once (replica batches), one persistent launch
+// each.
 #include <algorithm>
 
 #include "common.cuh"
@@ -32,7 +41,6 @@ namespace {
 
 constexpr int kWarps = 8;
 constexpr int kNT = kWarps * 32;
-constexpr int kWSeg = 64;  // wall partners per work item of the head-wall loop
 constexpr int kPackBlocks = 152 * 8;  // most blocks of the packing kernel
 static_assert(kPackBlocks <= kPackParts, "dipole shares");
 constexpr float kPf = (float)kP, kA1f = (float)kA1, kA2f = (float)kA2, kA3f = (float)kA3, kA4f = (float)kA4,
@@ -55,7 +63,7 @@ __device__ __forceinline__ float warp_sumf(float x) {
     return x;
 }
 
-// Energies of the current head type pair; flushed to shared FP64 sums when the pair type changes.
+// Energies of one pair type, summed per lane.
 struct EAcc {
     int ijt = -1;
     Kahan lj, qq;
@@ -71,10 +79,9 @@ __device__ __forceinline__ void e_flush(EAcc& e, double* s_e, int nijt) {
     e.qq = Kahan();
 }
 
-// End of the loops: lanes holding the warp's (largest) pair type reduce with shuffles in FP64 (a
+// All lanes of a warp: lanes holding the warp's (largest) pair type reduce with shuffles in FP64 (a
 // warp's total grows with the heads it took, and an FP32 reduction of it would round at that
-// size), one shared atomic per warp; lanes left with another type (mixed-type systems) flush one
-// by one.
+// size), one shared atomic per warp; lanes left with another type flush one by one.  Leaves e empty.
 __device__ __forceinline__ void e_final(EAcc& e, double* s_e, int nijt) {
     const int ij0 = __reduce_max_sync(0xffffffffu, e.ijt);
     if (ij0 < 0) return;
@@ -86,6 +93,7 @@ __device__ __forceinline__ void e_final(EAcc& e, double* s_e, int nijt) {
         atomicAdd(&s_e[nijt + ij0], qq);
     }
     if (!mine) e_flush(e, s_e, nijt);
+    e = EAcc();
 }
 
 __device__ __forceinline__ void e_add(EAcc& e, int ijt, float lj, float qq, double* s_e, int nijt) {
@@ -97,13 +105,43 @@ __device__ __forceinline__ void e_add(EAcc& e, int ijt, float lj, float qq, doub
     e.qq.add(qq);
 }
 
+// The approximate instructions without the code that __expf, rsqrtf and __fdividef add for subnormal
+// arguments and results (squared distances and erfc factors that far down are zero here).
+__device__ __forceinline__ float ex2_ftz(float x) {
+    float y;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rcp_ftz(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float rsqrt_ftz(float x) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+constexpr float kLog2e = 1.4426950408889634f;
+
 // Abramowitz-Stegun 7.1.26 erfc(alpha r) and the Ewald force factor (src/forcem.f90:334-340).
 __device__ __forceinline__ float erfc_as(float alfar, float* ff, float spii) {
-    const float t = __fdividef(1.0f, 1.0f + kPf * alfar);
-    const float exp2a = __expf(-alfar * alfar);
+    const float t = rcp_ftz(fmaf(kPf, alfar, 1.0f));
+    const float exp2a = ex2_ftz(kLog2e * (-alfar * alfar));
     const float erfx = ((((kA5f * t + kA4f) * t + kA3f) * t + kA2f) * t + kA1f) * t * exp2a;
     *ff = spii * alfar * exp2a + erfx;
     return erfx;
+}
+
+// One site pair at separation d with the charges' product q: adds the energy to e, returns f/r.
+__device__ __forceinline__ float site_pair(float dx, float dy, float dz, float q, float alfa, float spii, float& e) {
+    const float r2 = dx * dx + dy * dy + dz * dz;
+    const float ri = rsqrt_ftz(r2);
+    const float rr = r2 * ri;
+    const float au = q * ri;
+    float ff;
+    e += erfc_as(alfa * rr, &ff, spii) * au;
+    return ff * au * (ri * ri);
 }
 
 __device__ __forceinline__ void red_v4(float4* p, float a, float b, float c) {
@@ -199,7 +237,7 @@ __device__ __forceinline__ float vdw_term(const float* par, float rsqi, float ri
     if (vk == 2) {
         const float r6 = par[5] * (rsqi * rsqi * rsqi);
         const float rh = par[4];
-        const float aux = par[3] * __expf(-rij * rh);
+        const float aux = par[3] * ex2_ftz(kLog2e * (-rij * rh));
         *fij = aux * rh * rinv - 6.0f * rsqi * r6;
         return aux - r6;
     }
@@ -207,103 +245,214 @@ __device__ __forceinline__ float vdw_term(const float* par, float rsqi, float ri
     return 0.f;
 }
 
-// The head-head loop of one warp over the heads h0, h0 + hs, ... below v.nheads.
+// Sum over the warp of nine values with 14 shuffles (eight of them by halving: each step every lane
+// keeps half of its values, summed with its partner's); lane 4 k ends with value k < 8, lane 0 also
+// with value 8.  Returned: value 8 in lane 0's second component.
+__device__ __forceinline__ float2 warp_sum9(const float v[9]) {
+    const int lane = threadIdx.x & 31;
+    float a[4], b[2];
+    const bool u16 = lane & 16, u8 = lane & 8, u4 = lane & 4;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float keep = u16 ? v[k + 4] : v[k], send = u16 ? v[k] : v[k + 4];
+        a[k] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const float keep = u8 ? a[k + 2] : a[k], send = u8 ? a[k] : a[k + 2];
+        b[k] = keep + __shfl_xor_sync(0xffffffffu, send, 8);
+    }
+    float c = (u4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, u4 ? b[0] : b[1], 4);
+    c += __shfl_xor_sync(0xffffffffu, c, 2);
+    c += __shfl_xor_sync(0xffffffffu, c, 1);
+    return make_float2(c, warp_sumf(v[8]));
+}
+
+// A warp's site forces (fx, fy, fz of its nsi sites) summed and added to F[i..].
+__device__ __forceinline__ void add_sites(const Pk& pk, int i, int nsi, const float fx[3], const float fy[3],
+                                          const float fz[3]) {
+    const int lane = threadIdx.x & 31;
+    if (nsi == 3) {
+        const float v[9] = {fx[0], fy[0], fz[0], fx[1], fy[1], fz[1], fx[2], fy[2], fz[2]};
+        const float2 s = warp_sum9(v);
+        // lanes 0, 4, 8: the sites' sums, gathered from lanes 4 (3 site + component)
+        const int site = lane >> 2;
+        const float x = __shfl_sync(0xffffffffu, s.x, 4 * min(3 * site, 7));
+        const float y = __shfl_sync(0xffffffffu, s.x, 4 * min(3 * site + 1, 7));
+        const float z = __shfl_sync(0xffffffffu, s.x, 4 * min(3 * site + 2, 7));
+        if ((lane & 3) == 0 && site < 3)
+            red_v4(&pk.F[i + site], x, y, site == 2 ? s.y : z);
+        return;
+    }
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+        if (a >= nsi) break;
+        const float x = warp_sumf(fx[a]), y = warp_sumf(fy[a]), z = warp_sumf(fz[a]);
+        if (lane == 0) red_v4(&pk.F[i + a], x, y, z);
+    }
+}
+
+// A warp's partners inside the cutoff: separation, index and the record's type word, a ring of 64.
+struct QueueMem {
+    float4 q[64];
+    unsigned w[64];
+};
+struct Queue {
+    QueueMem* m;
+    int head = 0, n = 0;
+    __device__ __forceinline__ void push(bool in, float dx, float dy, float dz, int j, unsigned w) {
+        const unsigned b = __ballot_sync(0xffffffffu, in), lt = (1u << (threadIdx.x & 31)) - 1u;
+        const int k = (head + n + __popc(b & lt)) & 63;
+        if (in) {
+            m->q[k] = make_float4(dx, dy, dz, __int_as_float(j));
+            m->w[k] = w;
+        }
+        n += __popc(b);
+        __syncwarp();
+    }
+    // this lane's entry of the oldest 32 (any entry where there are fewer: the caller masks it)
+    __device__ __forceinline__ float4 front(unsigned& w) const {
+        const int k = (head + (threadIdx.x & 31)) & 63;
+        w = m->w[k];
+        return m->q[k];
+    }
+    __device__ __forceinline__ void pop() {
+        head = (head + 32) & 63;
+        n = max(n - 32, 0);
+        __syncwarp();
+    }
+};
+
+// The head-head loop of one warp over the heads h0, h0 + hs, ... below v.nheads; e: energies with
+// partners of the first site type and of the others.
 template <int ZPER>
-__device__ __forceinline__ void pair_heads(const View& v, const Pk& pk, const Tables& T, int h0, int hs, EAcc& e,
-                                           double* s_e) {
+__device__ __forceinline__ void pair_heads(const View& v, const Pk& pk, const Tables& T, int h0, int hs, EAcc e[2],
+                                           double* s_e, QueueMem* queue) {
     const int lane = threadIdx.x & 31;
     const float alfa = pk.alfa, spii = pk.spii, facq = pk.facq, rcutsq = pk.rcutsq;
+    int it_last = -1;
+    // the next head's atom, partner count and first partners load while this head is worked on
+    int i_next = h0 < v.nheads ? v.head_atom[h0] : 0, n_next = h0 < v.nheads ? v.nbcnt[h0] : 0;
+    int j_next = h0 < v.nheads && lane < n_next ? v.nb[(size_t)h0 * v.maxnb + lane] : 0;
     for (int h = h0; h < v.nheads; h += hs) {
-        const int i = v.head_atom[h];
+        const int i = i_next, n = n_next;
+        int j1 = j_next;
         const uint4 pi = pk.P[i];
+        uint4 p1 = lane < n ? pk.P[j1] : make_uint4(0u, 0u, 0u, 0u);
+        const int* nb = v.nb + (size_t)h * v.maxnb;
+        int j2 = lane + 32 < n ? nb[lane + 32] : 0;
+        if (h + hs < v.nheads) {
+            i_next = v.head_atom[h + hs];
+            n_next = v.nbcnt[h + hs];
+            if (lane < v.maxnb) j_next = v.nb[(size_t)(h + hs) * v.maxnb + lane];
+        }
         const int it = (int)(pi.w & 0x7fffffffu);
         const int nsi_i = T.nsi[it];
+        if (it != it_last && it_last >= 0) {
+            e_final(e[0], s_e, v.nijt);
+            e_final(e[1], s_e, v.nijt);
+        }
+        it_last = it;
         const float zli = ZPER ? 0.f : pk.zlo[i];
         float4 si[3];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) si[a] = a < nsi_i ? pk.Q[i + a] : make_float4(0.f, 0.f, 0.f, 0.f);
-        // i-side sums: a lane holds about n / 32 partners of the head, few enough for plain FP32
-        float fix[3] = {0, 0, 0}, fiy[3] = {0, 0, 0}, fiz[3] = {0, 0, 0};
-        const int n = v.nbcnt[h];
-        const int* nb = v.nb + (size_t)h * v.maxnb;
-        // software pipeline over the lane's partners: the record of the next partner and the
-        // index of the one after are loaded while this one is computed (one warp per head and
-        // one block per SM leave few warps to hide the dependent gathers otherwise)
-        int j1 = lane < n ? nb[lane] : 0;
-        int j2 = lane + 32 < n ? nb[lane + 32] : 0;
-        uint4 p1 = lane < n ? pk.P[j1] : make_uint4(0u, 0u, 0u, 0u);
-        for (int k = lane; k < n; k += 32) {
-            const int j = j1;
-            const uint4 pj = p1;
-            j1 = j2;
-            if (k + 32 < n) p1 = pk.P[j1];
-            if (k + 64 < n) j2 = nb[k + 64];
-            const int jt = (int)(pj.w & 0x7fffffffu);
-            const int nsi_j = T.nsi[jt];
-            float4 sj[3];  // the partner's sites, requested before the distance test
-#pragma unroll
-            for (int b = 0; b < 3; ++b) sj[b] = b < nsi_j ? pk.Q[j + b] : make_float4(0.f, 0.f, 0.f, 0.f);
-            float xio, yio, zio;
-            head_vec<ZPER>(pi, zli, pj, pk, j, xio, yio, zio);
-            const float rsq = xio * xio + yio * yio + zio * zio;
-            if (rsq > rcutsq) continue;
-            const int ijt = T.ijt[it * v.nit + jt];
-            const float rinv = rsqrtf(rsq);
-            const float rsqi = rinv * rinv;
-            const float rij = rsq * rinv;
-            float fij;
-            const float elj = vdw_term(T.par + 6 * ijt, rsqi, rinv, rij, &fij);
-            float ff;
-            const float auxq = facq * si[0].w * sj[0].w * rinv;
-            float eqq = erfc_as(alfa * rij, &ff, spii) * auxq;
-            fij = fij + ff * auxq * rsqi;
-            float fjx[3], fjy[3], fjz[3];
-            fix[0] = fmaf(xio, fij, fix[0]); fiy[0] = fmaf(yio, fij, fiy[0]); fiz[0] = fmaf(zio, fij, fiz[0]);
-            fjx[0] = -xio * fij; fjy[0] = -yio * fij; fjz[0] = -zio * fij;
-#pragma unroll
-            for (int b = 1; b < 3; ++b) fjx[b] = fjy[b] = fjz[b] = 0.f;
-#pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                if (a >= nsi_i) break;
-                const float xa = xio + si[a].x, ya = yio + si[a].y, za = zio + si[a].z;
-                const float qx = facq * si[a].w;
-#pragma unroll
-                for (int b = 0; b < 3; ++b) {
-                    if (b >= nsi_j) break;
-                    if (a == 0 && b == 0) continue;
-                    const float xd = xa - sj[b].x, yd = ya - sj[b].y, zd = za - sj[b].z;
-                    const float r2 = xd * xd + yd * yd + zd * zd;
-                    const float ri = rsqrtf(r2);
-                    const float rr = r2 * ri;
-                    const float au = qx * sj[b].w * ri;
-                    float fq;
-                    eqq += erfc_as(alfa * rr, &fq, spii) * au;
-                    const float fs = fq * au * (ri * ri);
-                    fix[a] = fmaf(xd, fs, fix[a]); fiy[a] = fmaf(yd, fs, fiy[a]); fiz[a] = fmaf(zd, fs, fiz[a]);
-                    fjx[b] -= xd * fs; fjy[b] -= yd * fs; fjz[b] -= zd * fs;
-                }
-            }
-#pragma unroll
-            for (int b = 0; b < 3; ++b) {
-                if (b >= nsi_j) break;
-                red_v4(&pk.F[j + b], fjx[b], fjy[b], fjz[b]);
-            }
-            e_add(e, ijt, elj, eqq, s_e, v.nijt);
-        }
-#pragma unroll
         for (int a = 0; a < 3; ++a) {
-            if (a >= nsi_i) break;
-            const float sx = warp_sumf(fix[a]), sy = warp_sumf(fiy[a]), sz = warp_sumf(fiz[a]);
-            if (lane == 0) red_v4(&pk.F[i + a], sx, sy, sz);
+            si[a] = a < nsi_i ? pk.Q[i + a] : make_float4(0.f, 0.f, 0.f, 0.f);
+            si[a].w *= facq;
         }
+        // sums of this head: a lane takes about n / 32 partners, few enough for plain FP32
+        float fix[3] = {0, 0, 0}, fiy[3] = {0, 0, 0}, fiz[3] = {0, 0, 0};
+        Queue Q{queue};
+        auto evaluate = [&](int m) {
+            unsigned wj;
+            const float4 d = Q.front(wj);
+            const bool on = lane < m;
+            const int j = __float_as_int(d.w);
+            const int jt = on ? (int)(wj & 0x7fffffffu) : it;
+            const int nsi_j = T.nsi[jt];
+            const bool three = nsi_i == 3 && __all_sync(0xffffffffu, nsi_j == 3);
+            if (on) {
+                const float4* qj = pk.Q + j;
+                const float4 s0 = qj[0];
+                const float rsq = d.x * d.x + d.y * d.y + d.z * d.z;
+                const int ijt = T.ijt[it * v.nit + jt];
+                const float rinv = rsqrt_ftz(rsq);
+                const float rsqi = rinv * rinv;
+                const float rij = rsq * rinv;
+                float fij, ff;
+                const float elj = vdw_term(T.par + 6 * ijt, rsqi, rinv, rij, &fij);
+                const float auxq = si[0].w * s0.w * rinv;
+                float eqq = erfc_as(alfa * rij, &ff, spii) * auxq;
+                fij = fij + ff * auxq * rsqi;
+                float fjx[3], fjy[3], fjz[3];
+                fjx[0] = d.x * fij;
+                fjy[0] = d.y * fij;
+                fjz[0] = d.z * fij;
+                fix[0] += fjx[0];
+                fiy[0] += fjy[0];
+                fiz[0] += fjz[0];
+                fjx[1] = fjy[1] = fjz[1] = fjx[2] = fjy[2] = fjz[2] = 0.f;
+                auto pair = [&](int a, int b, const float4& s) {
+                    const float xd = (d.x + si[a].x) - s.x, yd = (d.y + si[a].y) - s.y, zd = (d.z + si[a].z) - s.z;
+                    const float f = site_pair(xd, yd, zd, si[a].w * s.w, alfa, spii, eqq);
+                    fix[a] = fmaf(xd, f, fix[a]);
+                    fiy[a] = fmaf(yd, f, fiy[a]);
+                    fiz[a] = fmaf(zd, f, fiz[a]);
+                    fjx[b] = fmaf(xd, f, fjx[b]);
+                    fjy[b] = fmaf(yd, f, fjy[b]);
+                    fjz[b] = fmaf(zd, f, fjz[b]);
+                };
+                if (three) {
+                    const float4 s1 = qj[1], s2 = qj[2];
+                    pair(1, 0, s0);
+                    pair(2, 0, s0);
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) {
+                        pair(a, 1, s1);
+                        pair(a, 2, s2);
+                    }
+                    red_v4(&pk.F[j + 1], -fjx[1], -fjy[1], -fjz[1]);
+                    red_v4(&pk.F[j + 2], -fjx[2], -fjy[2], -fjz[2]);
+                } else {
+#pragma unroll
+                    for (int b = 0; b < 3; ++b) {
+                        if (b >= nsi_j) break;
+                        const float4 s = b ? qj[b] : s0;
+#pragma unroll
+                        for (int a = 0; a < 3; ++a)
+                            if (a < nsi_i && a + b > 0) pair(a, b, s);
+                        if (b) red_v4(&pk.F[j + b], -fjx[b], -fjy[b], -fjz[b]);
+                    }
+                }
+                red_v4(&pk.F[j], -fjx[0], -fjy[0], -fjz[0]);
+                if (jt == 0) e_add(e[0], ijt, elj, eqq, s_e, v.nijt);
+                else e_add(e[1], ijt, elj, eqq, s_e, v.nijt);
+            }
+            Q.pop();
+        };
+        // the record of the next partner and the index of the one after load while this one is tested
+        for (int k0 = 0; k0 < n || Q.n > 0;) {
+            for (; k0 < n && Q.n < 32; k0 += 32) {
+                const int k = k0 + lane, j = j1;
+                const uint4 pj = p1;
+                j1 = j2;
+                if (k + 32 < n) p1 = pk.P[j1];
+                if (k + 64 < n) j2 = nb[k + 64];
+                float dx, dy, dz;
+                head_vec<ZPER>(pi, zli, pj, pk, j, dx, dy, dz);
+                Q.push(k < n && dx * dx + dy * dy + dz * dz <= rcutsq, dx, dy, dz, j, pj.w);
+            }
+            if (Q.n > 0) evaluate(min(Q.n, 32));
+        }
+        add_sites(pk, i, nsi_i, fix, fiy, fiz);
     }
 }
 
 // The block's energy sums into the system's accumulators (all threads; the shared sums are free
 // for the next system's tables afterwards).
-__device__ __forceinline__ void pair_flush(const View& v, EAcc& e, double* s_e) {
-    e_final(e, s_e, v.nijt);
-    e = EAcc();
+__device__ __forceinline__ void pair_flush(const View& v, EAcc e[2], double* s_e) {
+    e_final(e[0], s_e, v.nijt);
+    e_final(e[1], s_e, v.nijt);
     __syncthreads();
     for (int k = threadIdx.x; k < 2 * v.nijt; k += blockDim.x)
         if (s_e[k] != 0.0) atomicAdd(&v.acc[k], s_e[k]);
@@ -311,19 +460,21 @@ __device__ __forceinline__ void pair_flush(const View& v, EAcc& e, double* s_e) 
 }
 
 template <int ZPER>
-__global__ void __launch_bounds__(kNT) k_pair_mx(View v, Pk pk) {
+__global__ void __launch_bounds__(kNT, 2) k_pair_mx(View v, Pk pk) {
     extern __shared__ double s_e[];
+    __shared__ QueueMem queue[kWarps];
     const Tables T = load_tables(v, pk, s_e, 0);
-    EAcc e;
-    pair_heads<ZPER>(v, pk, T, blockIdx.x * kWarps + (threadIdx.x >> 5), gridDim.x * kWarps, e, s_e);
+    EAcc e[2];
+    const int warp = threadIdx.x >> 5;
+    pair_heads<ZPER>(v, pk, T, blockIdx.x * kWarps + warp, gridDim.x * kWarps, e, s_e, &queue[warp]);
     pair_flush(v, e, s_e);
 }
 
 // Head-wall work units of a system: (head, segment of seg wall partners), so that the few heads
-// next to a wall with hundreds of partners are shared by several warps (seg = kWSeg for one
-// system; a batch of systems has parallelism to spare and takes kWSegBatch, which halves the per-unit
-// work of the head's loads and reductions).  A lane sees at most seg / 32 partners per unit, so its
-// FP32 sums within a unit are short and need no compensation.
+// next to a wall with hundreds of partners are shared by several warps (seg by the system's heads, see
+// walls_mixed; a batch of systems has parallelism to spare and takes kWSegBatch, which halves the
+// per-unit work of the head's loads and reductions).  A lane sees at most seg / 32 partners per unit,
+// so its FP32 sums within a unit are short and need no compensation.
 constexpr int kWSegBatch = 256;
 __host__ __device__ __forceinline__ long wall_units(const View& v, int seg) {
     return (long)v.nheads * ((v.maxwnb + seg - 1) / seg);
@@ -341,91 +492,106 @@ struct WAcc {
 // The head-wall loop of one warp over the units u0, u0 + us, ... below wall_units(v, seg).
 template <int ZPER>
 __device__ __forceinline__ void wall_heads(const View& v, const Pk& pk, const Tables& T, long u0, long us, int seg,
-                                           WAcc& w) {
+                                           WAcc& w, QueueMem* queue) {
     const int lane = threadIdx.x & 31;
     const float alfa = pk.alfa, spii = pk.spii, facq = pk.facq, rcutsq = pk.rcutsq;
     const int wt0 = v.nit - 2;
     const int nseg = (v.maxwnb + seg - 1) / seg;
-    const long nitems = (long)v.nheads * nseg;
-    for (long item = u0; item < nitems; item += us) {
-        const int h = (int)(item / nseg), sg = (int)(item % nseg);
+    // units in order of segments, then heads: a stride that is a multiple of 3 keeps a warp on heads of
+    // one type where molecules have three heads each (constrained waters)
+    int it_last = -1, sg = (int)(u0 / v.nheads);
+    long hl = u0 % v.nheads;
+    for (; sg < nseg; hl += us) {
+        while (hl >= v.nheads && sg < nseg) {
+            hl -= v.nheads;
+            ++sg;
+        }
+        if (sg >= nseg) break;
+        const int h = (int)hl;
         const int n = min(v.wnbcnt[h], (sg + 1) * seg);
         if (sg * seg >= n) continue;
         const int i = v.head_atom[h];
         const uint4 pi = pk.P[i];
         const int it = (int)(pi.w & 0x7fffffffu);
         const int nsi_i = T.nsi[it];
+        if (it != it_last && it_last >= 0) {
+            e_final(w.ew[0], w.s_e, v.nijt);
+            e_final(w.ew[1], w.s_e, v.nijt);
+        }
+        it_last = it;
         const bool book = (it + 1) <= v.nltype;
         const float zli = ZPER ? 0.f : pk.zlo[i];
         float4 si[3];
 #pragma unroll
-        for (int a = 0; a < 3; ++a) si[a] = a < nsi_i ? pk.Q[i + a] : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int a = 0; a < 3; ++a) {
+            si[a] = a < nsi_i ? pk.Q[i + a] : make_float4(0.f, 0.f, 0.f, 0.f);
+            si[a].w *= facq;
+        }
         float fix[3] = {0, 0, 0}, fiy[3] = {0, 0, 0}, fiz[3] = {0, 0, 0};
         // wall reaction sums of this unit, lower wall (z < 0) in l*, upper in u*: plain registers
         // updated through selects (x - 0 is exact, so each sum is what a per-wall array gives)
         float lx = 0.f, ly = 0.f, lz = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
-        const int* nb = v.wnb + (size_t)h * v.maxwnb;
-        const float* qw = reinterpret_cast<const float*>(pk.Q) + 3;  // charges: Q[j].w = qw[4 j]
-        // software pipeline as in the head-head loop: the next partner's record and charge and
-        // the index after it load while this partner is computed
-        const int k0 = sg * seg + lane;
-        int j1 = k0 < n ? nb[k0] : 0;
-        int j2 = k0 + 32 < n ? nb[k0 + 32] : 0;
-        uint4 p1 = k0 < n ? pk.P[j1] : make_uint4(0u, 0u, 0u, 0u);
-        float q1 = k0 < n ? qw[4 * (size_t)j1] : 0.f;
-        for (int k = k0; k < n; k += 32) {
-            const int j = j1;
-            const uint4 pj = p1;
-            const float qj = q1;
-            j1 = j2;
-            if (k + 32 < n) {
-                p1 = pk.P[j1];
-                q1 = qw[4 * (size_t)j1];
-            }
-            if (k + 64 < n) j2 = nb[k + 64];
-            float xi, yi, zi;
-            head_vec<ZPER>(pi, zli, pj, pk, j, xi, yi, zi);
-            const float rsq = xi * xi + yi * yi + zi * zi;
-            if (rsq > rcutsq) continue;
-            const bool lower = (pj.w & 0x80000000u) != 0;
-            const int jt = (int)(pj.w & 0x7fffffffu);
-            const int ijt = T.ijt[it * v.nit + jt];
-            const float rinv = rsqrtf(rsq);
-            float fij;
-            const float elj = vdw_term(T.par + 6 * ijt, rinv * rinv, rinv, rsq * rinv, &fij);
-            const float qx = facq * qj;
-            float eqq = 0.f;
+        Queue Q{queue};
+        auto evaluate = [&](int m) {
+            unsigned pw;
+            const float4 d = Q.front(pw);
+            if (lane < m) {
+                const int j = __float_as_int(d.w);
+                const float qj = pk.Q[j].w;
+                const bool lower = (pw & 0x80000000u) != 0;
+                const int jt = (int)(pw & 0x7fffffffu);
+                const int ijt = T.ijt[it * v.nit + jt];
+                const float rsq = d.x * d.x + d.y * d.y + d.z * d.z;
+                const float rinv = rsqrt_ftz(rsq);
+                float fij;
+                const float elj = vdw_term(T.par + 6 * ijt, rinv * rinv, rinv, rsq * rinv, &fij);
+                float eqq = 0.f;
 #pragma unroll
-            for (int a = 0; a < 3; ++a) {
-                if (a >= nsi_i) break;
-                const float xd = xi + si[a].x, yd = yi + si[a].y, zd = zi + si[a].z;
-                const float r2 = xd * xd + yd * yd + zd * zd;
-                const float ri = rsqrtf(r2);
-                const float rr = r2 * ri;
-                const float au = qx * si[a].w * ri;
-                float fq;
-                eqq += erfc_as(alfa * rr, &fq, spii) * au;
-                fij = fij + fq * au * (ri * ri);
-                fix[a] = fmaf(xd, fij, fix[a]);
-                fiy[a] = fmaf(yd, fij, fiy[a]);
-                fiz[a] = fmaf(zd, fij, fiz[a]);
-                if (book) {
-                    const float sx = xd * fij, sy = yd * fij, sz = zd * fij;
-                    lx -= lower ? sx : 0.f; ly -= lower ? sy : 0.f; lz -= lower ? sz : 0.f;
-                    ux -= lower ? 0.f : sx; uy -= lower ? 0.f : sy; uz -= lower ? 0.f : sz;
+                for (int a = 0; a < 3; ++a) {
+                    if (a >= nsi_i) break;
+                    const float xd = d.x + si[a].x, yd = d.y + si[a].y, zd = d.z + si[a].z;
+                    const float r2 = xd * xd + yd * yd + zd * zd;
+                    const float ri = rsqrt_ftz(r2);
+                    const float au = qj * si[a].w * ri;
+                    float fq;
+                    eqq += erfc_as(alfa * (r2 * ri), &fq, spii) * au;
+                    fij = fij + fq * au * (ri * ri);
+                    fix[a] = fmaf(xd, fij, fix[a]);
+                    fiy[a] = fmaf(yd, fij, fiy[a]);
+                    fiz[a] = fmaf(zd, fij, fiz[a]);
+                    if (book) {
+                        const float sx = xd * fij, sy = yd * fij, sz = zd * fij;
+                        lx -= lower ? sx : 0.f; ly -= lower ? sy : 0.f; lz -= lower ? sz : 0.f;
+                        ux -= lower ? 0.f : sx; uy -= lower ? 0.f : sy; uz -= lower ? 0.f : sz;
+                    }
+                    fij = 0.f;
                 }
-                fij = 0.f;
+                // energy sums per wall site type (the last two site types)
+                if (jt > wt0) e_add(w.ew[1], ijt, elj, eqq, w.s_e, v.nijt);
+                else e_add(w.ew[0], ijt, elj, eqq, w.s_e, v.nijt);
             }
-            // energy sums per wall site type (the last two site types)
-            if (jt > wt0) e_add(w.ew[1], ijt, elj, eqq, w.s_e, v.nijt);
-            else e_add(w.ew[0], ijt, elj, eqq, w.s_e, v.nijt);
+            Q.pop();
+        };
+        const int* nb = v.wnb + (size_t)h * v.maxwnb;
+        // the next partner's record and the index after it load while this partner is tested
+        const int s0 = sg * seg;
+        int j1 = s0 + lane < n ? nb[s0 + lane] : 0;
+        int j2 = s0 + lane + 32 < n ? nb[s0 + lane + 32] : 0;
+        uint4 p1 = s0 + lane < n ? pk.P[j1] : make_uint4(0u, 0u, 0u, 0u);
+        for (int k0 = s0; k0 < n || Q.n > 0;) {
+            for (; k0 < n && Q.n < 32; k0 += 32) {
+                const int k = k0 + lane, j = j1;
+                const uint4 pj = p1;
+                j1 = j2;
+                if (k + 32 < n) p1 = pk.P[j1];
+                if (k + 64 < n) j2 = nb[k + 64];
+                float dx, dy, dz;
+                head_vec<ZPER>(pi, zli, pj, pk, j, dx, dy, dz);
+                Q.push(k < n && dx * dx + dy * dy + dz * dz <= rcutsq, dx, dy, dz, j, pj.w);
+            }
+            if (Q.n > 0) evaluate(min(Q.n, 32));
         }
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            if (a >= nsi_i) break;
-            const float sx = warp_sumf(fix[a]), sy = warp_sumf(fiy[a]), sz = warp_sumf(fiz[a]);
-            if (lane == 0) red_v4(&pk.F[i + a], sx, sy, sz);
-        }
+        add_sites(pk, i, nsi_i, fix, fiy, fiz);
         if (book) {
             w.ws[0] += (double)lx; w.ws[1] += (double)ly; w.ws[2] += (double)lz;
             w.ws[3] += (double)ux; w.ws[4] += (double)uy; w.ws[5] += (double)uz;
@@ -438,8 +604,6 @@ __device__ __forceinline__ void wall_flush(const View& v, WAcc& w) {
     double* s_e = w.s_e;
     e_final(w.ew[0], s_e, v.nijt);
     e_final(w.ew[1], s_e, v.nijt);
-    w.ew[0] = EAcc();
-    w.ew[1] = EAcc();
 #pragma unroll
     for (int k = 0; k < 6; ++k) {
         const double s = warp_sum(w.ws[k]);
@@ -458,12 +622,14 @@ __device__ __forceinline__ void wall_flush(const View& v, WAcc& w) {
 }
 
 template <int ZPER>
-__global__ void __launch_bounds__(kNT) k_wall_mx(View v, Pk pk) {
+__global__ void __launch_bounds__(kNT) k_wall_mx(View v, Pk pk, int seg) {
     extern __shared__ double s_e[];
+    __shared__ QueueMem queue[kWarps];
     const Tables T = load_tables(v, pk, s_e, 6);
     WAcc w;
     w.s_e = s_e;
-    wall_heads<ZPER>(v, pk, T, blockIdx.x * kWarps + (threadIdx.x >> 5), (long)gridDim.x * kWarps, kWSeg, w);
+    const int warp = threadIdx.x >> 5;
+    wall_heads<ZPER>(v, pk, T, blockIdx.x * kWarps + warp, (long)gridDim.x * kWarps, seg, w, &queue[warp]);
     wall_flush(v, w);
 }
 
@@ -516,9 +682,10 @@ __global__ void __launch_bounds__(kNT) k_pair_mx_batch(const RsRep* __restrict__
     const int b0 = (int)((long)nitems * blockIdx.x / gridDim.x);
     const int b1 = (int)((long)nitems * (blockIdx.x + 1) / gridDim.x);
     const int warp = threadIdx.x >> 5;
+    __shared__ QueueMem queue[kWarps];
     int r = -1;
     Tables T{};
-    EAcc e;
+    EAcc e[2];
     for (int it = b0; it < b1; ++it) {
         const int rn = rep_of(first, nrep, it, r);
         if (rn != r) {
@@ -528,7 +695,7 @@ __global__ void __launch_bounds__(kNT) k_pair_mx_batch(const RsRep* __restrict__
             r = rn;
         }
         const int n = first[r + 1] - first[r], k = it - first[r];
-        pair_heads<ZPER>(sr.v, sr.pk, T, k + n * warp, n * kWarps, e, s_e);
+        pair_heads<ZPER>(sr.v, sr.pk, T, k + n * warp, n * kWarps, e, s_e, &queue[warp]);
     }
     if (r >= 0) pair_flush(sr.v, e, s_e);
 }
@@ -543,6 +710,7 @@ __global__ void __launch_bounds__(kNT) k_wall_mx_batch(const RsRep* __restrict__
     const int b0 = (int)((long)nitems * blockIdx.x / gridDim.x);
     const int b1 = (int)((long)nitems * (blockIdx.x + 1) / gridDim.x);
     const int warp = threadIdx.x >> 5;
+    __shared__ QueueMem queue[kWarps];
     int r = -1;
     Tables T{};
     WAcc w;
@@ -556,7 +724,7 @@ __global__ void __launch_bounds__(kNT) k_wall_mx_batch(const RsRep* __restrict__
             r = rn;
         }
         const long n = first[r + 1] - first[r], k = it - first[r];
-        wall_heads<ZPER>(sr.v, sr.pk, T, k + n * warp, n * kWarps, kWSegBatch, w);
+        wall_heads<ZPER>(sr.v, sr.pk, T, k + n * warp, n * kWarps, kWSegBatch, w, &queue[warp]);
     }
     if (r >= 0) wall_flush(sr.v, w);
 }
@@ -582,9 +750,14 @@ __global__ void k_merge_f(View v, Pk pk, const double* __restrict__ frc, double 
     }
 }
 
-int blocks(const Ctx& c, int nheads) {
-    const int b = std::max(1, std::min((nheads + kWarps - 1) / kWarps, 152 * 16));
-    return c.pair_blocks > 0 ? std::min(b, c.pair_blocks) : b;
+// Blocks of the real-space loops: one warp per head, at most the resident ones (two per SM), so that a
+// block's tables, first loads and energy sums are paid once (32,768 waters: 2,432 blocks 102 us, 304
+// 77 us); a multiple of 3, which keeps a warp on heads of one
+// type where molecules have three heads each (constrained waters: the energy sums flush at a change).
+int blocks(const Ctx& c, int nheads, int most) {
+    int b = (nheads + kWarps - 1) / kWarps;
+    b = std::min(b, c.pair_blocks > 0 ? c.pair_blocks : most);
+    return std::max(1, b >= 150 ? b / 3 * 3 : b);
 }
 
 size_t table_smem(const View& v, int nextra) {
@@ -645,11 +818,10 @@ void merge_mixed(Ctx& c, const double* frc, bool dipole) {
 void pairs_mixed(Ctx& c, bool merge) {
     const View& v = c.v;
     if (v.nheads == 0) return;
-    // Beside the head-wall loop and the reciprocal sum (merge false: the concurrent form) the
-    // head-head loop has time to spare; it keeps to one block per SM, leaving room for the
-    // reciprocal branch's kernels (measured on the slab: its reduction 18 -> 13 us, the step 2 %).
-    int nb = blocks(c, v.nheads);
-    if (!merge) nb = std::min(nb, 152);
+    // Beside the head-wall loop and the reciprocal sum the head-head loop has time to spare; it keeps
+    // to one block per SM, leaving room for the reciprocal branch's kernels (slab of 2,048 waters, 20
+    // steps: 2.04 ms, with two blocks of either loop 2.20).
+    const int nb = blocks(c, v.nheads, !merge && v.nwall > 0 ? 152 : 304);
     if (c.pk.zper) k_pair_mx<1><<<nb, kNT, table_smem(v, 0), c.stream>>>(v, c.pk);
     else k_pair_mx<0><<<nb, kNT, table_smem(v, 0), c.stream>>>(v, c.pk);
     if (merge) merge_mixed(c, nullptr, false);
@@ -658,12 +830,12 @@ void pairs_mixed(Ctx& c, bool merge) {
 void walls_mixed(Ctx& c, bool concurrent) {
     const View& v = c.v;
     if (v.nheads == 0 || v.nwall == 0) return;
-    // beside the head-head loop and the reciprocal sum, one block per SM, as the head-head loop
-    // (measured on the slab: the reciprocal reduction gets the room, the step 2 % shorter)
-    int nb = blocks(c, v.nheads);
-    if (concurrent) nb = std::min(nb, 152);
-    if (c.pk.zper) k_wall_mx<1><<<nb, kNT, table_smem(v, 6), c.stream>>>(v, c.pk);
-    else k_wall_mx<0><<<nb, kNT, table_smem(v, 6), c.stream>>>(v, c.pk);
+    const int nb = blocks(c, v.nheads, concurrent ? 152 : 304);
+    // fewer, longer units where the heads alone fill the GPU (14,739 heads: units of 64 partners 121 us,
+    // 128 87, 256 63; 2,048 heads: 26, 24, 29)
+    const int seg = v.nheads >= 8192 ? 256 : 128;
+    if (c.pk.zper) k_wall_mx<1><<<nb, kNT, table_smem(v, 6), c.stream>>>(v, c.pk, seg);
+    else k_wall_mx<0><<<nb, kNT, table_smem(v, 6), c.stream>>>(v, c.pk, seg);
 }
 
 // ---- replica batches: host side ------------------------------------------------------------
