@@ -235,7 +235,7 @@ struct Ctx {
     float4* d_wpos = nullptr;     // wrapped wall positions sorted by cell
     double4* d_hpos = nullptr;    // wrapped head positions in head order
     // SHAKE
-    int ncons = 0, ncmax = 0, shake_seq = 0, maxit = 10;
+    int ncons = 0, ncmax = 0, shake_seq = 0, shake_tri = 0, maxit = 10;
     double tol2 = 1e-8, rptol = 0.85;
     int* d_cons = nullptr;        // ncons * 3 * 2 atom indices (0-based), -1 unused
     double* d_clen2 = nullptr;    // ncons * 3 squared lengths
