@@ -61,6 +61,7 @@ struct View {
     const int* ijt;            // nit*nit, 0-based pair index, [it*nit + jt]
     const int* vdw;            // nijt
     const double *eps, *sig, *aa, *rhoi, *cc;
+    const double2* etab = nullptr;  // Ewald pair functions (erfc_table.cuh)
     // forces
     double *fx, *fy, *fz;      // nmove
     // heads and lists
@@ -310,6 +311,7 @@ int ls_batch_setup(LsBatch& lb, const std::vector<Ctx*>& cs, std::string& err);
 void ls_batch_launch(const LsBatch& lb, cudaStream_t st);
 void ls_batch_free(LsBatch& lb);
 // pair.cu
+int pair_setup(Ctx& c);
 void pair_forces_fp64(Ctx& c);
 void wall_forces_fp64(Ctx& c);
 void surf_partition(Ctx& c);

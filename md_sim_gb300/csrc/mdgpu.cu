@@ -571,7 +571,9 @@ int mdg_create(const mdg_sysdesc* s, const mdg_params* p, const double* x0, cons
     lr_tables(c, s, p->rcut, lr);
     c.d_lr = upload(c, lr);
     c.uself = self_energy(s, x0, y0, z0, v.alfa, v.facq, v.spii);
-    int rc = recip_setup(c, p->kmax, x0, y0, z0);
+    int rc = pair_setup(c);
+    if (rc) return bail(rc);
+    rc = recip_setup(c, p->kmax, x0, y0, z0);
     if (rc) return bail(rc);
     if (c.precision == MDG_MIXED) {
         rc = recip_tc_setup(c);
