@@ -105,6 +105,7 @@ struct KSet {
     int* witem_row = nullptr;     // k_sfac work items: row
     int* witem_n = nullptr;       //                    first entry | entries << 16
     int nwork = 0;
+    int nent = 0;                 // entries (recip.cu)
     std::vector<int4> h_row;      // host copies of row and row_nlen
     std::vector<int> h_nlen;
 };
@@ -257,6 +258,9 @@ struct Ctx {
     std::vector<int64_t> h_moltypen, h_nt, h_ns, h_itype;  // molecule types and site types (cfgio.cu)
     int64_t widom_cap = 0;        // Widom insertion scratch (widom.cu)
     double *d_widom_pos = nullptr, *d_widom_rot = nullptr, *d_widom_res = nullptr;
+    double* d_widom_u = nullptr;     // FP64 form: real-space energies, points, their potentials and counts
+    float4* d_widom_atoms = nullptr; // FP64 form: sites the probe's O is tested against
+    double2* d_widom_pm = nullptr;   // FP64 form: the reciprocal sum's table
     int* d_widom_n = nullptr;
     float* d_widom_akf = nullptr;   // Ak in FP32 (mixed form)
     float2* d_widom_qsf = nullptr;  // S + S_wall in FP32 (mixed form)
@@ -389,6 +393,9 @@ void measure_do_launch(Ctx& c, const double* x, const double* y, const double* z
 int measure_get(Ctx& c, mdg_measure_out* o);
 // mdgpu.cu
 int resident_alloc(Ctx& c);
+void recip_pot_table(Ctx& c, double2* pm, cudaStream_t st);
+void recip_potential(Ctx& c, const double2* pm, const double* xyz, size_t stride, const int* np, int most, int likely,
+                     double* phi, cudaStream_t st);
 // widom.cu
 int widom(Ctx& c, const mdg_widom_params* p, double* seed, double* pave, int64_t* inave, int64_t* done);
 // shake.cu

@@ -259,6 +259,79 @@ __global__ void __launch_bounds__(kForceNT) k_kforce(View v, KDims d, int nrow, 
     }
 }
 
+// Widom insertion: P and M of every entry (two double2), from S and the walls' sums as they stand.
+__global__ void k_pot_table(int nrow, const int4* __restrict__ rows, const int* __restrict__ nlen,
+                            const int* __restrict__ ent, const double* __restrict__ ak, const double2* __restrict__ S,
+                            const double2* __restrict__ qw, double2* __restrict__ PM) {
+    const int lane = threadIdx.x & 31;
+    auto coef = [&](int k) {
+        const double a = ak[k];
+        return make_double2(a * (S[k].x + qw[k].x), -a * (S[k].y + qw[k].y));
+    };
+    for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrow; r += (gridDim.x * blockDim.x) >> 5) {
+        const int4 rw = rows[r];
+        const int ne = row_entries(rw.z, nlen[r]), kc = rw.w - rw.z;
+        for (int n = lane; n < ne; n += 32) {
+            double2 cp = make_double2(0.0, 0.0), cm = cp;
+            if (n > 0 || rw.z <= 0) cp = coef(kc + n);
+            if (n > 0 && rw.z <= 0) cm = coef(kc - n);
+            double2* o = PM + 2 * (size_t)(ent[r] + n);
+            o[0] = make_double2(cp.x + cm.x, cp.y + cm.y);
+            o[1] = make_double2(cp.x - cm.x, cp.y - cm.y);
+        }
+    }
+}
+
+// phi(r) = sum_k Re(C(k) e^{ik.r}) at the points (x, y, z)[0, *np): k_kforce's sums without the forces, 4
+// FMAs per entry.  A point costs the FMAs of nk / 2 entries whatever molecule it belongs to, so the
+// points of all insertions share the blocks.
+__global__ void __launch_bounds__(kForceNT) k_pot(KDims d, int nrow, const int4* __restrict__ rows,
+                                                  const int* __restrict__ nlen, const int* __restrict__ ent,
+                                                  const double2* __restrict__ PM, const double* __restrict__ xyz,
+                                                  size_t stride, const int* __restrict__ np, double* __restrict__ phi) {
+    extern __shared__ double2 sm[];
+    const int n_pts = *np;
+    if (blockIdx.x * kForceNT >= n_pts) return;
+    double2* em = sm + threadIdx.x;
+    double2* en = em + (size_t)(d.KM + 1) * kForceNT;
+    const int p = min(blockIdx.x * kForceNT + (int)threadIdx.x, n_pts - 1);
+    phase_table(d.py * xyz[stride + p], d.KM, em, kForceNT);
+    phase_table(d.pz * xyz[2 * stride + p], d.KN, en, kForceNT);
+    double s, c;
+    sincos(d.px * xyz[p], &s, &c);
+    const double2 el1 = make_double2(c, s);
+    double2 el = make_double2(1.0, 0.0);
+    int lcur = 0;
+    double sum = 0.0;
+    for (int r = blockIdx.y; r < nrow; r += gridDim.y) {
+        const int4 rw = rows[r];
+        while (lcur < rw.x) {
+            el = cmul(el, el1);
+            ++lcur;
+        }
+        double2 emm = em[(size_t)CK(abs(rw.y), d.KM + 1, 213) * kForceNT];
+        if (rw.y < 0) emm.y = -emm.y;
+        const double2 elm = cmul(el, emm);
+        const int ne = row_entries(rw.z, nlen[r]);
+        const double2* Ck = PM + 2 * (size_t)ent[r];
+        const double2 P0 = __ldg(Ck);
+        double tr0 = P0.x, tr1 = 0.0, ti0 = P0.y, ti1 = 0.0;
+#pragma unroll 4
+        for (int n = 1; n < ne; ++n) {
+            const double2 e = en[(size_t)CK(n, d.KN + 1, 214) * kForceNT];
+            const double2 P = __ldg(Ck + 2 * n), M = __ldg(Ck + 2 * n + 1);
+            tr0 = fma(P.x, e.x, tr0);
+            tr1 = fma(M.y, e.y, tr1);
+            ti0 = fma(P.y, e.x, ti0);
+            ti1 = fma(M.x, e.y, ti1);
+        }
+        sum += elm.x * (tr0 - tr1) - elm.y * (ti0 + ti1);
+    }
+    if (blockIdx.x * kForceNT + (int)threadIdx.x >= n_pts) return;
+    if (gridDim.y > 1) atomicAdd(&phi[p], sum);
+    else phi[p] = sum;
+}
+
 // Work items of k_sfac for the rows (n_first, nlen): (row, first entry | entries << 16), each row cut
 // into equal items of at most kChunk entries, sorted by length so that the lanes of a warp run alike.
 // Returns the number of entries of all rows; ent[r] is row r's first.
@@ -417,6 +490,8 @@ int recip_setup(Ctx& c, int64_t kmax, const double* x0, const double* y0, const 
     }
     MDG_CUDA(allow_max_smem(k_sfac));
     MDG_CUDA(allow_max_smem(k_kforce));
+    MDG_CUDA(allow_max_smem(k_pot));
+    ks.nent = nent;
     // (the limits that earlier tile sizes set: what they refused stays refused)
     const int per = (KL + 1 + KM + 1 + KN + 1) * (int)sizeof(double2) + (int)sizeof(double);
     if (128 * (KM + 1 + KN + 1) * (int)sizeof(double2) > 200 * 1024 ||
@@ -437,6 +512,26 @@ void recip_fp64(Ctx& c) {
     k_kenergy<<<std::min((ks.nrow + 7) / 8, 256), 256, 0, c.stream>>>(v, ks.nrow, ks.row, ks.row_nlen, ks.ent, ks.ak,
                                                                      ks.s, ks.qw, ks.c4);
     k_kforce<<<g.force, kForceNT, g.smem_force, c.stream>>>(v, d, ks.nrow, ks.row, ks.row_nlen, ks.ent, ks.c4);
+}
+
+void recip_pot_table(Ctx& c, double2* pm, cudaStream_t st) {
+    const KSet& ks = c.ks;
+    if (ks.nk == 0) return;
+    k_pot_table<<<std::min((ks.nrow + 7) / 8, 256), 256, 0, st>>>(ks.nrow, ks.row, ks.row_nlen, ks.ent, ks.ak, ks.s, ks.qw,
+                                                                  pm);
+}
+
+// np: number of points on the device, at most `most`, of which `likely` are expected.
+void recip_potential(Ctx& c, const double2* pm, const double* xyz, size_t stride, const int* np, int most, int likely,
+                     double* phi, cudaStream_t st) {
+    const KSet& ks = c.ks;
+    cudaMemsetAsync(phi, 0, sizeof(double) * most, st);
+    if (ks.nk == 0) return;
+    const KDims d{ks.klmax, ks.kmmax, ks.knmax, ks.pipix, ks.pipiy, ks.pipiz};
+    const int want = (152 * 8 * kForceNT + likely - 1) / likely;
+    const dim3 grid((most + kForceNT - 1) / kForceNT, std::max(1, std::min(std::min(want, kMaxSplit), ks.nrow)));
+    k_pot<<<grid, kForceNT, sizeof(double2) * kForceNT * (size_t)(d.KM + 1 + d.KN + 1), st>>>(
+        d, ks.nrow, ks.row, ks.row_nlen, ks.ent, pm, xyz, stride, np, phi);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -2,26 +2,40 @@
 //
 // The host draws the positions and orientations with the reference's congruential generator
 // (src/rndmod.f90:26-35) in the reference's order, assuming every position is accepted, and
-// records the generator state after each position and after its orientations.  One CTA per
-// position then (k_widom):
-//   - scans all sites for the O of the probe: overlap test (2.35 A to a water O, 2 A to others,
+// records the generator state after each position and after its orientations.  What an insertion needs:
+//   - all sites against the O of the probe: overlap test (2.35 A to a water O, 2 A to others,
 //     src/forcem.f90:1303-1313), vdW + Ewald erfc of the O (src/forcem.f90:1315-1334) and the
 //     neighbour list within rcut (every site that is not of the H type), kept in shared memory;
 //   - per orientation, the Ewald erfc terms of the probe's sites against the neighbours' sites
 //     (src/forcem.f90:1378-1423), the reciprocal term 0.5 Ak Re(sum_s q_s e^{ik r_s} conj(Qsum))
-//     with the phase tables built by repeated multiplication as the reference builds them
 //     (src/forcem.f90:1428-1474), the optional slab term and the O's wall tail (:1481-1494);
 //     exp(-beta u) summed over the orientations.
 // The host keeps the positions up to the first overlap (the reference leaves the insertion loop
 // there, src/forcem.f90:1342) unless MDG_WIDOM_SKIP_OVERLAP is set, and accumulates pave/inave.
-// Contexts of the FP64 form run everything in FP64; those of the mixed form run the orientation
-// loop in FP32 (block sums, the wall tail and the exponential stay FP64).
+//
+// FP64 contexts (FP64 operations bound it, so the kernels are cut to have few of them):
+//   k_widom_atoms  the sites that are not of the H type, in the box, in FP32
+//   k_widom_real   a CTA per position.  A scan in FP32 picks the sites that may be inside the cutoff
+//                  (margin far above FP32 rounding), these are tested in FP64; a site certainly too
+//                  near ends the position.  Terms of the O are summed once, those of the two H over
+//                  (orientation, neighbour) pairs dealt evenly to the threads, with the pair
+//                  function from a table (erfc_table.cuh).  Accepted positions append their points (the
+//                  O, two H per orientation) to one list.
+//   k_pot          (recip.cu) sum_k Ak Re(e^{ik r} conj(Qsum)) at all points of all positions: the O's once
+//                  per position, 2 FMAs per k and point where the product of the phase factors of
+//                  three sites per orientation takes about 37 operations per k
+//   k_widom_sum    energies and exponentials, a warp per position
+// 2,000 positions in a 2,048-water slab (4,338 k, 7,744 sites): 4.64 ms in one kernel per position before,
+// now 0.31 ms (k_pot), 0.23 ms (k_widom_real) and 0.015 ms for the other three.
+// Mixed contexts: k_widom, one CTA per position, the orientation loop in FP32 (block sums, the O's scan,
+// the wall tail and the exponential stay FP64).
 #include <algorithm>
 #include <cmath>
 #include <vector>
 
 #include "common.cuh"
 #include "ctx.h"
+#include "erfc_table.cuh"
 
 namespace mdg {
 
@@ -89,18 +103,219 @@ __device__ double block_sum_d(double x, double* red) {
     return s;
 }
 
-// MX: the orientation loop (real-space erfc terms and the reciprocal term) in FP32 with FP64 sums
-// per block, for contexts of the mixed form; the O scan, the wall tail and exp stay FP64.
-template <bool MX>
+// The O's wall tail (src/forcem.f90:1481-1494).
+__device__ double wall_tail(const View& v, const double* lr, double oz) {
+    const int nit = v.nit;
+    double u = 0.0;
+    for (int j = -1; j <= 1; j += 2) {
+        const double dw = v.lwh - (double)j * oz;
+        if (dw < v.rcut) {
+            u += lr[8 * nit];
+        } else {
+            u += lr[7 * nit];
+            const double dw3 = dw * dw * dw;
+            u += (lr[2 * nit] / (9.0 * (dw3 * dw3 * dw3)) - lr[3 * nit] / (3.0 * dw3));
+            const double tt = lr[6 * nit];
+            const double exp2a = lr[4 * nit] * exp(-dw / tt);
+            u += (tt * (2.0 * tt + dw) * exp2a - lr[5 * nit] / (3.0 * dw3));
+        }
+    }
+    return u;
+}
+
+constexpr int kRT = 128;           // threads per position of k_widom_real
+constexpr int kCand = 2048;        // sites picked by its FP32 scan (more are tested where they are found)
+constexpr int kPts = 1 + 2 * kMaxRot;
+
+// FP64 form's scratch of one call.
+struct W64 {
+    float4* atoms;   // x, y (in the box), z, index
+    int* cnt;        // sites in atoms, points
+    int* off;        // first point of each accepted position
+    double* u;       // [ins][kMaxRot] real-space energies
+    double* xyz;     // points: x, y, z, stride apart
+    double* phi;     // reciprocal potential at the points
+    size_t stride;
+    float lx, lxi, ly, lyi, rcut, near2, far2;  // below near2: certainly an overlap; above far2: certainly outside
+};
+
+__global__ void k_widom_atoms(View v, W64 s) {
+    const int a = blockIdx.x * blockDim.x + threadIdx.x;
+    if (a >= v.ntota || v.type[a] == 1) return;
+    const int k = atomicAdd(&s.cnt[0], 1);
+    s.atoms[k] = make_float4((float)minimg(v.x[a], v.lx, v.lxi), (float)minimg(v.y[a], v.ly, v.lyi), (float)v.z[a],
+                             __int_as_float(a));
+}
+
+__global__ void __launch_bounds__(kRT) k_widom_real(View v, WArgs w, W64 s) {
+    __shared__ int cand[kCand], nb_j[kWNb];          // water neighbours from the front, others from the back
+    __shared__ double nb_d[3 * kWNb];
+    __shared__ double so[kMaxRot][6], su[kMaxRot];   // H offsets from the O, sums per orientation
+    __shared__ double red[kRT / 32];
+    __shared__ int s_nc, s_nw, s_no, s_flag, s_off;
+    const int ins = blockIdx.x, t = threadIdx.x, lane = t & 31;
+    const double4 o = w.pos[ins];
+    const int nr = w.nrot[ins];
+    if (t == 0) s_nc = s_nw = s_no = s_flag = 0;
+    if (t < kMaxRot) su[t] = 0.0;
+    __syncthreads();
+    const double alfa2 = v.alfa * v.alfa, fq = v.facq * v.alfa;
+    double ux = 0.0;
+    // a site in FP64: overlap test, the O's terms with it (and, of a water, with its other sites), the list
+    auto visit = [&](int j) {
+        const int jt = v.type[j];
+        const double zio = o.z - v.z[j];
+        if (fabs(zio) > v.rcut) return;
+        const double xio = minimg(o.x - v.x[j], v.lx, v.lxi);
+        const double yio = minimg(o.y - v.y[j], v.ly, v.lyi);
+        const double rsq = xio * xio + yio * yio + zio * zio;
+        if (rsq > v.rcutsq) return;
+        if (rsq < w.rwinsmin && (jt == 0 || rsq < w.rinsmin)) {
+            atomicOr(&s_flag, 1);
+            return;
+        }
+        const int ijt = v.ijt[jt];  // it = 1 (the water O type)
+        const int vk = v.vdw[ijt];
+        if (vk == 1) {
+            const double rsqi = 1.0 / rsq;
+            const double r6 = v.sig[ijt] * (rsqi * rsqi * rsqi);
+            ux += v.eps[ijt] * r6 * (r6 - 1.0);
+        } else if (vk == 2) {
+            const double rsqi = 1.0 / rsq;
+            const double r6 = v.cc[ijt] * (rsqi * rsqi * rsqi);
+            ux += v.aa[ijt] * exp(-sqrt(rsq) * v.rhoi[ijt]) - r6;
+        }
+        double e = v.q[j] * ewald_g(alfa2 * rsq, v.etab, v.spii);
+        if (jt == 0)
+            for (int jx = j + 1; jx < j + v.nsi[0]; ++jx) {
+                const double xd = xio - v.rsx[jx], yd = yio - v.rsy[jx], zd = zio - v.rsz[jx];
+                e += v.q[jx] * ewald_g(alfa2 * (xd * xd + yd * yd + zd * zd), v.etab, v.spii);
+            }
+        ux += fq * w.q0 * e;
+        const int k = jt == 0 ? atomicAdd(&s_nw, 1) : kWNb - 1 - atomicAdd(&s_no, 1);
+        if (k >= 0 && k < kWNb) {
+            nb_j[k] = j;
+            nb_d[3 * k + 0] = xio;
+            nb_d[3 * k + 1] = yio;
+            nb_d[3 * k + 2] = zio;
+        }
+    };
+    {
+        const float ox = (float)minimg(o.x, v.lx, v.lxi), oy = (float)minimg(o.y, v.ly, v.lyi), oz = (float)o.z;
+        const int na = s.cnt[0];
+#pragma unroll 4
+        for (int k = t; k < na; k += kRT) {
+            const float4 a = s.atoms[k];
+            float dx = ox - a.x, dy = oy - a.y;
+            const float dz = oz - a.z;
+            dx -= s.lx * rintf(dx * s.lxi);
+            dy -= s.ly * rintf(dy * s.lyi);
+            const float r2 = dx * dx + dy * dy + dz * dz;
+            if (r2 > s.far2) continue;
+            if (r2 < s.near2) s_flag = 1;
+            const int c = atomicAdd(&s_nc, 1);
+            if (c < kCand) cand[c] = __float_as_int(a.w);
+            else visit(__float_as_int(a.w));
+        }
+    }
+    __syncthreads();
+    if (!(s_flag & 1))
+        for (int c = t; c < min(s_nc, kCand); c += kRT) visit(cand[c]);
+    __syncthreads();
+    const int nw = s_nw, no = s_no;
+    if ((s_flag & 1) || nw + no > kWNb) {
+        if (t == 0) w.res[ins] = make_double2(0.0, (s_flag & 1) ? 1.0 : 2.0);
+        return;
+    }
+    ux = warp_sum(ux);
+    if (lane == 0) red[t >> 5] = ux;
+    // the points: the O, then H1 and H2 of each orientation
+    if (t == 0) s_off = atomicAdd(&s.cnt[1], 1 + 2 * nr);
+    __syncthreads();
+    const double* rot = w.rot + (size_t)ins * kMaxRot * 6;
+    for (int k = t; k < 1 + 2 * nr; k += kRT) {
+        const size_t p = (size_t)s_off + k;
+        const double x = k ? rot[3 * (k - 1)] : o.x, y = k ? rot[3 * (k - 1) + 1] : o.y, z = k ? rot[3 * (k - 1) + 2] : o.z;
+        s.xyz[p] = x;
+        s.xyz[s.stride + p] = y;
+        s.xyz[2 * s.stride + p] = z;
+        if (k) {
+            double* d = &so[(k - 1) >> 1][3 * ((k - 1) & 1)];
+            d[0] = x - o.x;
+            d[1] = y - o.y;
+            d[2] = z - o.z;
+        }
+    }
+    __syncthreads();
+    // both H of an orientation with the sites of one neighbour
+    auto sweep = [&](int first, int cnt, bool water) {
+        const int total = nr * cnt;
+        for (int b = t - lane; b < total; b += kRT) {
+            const int i = min(b + lane, total - 1), r = i / cnt, k = first + i - r * cnt, j = nb_j[k];
+            double e = 0.0;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const double x = nb_d[3 * k] + so[r][3 * h], y = nb_d[3 * k + 1] + so[r][3 * h + 1],
+                             z = nb_d[3 * k + 2] + so[r][3 * h + 2];
+                if (water) {
+                    for (int jx = j; jx < j + v.nsi[0]; ++jx) {
+                        const double xd = x - v.rsx[jx], yd = y - v.rsy[jx], zd = z - v.rsz[jx];
+                        e += v.q[jx] * ewald_g(alfa2 * (xd * xd + yd * yd + zd * zd), v.etab, v.spii);
+                    }
+                } else {
+                    e += v.q[j] * ewald_g(alfa2 * (x * x + y * y + z * z), v.etab, v.spii);
+                }
+            }
+            if (b + lane >= total) e = 0.0;
+            const int r1 = min(b + 31, total - 1) / cnt;
+            for (int rr = b / cnt; rr <= r1; ++rr) {
+                const double sum = warp_sum(r == rr ? e : 0.0);
+                if (lane == 0) atomicAdd(&su[rr], sum);
+            }
+        }
+    };
+    if (nw) sweep(0, nw, true);
+    if (no) sweep(kWNb - no, no, false);
+    __syncthreads();
+    if (t < nr) {
+        double u0 = 0.0;
+        for (int k = 0; k < kRT / 32; ++k) u0 += red[k];
+        s.u[(size_t)ins * kMaxRot + t] = u0 + fq * w.q1 * su[t];
+    }
+    if (t == 0) {
+        s.off[ins] = s_off;
+        w.res[ins] = make_double2(0.0, 0.0);
+    }
+}
+
+__global__ void k_widom_sum(View v, WArgs w, W64 s, int nins) {
+    const int ins = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, r = threadIdx.x & 31;
+    if (ins >= nins || w.res[ins].y != 0.0) return;
+    double e = 0.0;
+    if (r < w.nrot[ins]) {
+        const double* rr = w.rot + ((size_t)ins * kMaxRot + r) * 6;
+        const double* phi = s.phi + s.off[ins];
+        const double oz = w.pos[ins].z;
+        const double u_rec = 0.5 * (w.q0 * phi[0] + w.q1 * (phi[1 + 2 * r] + phi[2 + 2 * r]));
+        double u = s.u[(size_t)ins * kMaxRot + r] + u_rec;
+        u -= w.crf * (w.q0 * oz + w.q1 * rr[2] + w.q1 * rr[5]);
+        u += wall_tail(v, w.lr, oz);
+        e = exp(-w.beta * u);
+    }
+    e = warp_sum(e);
+    if (r == 0) w.res[ins].x = e;
+}
+
+// Mixed form: the orientation loop (real-space erfc terms and the reciprocal term) in FP32 with FP64
+// sums per block; the O scan, the wall tail and exp stay FP64.
 __global__ void __launch_bounds__(kWT) k_widom(View v, WArgs w) {
     extern __shared__ __align__(16) unsigned char sm[];
     int* nb_j = reinterpret_cast<int*>(sm);
     double* nb_d = reinterpret_cast<double*>(sm + sizeof(int) * kWNb);           // [kWNb][3]
-    double2* tab = reinterpret_cast<double2*>(sm + sizeof(int) * kWNb + sizeof(double) * 3 * kWNb);
+    float2* elf = reinterpret_cast<float2*>(sm + sizeof(int) * kWNb + sizeof(double) * 3 * kWNb);  // [3][nl]
     const int nl = w.KL + 1, nm = 2 * w.KM + 1, nn = 2 * w.KN + 1;
-    double2* el = tab;                 // [3][nl]
-    double2* em = el + 3 * nl;         // [3][nm], index m + KM
-    double2* en = em + 3 * nm;         // [3][nn], index n + KN
+    float2* emf = elf + 3 * nl;        // [3][nm], index m + KM
+    float2* enf = emf + 3 * nm;        // [3][nn], index n + KN
     __shared__ double red[kWT / 32];
     __shared__ int s_nnb, s_flag;
     const int ins = blockIdx.x, t = threadIdx.x;
@@ -162,173 +377,90 @@ __global__ void __launch_bounds__(kWT) k_widom(View v, WArgs w) {
         const double* rr = w.rot + ((size_t)ins * kMaxRot + r) * 6;
         const double sx[3] = {ox, rr[0], rr[3]}, sy[3] = {oy, rr[1], rr[4]}, sz[3] = {oz, rr[2], rr[5]};
         double ur = 0.0, uk = 0.0;
-        if constexpr (!MX) {
-            // ---- real space: the probe's sites against the neighbours' sites
-            for (int k = t; k < nnb; k += kWT) {
-                const int j = nb_j[k];
-                const double xio = nb_d[3 * k], yio = nb_d[3 * k + 1], zio = nb_d[3 * k + 2];
-                const int jt = v.type[j];
-                if (jt == 0) {
-                    const int njx = v.nsi[jt];
-                    for (int ix = 0; ix < 3; ++ix) {
-                        const double xi = (xio + sx[ix]) - ox, yi = (yio + sy[ix]) - oy, zi = (zio + sz[ix]) - oz;
-                        const double qx = v.facq * qs3[ix];
-                        for (int jx = (ix == 0 ? j + 1 : j); jx < j + njx; ++jx) {
-                            const double xd = xi - v.rsx[jx], yd = yi - v.rsy[jx], zd = zi - v.rsz[jx];
-                            const double rsq = xd * xd + yd * yd + zd * zd;
-                            const double rij = sqrt(rsq);
-                            ur += ewald_e(rij, v.alfa) * (qx * v.q[jx] / rij);
-                        }
-                    }
-                } else {
-                    for (int ix = 1; ix < 3; ++ix) {
-                        const double xi = (xio + sx[ix]) - ox, yi = (yio + sy[ix]) - oy, zi = (zio + sz[ix]) - oz;
-                        const double rsq = xi * xi + yi * yi + zi * zi;
-                        const double rij = sqrt(rsq);
-                        ur += ewald_e(rij, v.alfa) * (v.facq * qs3[ix] * v.q[j] / rij);
-                    }
-                }
-            }
-            // ---- reciprocal space: per-site phase tables by repeated multiplication
-            if (t < 9) {
-                const int s = t / 3, ax = t % 3;
-                const double ang = ax == 0 ? w.pipix * sx[s] : (ax == 1 ? w.pipiy * sy[s] : w.pipiz * sz[s]);
-                double2 e1;
-                sincos(ang, &e1.y, &e1.x);
-                if (ax == 0) {
-                    double2* T = el + s * nl;
-                    T[0] = make_double2(1.0, 0.0);
-                    if (w.KL >= 1) T[1] = e1;
-                    for (int l = 2; l <= w.KL; ++l)
-                        T[l] = make_double2(T[l - 1].x * e1.x - T[l - 1].y * e1.y, T[l - 1].x * e1.y + T[l - 1].y * e1.x);
-                } else {
-                    const int K = ax == 1 ? w.KM : w.KN;
-                    double2* T = (ax == 1 ? em + s * nm : en + s * nn) + K;
-                    T[0] = make_double2(1.0, 0.0);
-                    if (K >= 1) T[1] = e1;
-                    for (int l = 2; l <= K; ++l)
-                        T[l] = make_double2(T[l - 1].x * e1.x - T[l - 1].y * e1.y, T[l - 1].x * e1.y + T[l - 1].y * e1.x);
-                    for (int l = 1; l <= K; ++l) T[-l] = make_double2(T[l].x, -T[l].y);
-                }
-            }
-            __syncthreads();
-            for (int k = t; k < w.nk; k += kWT) {
-                const int3 kv = w.kvec[k];
-                double xr = 0.0, xi = 0.0;
+        // ---- real space in FP32: site offsets from the O, neighbour sites from the FP32
+        // copy of rs and q
+        const float qx3[3] = {(float)(v.facq * qs3[0]), (float)(v.facq * qs3[1]), (float)(v.facq * qs3[2])};
+        float dsx[3], dsy[3], dsz[3];
 #pragma unroll
-                for (int s = 0; s < 3; ++s) {
-                    const double2 a = el[s * nl + kv.x], b = em[s * nm + kv.y + w.KM], c = en[s * nn + kv.z + w.KN];
-                    const double lr_ = qs3[s] * (a.x * b.x - a.y * b.y), li_ = qs3[s] * (a.x * b.y + a.y * b.x);
-                    xr += lr_ * c.x - li_ * c.y;
-                    xi += lr_ * c.y + li_ * c.x;
-                }
-                const double2 sk = w.sk[k], q = w.qw[k];
-                const double qr = sk.x + q.x, qi = sk.y + q.y;
-                uk += 0.5 * w.ak[k] * (xr * qr + xi * qi);
-            }
-
-        } else {
-            // ---- the same terms in FP32: site offsets from the O, neighbour sites from the FP32
-            // copy of rs and q
-            const float qx3[3] = {(float)(v.facq * qs3[0]), (float)(v.facq * qs3[1]), (float)(v.facq * qs3[2])};
-            float dsx[3], dsy[3], dsz[3];
-#pragma unroll
-            for (int ix = 0; ix < 3; ++ix) {
-                dsx[ix] = (float)(sx[ix] - ox);
-                dsy[ix] = (float)(sy[ix] - oy);
-                dsz[ix] = (float)(sz[ix] - oz);
-            }
-            const float alfa = (float)v.alfa;
-            float urf = 0.f;
-            for (int k = t; k < nnb; k += kWT) {
-                const int j = nb_j[k];
-                const float xio = (float)nb_d[3 * k], yio = (float)nb_d[3 * k + 1], zio = (float)nb_d[3 * k + 2];
-                const int jt = v.type[j];
-                if (jt == 0) {
-                    const int njx = v.nsi[jt];
-                    for (int ix = 0; ix < 3; ++ix) {
-                        const float xi = xio + dsx[ix], yi = yio + dsy[ix], zi = zio + dsz[ix];
-                        for (int jx = (ix == 0 ? j + 1 : j); jx < j + njx; ++jx) {
-                            const float4 qj = w.rsf[jx];
-                            const float xd = xi - qj.x, yd = yi - qj.y, zd = zi - qj.z;
-                            const float r2 = xd * xd + yd * yd + zd * zd;
-                            const float ri = rsqrtf(r2);
-                            urf += ewald_ef(r2 * ri, alfa) * (qx3[ix] * qj.w * ri);
-                        }
-                    }
-                } else {
-                    const float qj = w.rsf[j].w;
-                    for (int ix = 1; ix < 3; ++ix) {
-                        const float xi = xio + dsx[ix], yi = yio + dsy[ix], zi = zio + dsz[ix];
-                        const float r2 = xi * xi + yi * yi + zi * zi;
-                        const float ri = rsqrtf(r2);
-                        urf += ewald_ef(r2 * ri, alfa) * (qx3[ix] * qj * ri);
-                    }
-                }
-            }
-            ur = (double)urf;
-            float2* elf = reinterpret_cast<float2*>(tab);
-            float2* emf = elf + 3 * nl;
-            float2* enf = emf + 3 * nm;
-            if (t < 9) {
-                const int s = t / 3, ax = t % 3;
-                const double ang = ax == 0 ? w.pipix * sx[s] : (ax == 1 ? w.pipiy * sy[s] : w.pipiz * sz[s]);
-                double cd, sd;
-                sincos(ang, &sd, &cd);
-                const float2 e1 = make_float2((float)cd, (float)sd);
-                if (ax == 0) {
-                    float2* T = elf + s * nl;
-                    T[0] = make_float2(1.f, 0.f);
-                    if (w.KL >= 1) T[1] = e1;
-                    for (int l = 2; l <= w.KL; ++l)
-                        T[l] = make_float2(T[l - 1].x * e1.x - T[l - 1].y * e1.y, T[l - 1].x * e1.y + T[l - 1].y * e1.x);
-                } else {
-                    const int K = ax == 1 ? w.KM : w.KN;
-                    float2* T = (ax == 1 ? emf + s * nm : enf + s * nn) + K;
-                    T[0] = make_float2(1.f, 0.f);
-                    if (K >= 1) T[1] = e1;
-                    for (int l = 2; l <= K; ++l)
-                        T[l] = make_float2(T[l - 1].x * e1.x - T[l - 1].y * e1.y, T[l - 1].x * e1.y + T[l - 1].y * e1.x);
-                    for (int l = 1; l <= K; ++l) T[-l] = make_float2(T[l].x, -T[l].y);
-                }
-            }
-            __syncthreads();
-            const float q3f[3] = {(float)qs3[0], (float)qs3[1], (float)qs3[2]};
-            float ukf = 0.f;
-            for (int k = t; k < w.nk; k += kWT) {
-                const int3 kv = w.kvec[k];
-                float xr = 0.f, xi = 0.f;
-#pragma unroll
-                for (int s = 0; s < 3; ++s) {
-                    const float2 a = elf[s * nl + kv.x], b = emf[s * nm + kv.y + w.KM], cc = enf[s * nn + kv.z + w.KN];
-                    const float lr_ = q3f[s] * (a.x * b.x - a.y * b.y), li_ = q3f[s] * (a.x * b.y + a.y * b.x);
-                    xr += lr_ * cc.x - li_ * cc.y;
-                    xi += lr_ * cc.y + li_ * cc.x;
-                }
-                const float2 q = w.qsf[k];
-                ukf += 0.5f * w.akf[k] * (xr * q.x + xi * q.y);
-            }
-            uk = (double)ukf;
+        for (int ix = 0; ix < 3; ++ix) {
+            dsx[ix] = (float)(sx[ix] - ox);
+            dsy[ix] = (float)(sy[ix] - oy);
+            dsz[ix] = (float)(sz[ix] - oz);
         }
+        const float alfa = (float)v.alfa;
+        float urf = 0.f;
+        for (int k = t; k < nnb; k += kWT) {
+            const int j = nb_j[k];
+            const float xio = (float)nb_d[3 * k], yio = (float)nb_d[3 * k + 1], zio = (float)nb_d[3 * k + 2];
+            const int jt = v.type[j];
+            if (jt == 0) {
+                const int njx = v.nsi[jt];
+                for (int ix = 0; ix < 3; ++ix) {
+                    const float xi = xio + dsx[ix], yi = yio + dsy[ix], zi = zio + dsz[ix];
+                    for (int jx = (ix == 0 ? j + 1 : j); jx < j + njx; ++jx) {
+                        const float4 qj = w.rsf[jx];
+                        const float xd = xi - qj.x, yd = yi - qj.y, zd = zi - qj.z;
+                        const float r2 = xd * xd + yd * yd + zd * zd;
+                        const float ri = rsqrtf(r2);
+                        urf += ewald_ef(r2 * ri, alfa) * (qx3[ix] * qj.w * ri);
+                    }
+                }
+            } else {
+                const float qj = w.rsf[j].w;
+                for (int ix = 1; ix < 3; ++ix) {
+                    const float xi = xio + dsx[ix], yi = yio + dsy[ix], zi = zio + dsz[ix];
+                    const float r2 = xi * xi + yi * yi + zi * zi;
+                    const float ri = rsqrtf(r2);
+                    urf += ewald_ef(r2 * ri, alfa) * (qx3[ix] * qj * ri);
+                }
+            }
+        }
+        ur = (double)urf;
+        if (t < 9) {
+            const int s = t / 3, ax = t % 3;
+            const double ang = ax == 0 ? w.pipix * sx[s] : (ax == 1 ? w.pipiy * sy[s] : w.pipiz * sz[s]);
+            double cd, sd;
+            sincos(ang, &sd, &cd);
+            const float2 e1 = make_float2((float)cd, (float)sd);
+            if (ax == 0) {
+                float2* T = elf + s * nl;
+                T[0] = make_float2(1.f, 0.f);
+                if (w.KL >= 1) T[1] = e1;
+                for (int l = 2; l <= w.KL; ++l)
+                    T[l] = make_float2(T[l - 1].x * e1.x - T[l - 1].y * e1.y, T[l - 1].x * e1.y + T[l - 1].y * e1.x);
+            } else {
+                const int K = ax == 1 ? w.KM : w.KN;
+                float2* T = (ax == 1 ? emf + s * nm : enf + s * nn) + K;
+                T[0] = make_float2(1.f, 0.f);
+                if (K >= 1) T[1] = e1;
+                for (int l = 2; l <= K; ++l)
+                    T[l] = make_float2(T[l - 1].x * e1.x - T[l - 1].y * e1.y, T[l - 1].x * e1.y + T[l - 1].y * e1.x);
+                for (int l = 1; l <= K; ++l) T[-l] = make_float2(T[l].x, -T[l].y);
+            }
+        }
+        __syncthreads();
+        const float q3f[3] = {(float)qs3[0], (float)qs3[1], (float)qs3[2]};
+        float ukf = 0.f;
+        for (int k = t; k < w.nk; k += kWT) {
+            const int3 kv = w.kvec[k];
+            float xr = 0.f, xi = 0.f;
+#pragma unroll
+            for (int s = 0; s < 3; ++s) {
+                const float2 a = elf[s * nl + kv.x], b = emf[s * nm + kv.y + w.KM], cc = enf[s * nn + kv.z + w.KN];
+                const float lr_ = q3f[s] * (a.x * b.x - a.y * b.y), li_ = q3f[s] * (a.x * b.y + a.y * b.x);
+                xr += lr_ * cc.x - li_ * cc.y;
+                xi += lr_ * cc.y + li_ * cc.x;
+            }
+            const float2 q = w.qsf[k];
+            ukf += 0.5f * w.akf[k] * (xr * q.x + xi * q.y);
+        }
+        uk = (double)ukf;
         const double u_real = block_sum_d(ur, red);
         const double u_rec = block_sum_d(uk, red);
         if (t == 0) {
             double u = u_real + ux + u_rec;
             u -= w.crf * (w.q0 * sz[0] + w.q1 * sz[1] + w.q1 * sz[2]);
-            const int nit = v.nit;
-            for (int j = -1; j <= 1; j += 2) {
-                const double dw = v.lwh - (double)j * oz;
-                if (dw < v.rcut) {
-                    u += w.lr[8 * nit];
-                } else {
-                    u += w.lr[7 * nit];
-                    const double dw3 = dw * dw * dw;
-                    u += (w.lr[2 * nit] / (9.0 * (dw3 * dw3 * dw3)) - w.lr[3 * nit] / (3.0 * dw3));
-                    const double tt = w.lr[6 * nit];
-                    const double exp2a = w.lr[4 * nit] * exp(-dw / tt);
-                    u += (tt * (2.0 * tt + dw) * exp2a - w.lr[5 * nit] / (3.0 * dw3));
-                }
-            }
+            u += wall_tail(v, w.lr, oz);
             acc += exp(-w.beta * u);
         }
         __syncthreads();  // tables are rebuilt for the next orientation
@@ -416,6 +548,13 @@ int widom(Ctx& c, const mdg_widom_params* p, double* seed, double* pave, int64_t
         c.d_widom_n = (int*)dalloc(c, sizeof(int) * cap);
         c.d_widom_res = (double*)dalloc(c, sizeof(double) * 2 * cap);
         if (c.alloc_failed) return set_err(&c, MDG_E_CUDA, "Widom insertion: out of device memory");
+        if (c.precision != MDG_MIXED) {
+            // real-space energies, points, potentials (doubles), first points and two counts (int)
+            c.d_widom_u = (double*)dalloc(c, (sizeof(double) * (kMaxRot + 4 * kPts) + sizeof(int)) * cap + 2 * sizeof(int));
+            if (!c.d_widom_pm) c.d_widom_pm = (double2*)dalloc(c, 2 * sizeof(double2) * std::max(ks.nent, 1));
+            if (!c.d_widom_atoms) c.d_widom_atoms = (float4*)dalloc(c, sizeof(float4) * std::max(v.ntota, 1));
+            if (c.alloc_failed) return set_err(&c, MDG_E_CUDA, "Widom insertion: out of device memory");
+        }
         c.widom_cap = cap;
     }
     MDG_CUDA(cudaMemcpyAsync(c.d_widom_pos, hp.data(), sizeof(double) * 4 * nins, cudaMemcpyHostToDevice, c.stream));
@@ -449,11 +588,10 @@ int widom(Ctx& c, const mdg_widom_params* p, double* seed, double* pave, int64_t
     w.q0 = (double)-0.8476f;
     w.q1 = (double)0.4238f;
     const size_t smem = sizeof(int) * kWNb + sizeof(double) * 3 * kWNb +
-                        sizeof(double2) * 3 * (size_t)((ks.klmax + 1) + (2 * ks.kmmax + 1) + (2 * ks.knmax + 1));
+                        sizeof(float2) * 3 * (size_t)((ks.klmax + 1) + (2 * ks.kmmax + 1) + (2 * ks.knmax + 1));
     const bool mx = c.precision == MDG_MIXED;
     if (!c.widom_attr) {
-        MDG_CUDA(allow_max_smem(k_widom<false>));
-        MDG_CUDA(allow_max_smem(k_widom<true>));
+        MDG_CUDA(allow_max_smem(k_widom));
         c.widom_attr = true;
     }
     w.qsf = nullptr;
@@ -477,9 +615,32 @@ int widom(Ctx& c, const mdg_widom_params* p, double* seed, double* pave, int64_t
         w.qsf = c.d_widom_qsf;
         w.akf = c.d_widom_akf;
         w.rsf = c.d_widom_rsf;
-        k_widom<true><<<(unsigned)nins, kWT, smem, c.stream>>>(v, w);
+        k_widom<<<(unsigned)nins, kWT, smem, c.stream>>>(v, w);
     } else {
-        k_widom<false><<<(unsigned)nins, kWT, smem, c.stream>>>(v, w);
+        W64 s;
+        s.atoms = c.d_widom_atoms;
+        s.stride = (size_t)kPts * c.widom_cap;
+        s.u = c.d_widom_u;
+        s.xyz = s.u + (size_t)kMaxRot * c.widom_cap;
+        s.phi = s.xyz + 3 * s.stride;
+        s.off = reinterpret_cast<int*>(s.phi + s.stride);
+        s.cnt = s.off + c.widom_cap;
+        s.lx = (float)v.lx;
+        s.ly = (float)v.ly;
+        s.lxi = (float)v.lxi;
+        s.lyi = (float)v.lyi;
+        s.rcut = (float)v.rcut;
+        // FP32 rounding moves a squared distance r^2 by less than 4e-7 r (r + box edge)
+        const double box = std::max(v.lx, std::max(v.ly, v.lz));
+        s.far2 = (float)(v.rcutsq + 1e-5 * v.rcut * (v.rcut + box));
+        s.near2 = (float)(std::min(w.rinsmin, v.rcutsq) - 1e-5 * 2.0 * (2.0 + box));
+        MDG_CUDA(cudaMemsetAsync(s.cnt, 0, 2 * sizeof(int), c.stream));
+        k_widom_atoms<<<(v.ntota + 255) / 256, 256, 0, c.stream>>>(v, s);
+        recip_pot_table(c, c.d_widom_pm, c.stream);
+        k_widom_real<<<(unsigned)nins, kRT, 0, c.stream>>>(v, w, s);
+        recip_potential(c, c.d_widom_pm, s.xyz, s.stride, s.cnt + 1, (int)(kPts * nins), (int)(kPts * nins / 2 + 1), s.phi,
+                        c.stream);
+        k_widom_sum<<<(unsigned)((nins + 7) / 8), 256, 0, c.stream>>>(v, w, s, (int)nins);
     }
     MDG_CUDA(cudaGetLastError());
     std::vector<double> res(2 * nins);
