@@ -257,11 +257,12 @@ struct Ctx {
     Meas meas;                    // measurement histograms (measure.cu)
     std::vector<int64_t> h_moltypen, h_nt, h_ns, h_itype;  // molecule types and site types (cfgio.cu)
     int64_t widom_cap = 0;        // Widom insertion scratch (widom.cu)
-    double *d_widom_pos = nullptr, *d_widom_rot = nullptr, *d_widom_res = nullptr;
+    double *d_widom_draw = nullptr, *d_widom_rot = nullptr, *d_widom_res = nullptr;
+    double* h_widom_draw = nullptr;  // pinned, two chunks
+    cudaEvent_t widom_read[2] = {nullptr, nullptr};
     double* d_widom_u = nullptr;     // FP64 form: real-space energies, points, their potentials and counts
     float4* d_widom_atoms = nullptr; // FP64 form: sites the probe's O is tested against
     double2* d_widom_pm = nullptr;   // FP64 form: the reciprocal sum's table
-    int* d_widom_n = nullptr;
     float* d_widom_akf = nullptr;   // Ak in FP32 (mixed form)
     float2* d_widom_qsf = nullptr;  // S + S_wall in FP32 (mixed form)
     float4* d_widom_rsf = nullptr;  // rs offsets and charges in FP32 (mixed form)

@@ -368,6 +368,9 @@ void mdg_destroy(mdg_ctx* c) {
     if (c->h_acc) cudaFreeHost(c->h_acc);
     if (c->h_status) cudaFreeHost(c->h_status);
     if (c->h_small) cudaFreeHost(c->h_small);
+    if (c->h_widom_draw) cudaFreeHost(c->h_widom_draw);
+    for (cudaEvent_t e : c->widom_read)
+        if (e) cudaEventDestroy(e);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     else if (c->stream) cudaStreamDestroy(c->stream);
     if (c->side) cudaStreamDestroy(c->side);

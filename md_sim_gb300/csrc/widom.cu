@@ -2,7 +2,10 @@
 //
 // The host draws the positions and orientations with the reference's congruential generator
 // (src/rndmod.f90:26-35) in the reference's order, assuming every position is accepted, and
-// records the generator state after each position and after its orientations.  What an insertion needs:
+// records the generator state after each position and after its orientations, a chunk of positions while the
+// device evaluates the one before; the device makes the orientations from the states they start at.
+// (2,000 positions: 4.9 ms a call when they were drawn with fmod, up front and on one buffer, 1.46 ms now,
+// about 1 ms of it the drawing of 40,000 orientations.)  What an insertion needs:
 //   - all sites against the O of the probe: overlap test (2.35 A to a water O, 2 A to others,
 //     src/forcem.f90:1303-1313), vdW + Ewald erfc of the O (src/forcem.f90:1315-1334) and the
 //     neighbour list within rcut (every site that is not of the H type), kept in shared memory;
@@ -44,16 +47,56 @@ namespace {
 constexpr int kWT = 256;        // threads per insertion
 constexpr int kWNb = 1024;      // neighbour capacity per insertion
 constexpr int kMaxRot = 20;
+constexpr int kIns = 512;       // positions drawn, copied and evaluated at a time
+constexpr int kDraw = 4 + kMaxRot;  // doubles per position: O and orientations, generator states
+
+// The reference's generator (src/rndmod.f90:26-35): seed <- mod(8192 seed, 67099547).
+constexpr double kRndMod = 67099547.0, kRndScale = 1.4903230270690e-8;
+
+// Its states one after the other, drawn ahead 1,024 at a time: from an integer state (what any integer seed
+// gives) eight interleaved chains of integer arithmetic, each eight steps a turn, with the same values
+// as fmod one by one, whose latency was most of a call (40 ns a number, 4.3 ms of a call with 2,000 positions).
+class Generator {
+public:
+    explicit Generator(double seed) : last_(seed) {}
+    double state() {
+        if (k_ == kAhead) fill();
+        return buf_[k_++];
+    }
+    double number() { return state() * kRndScale; }
+
+private:
+    static constexpr int kAhead = 1024;
+    void fill() {
+        constexpr uint64_t M = 67099547;
+        const double first = std::fmod(8192.0 * last_, kRndMod);
+        if (first >= 0.0 && first == std::floor(first)) {
+            uint64_t x[8] = {(uint64_t)first}, a = 8192;  // products stay below 2^52
+            for (int i = 1; i < 8; ++i) {
+                x[i] = x[i - 1] * 8192 % M;
+                a = a * 8192 % M;
+            }
+            for (int k = 0; k < kAhead; k += 8)
+                for (int i = 0; i < 8; ++i) {
+                    buf_[k + i] = (double)x[i];
+                    x[i] = x[i] * a % M;
+                }
+        } else {
+            buf_[0] = first;
+            for (int k = 1; k < kAhead; ++k) buf_[k] = std::fmod(8192.0 * buf_[k - 1], kRndMod);
+        }
+        last_ = buf_[kAhead - 1];
+        k_ = 0;
+    }
+    double last_, buf_[kAhead];
+    int k_ = kAhead;
+};
 
 struct WArgs {
-    const double4* pos;   // O position per insertion (w: unused)
+    const double4* pos;   // O position per insertion, w: its orientations
     const double* rot;    // [ins][kMaxRot][6]: H1 x y z, H2 x y z (the reference's rins(2,:), rins(3,:))
-    const int* nrot;      // orientations per insertion
     double2* res;         // (sum exp(-beta u), status: 0 accepted, 1 overlap, 2 neighbour overflow)
     const int3* kvec;     // k set in the reference's order
-    const double* ak;
-    const double2* sk;    // moving-site S(k) of the last evaluation
-    const double2* qw;    // wall S(k)
     const double* lr;     // [9][nit] wall tail tables
     int nk, KL, KM, KN;
     double pipix, pipiy, pipiz;
@@ -103,6 +146,33 @@ __device__ double block_sum_d(double x, double* red) {
     return s;
 }
 
+// Orientations (src/forcem.f90:1345-1377) from the generator's state at the first of their four numbers.
+__global__ void k_widom_rot(const double4* __restrict__ pos, const double* __restrict__ states, double* __restrict__ rot,
+                            int nins) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, ins = t / kMaxRot;
+    if (ins >= nins) return;
+    const double4 o = pos[ins];
+    if (t - ins * kMaxRot >= (int)o.w) return;
+    double sd = states[t], h1[3];
+    for (int d = 0; d < 3; ++d) {
+        h1[d] = sd * kRndScale - 0.5;
+        sd = fmod(8192.0 * sd, kRndMod);
+    }
+    double ri = 1.0 / sqrt(h1[0] * h1[0] + h1[1] * h1[1] + h1[2] * h1[2]);
+    for (int d = 0; d < 3; ++d) h1[d] *= ri;
+    ri = 1.0 / sqrt(h1[0] * h1[0] + h1[1] * h1[1]);
+    const double h2[3] = {-h1[1] * ri, h1[0] * ri, 0.0};
+    const double mr[3] = {h2[1] * h1[2] - h2[2] * h1[1], h2[2] * h1[0] - h2[0] * h1[2], h2[0] * h1[1] - h2[1] * h1[0]};
+    const double alph = 2.0 * (double)3.1415926535898f * (sd * kRndScale);
+    double sina, cosa;
+    sincos(alph, &sina, &cosa);
+    const double aco = (double)-0.333333f, asi = (double)0.942809f, oo[3] = {o.x, o.y, o.z};
+    for (int d = 0; d < 3; ++d) {
+        rot[6 * (size_t)t + d] = oo[d] + aco * h1[d] + asi * (cosa * h2[d] + sina * mr[d]);
+        rot[6 * (size_t)t + 3 + d] = oo[d] + h1[d];
+    }
+}
+
 // The O's wall tail (src/forcem.f90:1481-1494).
 __device__ double wall_tail(const View& v, const double* lr, double oz) {
     const int nit = v.nit;
@@ -136,7 +206,7 @@ struct W64 {
     double* xyz;     // points: x, y, z, stride apart
     double* phi;     // reciprocal potential at the points
     size_t stride;
-    float lx, lxi, ly, lyi, rcut, near2, far2;  // below near2: certainly an overlap; above far2: certainly outside
+    float lx, lxi, ly, lyi, near2, far2;  // below near2: certainly an overlap; above far2: certainly outside
 };
 
 __global__ void k_widom_atoms(View v, W64 s) {
@@ -155,7 +225,7 @@ __global__ void __launch_bounds__(kRT) k_widom_real(View v, WArgs w, W64 s) {
     __shared__ int s_nc, s_nw, s_no, s_flag, s_off;
     const int ins = blockIdx.x, t = threadIdx.x, lane = t & 31;
     const double4 o = w.pos[ins];
-    const int nr = w.nrot[ins];
+    const int nr = (int)o.w;
     if (t == 0) s_nc = s_nw = s_no = s_flag = 0;
     if (t < kMaxRot) su[t] = 0.0;
     __syncthreads();
@@ -292,7 +362,7 @@ __global__ void k_widom_sum(View v, WArgs w, W64 s, int nins) {
     const int ins = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, r = threadIdx.x & 31;
     if (ins >= nins || w.res[ins].y != 0.0) return;
     double e = 0.0;
-    if (r < w.nrot[ins]) {
+    if (r < (int)w.pos[ins].w) {
         const double* rr = w.rot + ((size_t)ins * kMaxRot + r) * 6;
         const double* phi = s.phi + s.off[ins];
         const double oz = w.pos[ins].z;
@@ -372,7 +442,7 @@ __global__ void __launch_bounds__(kWT) k_widom(View v, WArgs w) {
     }
     const double qs3[3] = {w.q0, w.q1, w.q1};
     double acc = 0.0;
-    const int nr = w.nrot[ins];
+    const int nr = (int)o.w;
     for (int r = 0; r < nr; ++r) {
         const double* rr = w.rot + ((size_t)ins * kMaxRot + r) * 6;
         const double sx[3] = {ox, rr[0], rr[3]}, sy[3] = {oy, rr[1], rr[4]}, sz[3] = {oz, rr[2], rr[5]};
@@ -468,12 +538,6 @@ __global__ void __launch_bounds__(kWT) k_widom(View v, WArgs w) {
     if (t == 0) w.res[ins] = make_double2(acc, 0.0);
 }
 
-// The reference's generator: seed <- mod(8192 seed, 67099547), rnd = seed * 1.4903230270690e-8.
-inline double rnd(double& seed) {
-    seed = std::fmod(8192.0 * seed, 67099547.0);
-    return seed * 1.4903230270690e-8;
-}
-
 }  // namespace
 
 int widom(Ctx& c, const mdg_widom_params* p, double* seed, double* pave, int64_t* inave, int64_t* done) {
@@ -492,86 +556,35 @@ int widom(Ctx& c, const mdg_widom_params* p, double* seed, double* pave, int64_t
     const double chtemper = p->temper > 0.0 ? p->temper : 300.0;
     const double beta = 1000.0 / ((double)8.31441f * chtemper);
     const double M_PI_R = (double)3.1415926535898f;
-    const double aco = (double)-0.333333f, asi = (double)0.942809f;
-    // draw the positions and orientations in the reference's order (src/forcem.f90:1256-1377)
-    std::vector<double> hp(4 * nins), hr((size_t)nins * kMaxRot * 6, 0.0), seed_pos(nins), seed_rot(nins);
-    std::vector<int> hn(nins), hil(nins);
-    double sd = *seed;
-    for (int64_t ic = 0; ic < nins; ++ic) {
-        const double oxr = (rnd(sd) - 0.5) * v.lx;
-        const double oyr = (rnd(sd) - 0.5) * v.ly;
-        double ozr;
-        for (int guard = 0;; ++guard) {
-            ozr = ((rnd(sd) - 0.5) * zhi * 2.0);
-            if (std::fabs(ozr) > zlo) break;
-            if (guard > 100000000) return set_err(&c, MDG_E_ARG, "Widom insertion: empty band");
-        }
-        seed_pos[ic] = sd;
-        const int il = (int)((std::fabs(ozr) - zlo) * facbin) + 1;
-        if (il < 1 || il > p->lchmax) return set_err(&c, MDG_E_ARG, "Widom insertion: bin outside lchmax");
-        hil[ic] = il;
-        hn[ic] = il > p->ilmid ? 20 : 1;
-        hp[4 * ic] = oxr;
-        hp[4 * ic + 1] = oyr;
-        hp[4 * ic + 2] = ozr;
-        for (int ir = 0; ir < hn[ic]; ++ir) {
-            double h1[3], ri;
-            for (;;) {
-                h1[0] = rnd(sd) - 0.5;
-                h1[1] = rnd(sd) - 0.5;
-                h1[2] = rnd(sd) - 0.5;
-                ri = h1[0] * h1[0] + h1[1] * h1[1] + h1[2] * h1[2];
-                if (ri < 0.25 && ri > (double)0.001f) break;
-            }
-            ri = 1.0 / std::sqrt(ri);
-            for (double& hh : h1) hh = hh * ri;
-            ri = 1.0 / std::sqrt(h1[0] * h1[0] + h1[1] * h1[1]);
-            const double h2[3] = {-h1[1] * ri, h1[0] * ri, 0.0};
-            const double mr[3] = {h2[1] * h1[2] - h2[2] * h1[1], h2[2] * h1[0] - h2[0] * h1[2],
-                                  h2[0] * h1[1] - h2[1] * h1[0]};
-            const double alph = 2.0 * M_PI_R * rnd(sd);
-            const double cosa = std::cos(alph), sina = std::sin(alph);
-            const double o[3] = {oxr, oyr, ozr};
-            double* dst = &hr[((size_t)ic * kMaxRot + ir) * 6];
-            for (int d = 0; d < 3; ++d) {
-                dst[d] = o[d] + aco * h1[d] + asi * (cosa * h2[d] + sina * mr[d]);
-                dst[3 + d] = o[d] + h1[d];
-            }
-        }
-        seed_rot[ic] = sd;
-    }
-    // device scratch, grown on demand
+    // scratch: results grow on demand, the rest is sized for one chunk
     if (c.widom_cap < nins) {
         const int64_t cap = std::max<int64_t>(nins, 256);
-        c.d_widom_pos = (double*)dalloc(c, sizeof(double) * 4 * cap);
-        c.d_widom_rot = (double*)dalloc(c, sizeof(double) * cap * kMaxRot * 6);
-        c.d_widom_n = (int*)dalloc(c, sizeof(int) * cap);
         c.d_widom_res = (double*)dalloc(c, sizeof(double) * 2 * cap);
         if (c.alloc_failed) return set_err(&c, MDG_E_CUDA, "Widom insertion: out of device memory");
-        if (c.precision != MDG_MIXED) {
-            // real-space energies, points, potentials (doubles), first points and two counts (int)
-            c.d_widom_u = (double*)dalloc(c, (sizeof(double) * (kMaxRot + 4 * kPts) + sizeof(int)) * cap + 2 * sizeof(int));
-            if (!c.d_widom_pm) c.d_widom_pm = (double2*)dalloc(c, 2 * sizeof(double2) * std::max(ks.nent, 1));
-            if (!c.d_widom_atoms) c.d_widom_atoms = (float4*)dalloc(c, sizeof(float4) * std::max(v.ntota, 1));
-            if (c.alloc_failed) return set_err(&c, MDG_E_CUDA, "Widom insertion: out of device memory");
-        }
         c.widom_cap = cap;
     }
-    MDG_CUDA(cudaMemcpyAsync(c.d_widom_pos, hp.data(), sizeof(double) * 4 * nins, cudaMemcpyHostToDevice, c.stream));
-    MDG_CUDA(cudaMemcpyAsync(c.d_widom_rot, hr.data(), sizeof(double) * hr.size(), cudaMemcpyHostToDevice, c.stream));
-    MDG_CUDA(cudaMemcpyAsync(c.d_widom_n, hn.data(), sizeof(int) * nins, cudaMemcpyHostToDevice, c.stream));
+    if (!c.d_widom_draw) {
+        c.d_widom_rot = (double*)dalloc(c, sizeof(double) * kIns * kMaxRot * 6);
+        if (c.precision != MDG_MIXED) {
+            // real-space energies, points, potentials (doubles), first points and two counts (int)
+            c.d_widom_u = (double*)dalloc(c, (sizeof(double) * (kMaxRot + 4 * kPts) + sizeof(int)) * kIns + 2 * sizeof(int));
+            c.d_widom_pm = (double2*)dalloc(c, 2 * sizeof(double2) * std::max(ks.nent, 1));
+            c.d_widom_atoms = (float4*)dalloc(c, sizeof(float4) * std::max(v.ntota, 1));
+        }
+        c.d_widom_draw = (double*)dalloc(c, sizeof(double) * kIns * kDraw);
+        if (!c.alloc_failed && (cudaMallocHost(&c.h_widom_draw, sizeof(double) * 2 * kIns * kDraw) != cudaSuccess ||
+                                cudaEventCreateWithFlags(&c.widom_read[0], cudaEventDisableTiming) != cudaSuccess ||
+                                cudaEventCreateWithFlags(&c.widom_read[1], cudaEventDisableTiming) != cudaSuccess))
+            c.alloc_failed = true;
+        if (c.alloc_failed) return set_err(&c, MDG_E_CUDA, "Widom insertion: out of memory");
+    }
     double dipz = 0.0;
     if (p->flags & MDG_WIDOM_EW3DC)
         MDG_CUDA(cudaMemcpy(&dipz, v.acc + 2 * v.nijt + ACC_DIPZ, sizeof(double), cudaMemcpyDeviceToHost));
     WArgs w;
-    w.pos = reinterpret_cast<const double4*>(c.d_widom_pos);
+    w.pos = reinterpret_cast<const double4*>(c.d_widom_draw);
     w.rot = c.d_widom_rot;
-    w.nrot = c.d_widom_n;
-    w.res = reinterpret_cast<double2*>(c.d_widom_res);
     w.kvec = ks.kvec;
-    w.ak = ks.ak;
-    w.sk = ks.s;
-    w.qw = ks.qw;
     w.lr = c.d_lr;
     w.nk = ks.nk;
     w.KL = ks.klmax;
@@ -597,6 +610,7 @@ int widom(Ctx& c, const mdg_widom_params* p, double* seed, double* pave, int64_t
     w.qsf = nullptr;
     w.akf = nullptr;
     w.rsf = nullptr;
+    W64 s{};
     if (mx) {
         if (!c.d_widom_akf) {
             std::vector<float> akf(std::max(ks.nk, 1));
@@ -615,32 +629,87 @@ int widom(Ctx& c, const mdg_widom_params* p, double* seed, double* pave, int64_t
         w.qsf = c.d_widom_qsf;
         w.akf = c.d_widom_akf;
         w.rsf = c.d_widom_rsf;
-        k_widom<<<(unsigned)nins, kWT, smem, c.stream>>>(v, w);
     } else {
-        W64 s;
         s.atoms = c.d_widom_atoms;
-        s.stride = (size_t)kPts * c.widom_cap;
+        s.stride = (size_t)kPts * kIns;
         s.u = c.d_widom_u;
-        s.xyz = s.u + (size_t)kMaxRot * c.widom_cap;
+        s.xyz = s.u + (size_t)kMaxRot * kIns;
         s.phi = s.xyz + 3 * s.stride;
         s.off = reinterpret_cast<int*>(s.phi + s.stride);
-        s.cnt = s.off + c.widom_cap;
+        s.cnt = s.off + kIns;
         s.lx = (float)v.lx;
         s.ly = (float)v.ly;
         s.lxi = (float)v.lxi;
         s.lyi = (float)v.lyi;
-        s.rcut = (float)v.rcut;
         // FP32 rounding moves a squared distance r^2 by less than 4e-7 r (r + box edge)
         const double box = std::max(v.lx, std::max(v.ly, v.lz));
         s.far2 = (float)(v.rcutsq + 1e-5 * v.rcut * (v.rcut + box));
         s.near2 = (float)(std::min(w.rinsmin, v.rcutsq) - 1e-5 * 2.0 * (2.0 + box));
-        MDG_CUDA(cudaMemsetAsync(s.cnt, 0, 2 * sizeof(int), c.stream));
+        MDG_CUDA(cudaMemsetAsync(s.cnt, 0, sizeof(int), c.stream));
         k_widom_atoms<<<(v.ntota + 255) / 256, 256, 0, c.stream>>>(v, s);
         recip_pot_table(c, c.d_widom_pm, c.stream);
-        k_widom_real<<<(unsigned)nins, kRT, 0, c.stream>>>(v, w, s);
-        recip_potential(c, c.d_widom_pm, s.xyz, s.stride, s.cnt + 1, (int)(kPts * nins), (int)(kPts * nins / 2 + 1), s.phi,
-                        c.stream);
-        k_widom_sum<<<(unsigned)((nins + 7) / 8), 256, 0, c.stream>>>(v, w, s, (int)nins);
+    }
+    // Chunks: while the device evaluates one the host draws the next, positions and orientations in the
+    // reference's order (src/forcem.f90:1256-1377); the states that orientations are made from go to
+    // the device (192 bytes per position; the H positions were 964).
+    std::vector<double> seed_pos(nins), seed_rot(nins);
+    std::vector<int> hn(nins), hil(nins);
+    Generator g(*seed);
+    for (int64_t base = 0, chunk = 0; base < nins; base += kIns, ++chunk) {
+        const int n = (int)std::min<int64_t>(kIns, nins - base);
+        double* hp = c.h_widom_draw + (chunk & 1) * kIns * kDraw;
+        double* hs = hp + 4 * n;
+        if (chunk >= 2) MDG_CUDA(cudaEventSynchronize(c.widom_read[chunk & 1]));
+        for (int i = 0; i < n; ++i) {
+            const int64_t ic = base + i;
+            const double oxr = (g.number() - 0.5) * v.lx;
+            const double oyr = (g.number() - 0.5) * v.ly;
+            double ozr, sd;
+            for (int guard = 0;; ++guard) {
+                sd = g.state();
+                ozr = ((sd * kRndScale - 0.5) * zhi * 2.0);
+                if (std::fabs(ozr) > zlo) break;
+                if (guard > 100000000) {
+                    cudaStreamSynchronize(c.stream);
+                    return set_err(&c, MDG_E_ARG, "Widom insertion: empty band");
+                }
+            }
+            seed_pos[ic] = sd;
+            const int il = (int)((std::fabs(ozr) - zlo) * facbin) + 1;
+            if (il < 1 || il > p->lchmax) {
+                cudaStreamSynchronize(c.stream);
+                return set_err(&c, MDG_E_ARG, "Widom insertion: bin outside lchmax");
+            }
+            hil[ic] = il;
+            hn[ic] = il > p->ilmid ? 20 : 1;
+            hp[4 * i] = oxr;
+            hp[4 * i + 1] = oyr;
+            hp[4 * i + 2] = ozr;
+            hp[4 * i + 3] = hn[ic];
+            for (int ir = 0; ir < hn[ic]; ++ir) {
+                double first, ri;
+                do {
+                    first = g.state();
+                    const double a = first * kRndScale - 0.5, b = g.number() - 0.5, d = g.number() - 0.5;
+                    ri = a * a + b * b + d * d;
+                } while (!(ri < 0.25 && ri > (double)0.001f));
+                hs[(size_t)i * kMaxRot + ir] = first;
+                sd = g.state();
+            }
+            seed_rot[ic] = sd;
+        }
+        w.res = reinterpret_cast<double2*>(c.d_widom_res) + base;
+        MDG_CUDA(cudaMemcpyAsync(c.d_widom_draw, hp, sizeof(double) * kDraw * n, cudaMemcpyHostToDevice, c.stream));
+        MDG_CUDA(cudaEventRecord(c.widom_read[chunk & 1], c.stream));
+        k_widom_rot<<<(n * kMaxRot + 127) / 128, 128, 0, c.stream>>>(w.pos, c.d_widom_draw + 4 * n, c.d_widom_rot, n);
+        if (mx) {
+            k_widom<<<n, kWT, smem, c.stream>>>(v, w);
+        } else {
+            MDG_CUDA(cudaMemsetAsync(s.cnt + 1, 0, sizeof(int), c.stream));
+            k_widom_real<<<n, kRT, 0, c.stream>>>(v, w, s);
+            recip_potential(c, c.d_widom_pm, s.xyz, s.stride, s.cnt + 1, kPts * n, kPts * n / 2 + 1, s.phi, c.stream);
+            k_widom_sum<<<(n + 7) / 8, 256, 0, c.stream>>>(v, w, s, n);
+        }
     }
     MDG_CUDA(cudaGetLastError());
     std::vector<double> res(2 * nins);

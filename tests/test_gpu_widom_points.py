@@ -36,3 +36,20 @@ def test_too_many_sites_around_the_probe(gpulib):
     with pytest.raises(Exception, match="more than 1024 sites"):
         c.widom(200, 1.0, 3.0, 8, 8, SEED0, flags=abi.MDG_WIDOM_SKIP_OVERLAP)
     c.close()
+
+
+@pytest.mark.parametrize("nins,seed", [(512, SEED0), (513, SEED0), (1030, 67099546.0), (600, 12345.678), (300, 3.0e9 + 0.5)])
+def test_chunks_and_seeds(nins, seed, gpulib, oracle):
+    """Positions drawn in chunks, from integer states (drawn ahead) and others: the generator's state and the
+    counts are the oracle's to the bit."""
+    s, prm = configs.slab_water(nwat=64, cells=6, placement="lattice", kmax=3)
+    out = []
+    for lib in (gpulib, oracle):
+        c = abi.Context(lib, s.copy(), prm)
+        c.force_get(s.copy())
+        out.append(c.widom(nins, 1.0, 2.0, 5, 4, seed, flags=abi.MDG_WIDOM_SKIP_OVERLAP))
+        c.close()
+    a, b = out
+    assert a["done"] == b["done"] == nins and a["seed"] == b["seed"]
+    np.testing.assert_array_equal(a["inave"], b["inave"])
+    assert np.abs(a["pave"] - b["pave"]).max() <= 1e-9 * max(b["pave"].max(), 1e-300)
