@@ -110,32 +110,55 @@ struct KSet {
     std::vector<int> h_nlen;
 };
 
-// Device arrays and sizes of the gridded reciprocal sum (recip_nu.cu), passed to kernels by value.
-struct NuView {
+// Pairs and quads of a gridded sum's numbers.
+template <typename T>
+struct NuVec;
+template <>
+struct NuVec<float> {
+    typedef float2 V2;
+    typedef float4 V4;
+};
+template <>
+struct NuVec<double> {
+    typedef double2 V2;
+    struct __align__(16) V4 {
+        double x, y, z, w;
+    };
+};
+
+// Device arrays and sizes of a gridded reciprocal sum (recip_nu.cu in FP32, recip_nu64.cu in FP64), passed
+// to kernels by value.
+template <typename T>
+struct NuViewT {
+    typedef typename NuVec<T>::V2 V2;
     int M[3], K[3];          // grid points and largest frequency per direction
     int n8[3], nblk;         // blocks of 8 x 8 x 8 cells
     int cap, split, ngrp, mgrp, ygrp, yrows;
-    float scale[3];          // d(grid coordinate)/d(position), with the reference's pi
+    T scale[3];              // d(grid coordinate)/d(position), with the reference's pi
     int* cnt = nullptr;      // atoms per block (beyond cap: in ovf), then those in ovf; 0 between evaluations
     int* cntf = nullptr;     // the same counts for the force kernel
     int* bucket = nullptr;   // their indices, cap per block
     int* novf = nullptr;     // cnt + nblk: atoms that found their bucket full
     int* ovf = nullptr;      // their indices
-    float* grid = nullptr;   // charges [x][y][z], zero between evaluations
-    float* pot = nullptr;    // potential [x][y][z]
-    float2* H = nullptr;     // [n][x][m + KM]
-    float2 *tw[3], *twt[3];  // twiddles by (point, frequency) and by (frequency, point)
+    T* grid = nullptr;       // charges [x][y][z], zero between evaluations
+    T* pot = nullptr;        // potential [x][y][z]
+    V2* H = nullptr;         // [n][x][m + KM]
+    V2 *tw[3], *twt[3];      // twiddles by (point, frequency) and by (frequency, point)
     double* dec[3];          // 1 / transform of the spreading window, then of the force window
     int* kmap = nullptr;     // [n][m + KM][l + KL]: 2 k + (conjugate), or -1
     double2* S = nullptr;    // the k set's arrays (KSet)
     const double2* qw = nullptr;
     const double* ak = nullptr;
 };
-struct NuPlan {
+typedef NuViewT<float> NuView;
+template <typename T>
+struct NuPlanT {
     bool ready = false;
-    NuView g{};
+    NuViewT<T> g{};
     int smem_zy = 0, smem_x = 0, smem_yz = 0;
+    double2* rec = nullptr;  // FP64 form: grid coordinates and charge of each place in a bucket, then of ovf
 };
+typedef NuPlanT<float> NuPlan;
 
 // Per-step packed atom records of the mixed-precision real-space kernels (pair_mx.cu).
 struct Pk {
@@ -209,6 +232,7 @@ struct Ctx {
     KSet ks;
     TcPlan tcp;
     NuPlan nu;
+    NuPlanT<double> nu64;
     Pk pk;
     uint4* d_tc_atoms = nullptr;        // fixed-point phases + charge per moving atom
     unsigned char* d_tc_img = nullptr;  // packed C(k) operand chunks
@@ -370,6 +394,8 @@ int recip_tc_throughput(Ctx& c, bool on);
 void recip_tc(Ctx& c);  // (or the gridded sum, by the size of the system)
 // recip_nu.cu
 int recip_nu_setup(Ctx& c);
+int recip_nu64_setup(Ctx& c);
+void recip_nu64(Ctx& c);
 void recip_nu(Ctx& c);
 int umma_selftest(int n, int k, const float* a, const float* b, float* d, std::string& err);
 // mlp.cu

@@ -578,6 +578,10 @@ int mdg_create(const mdg_sysdesc* s, const mdg_params* p, const double* x0, cons
     if (rc) return bail(rc);
     rc = recip_setup(c, p->kmax, x0, y0, z0);
     if (rc) return bail(rc);
+    if (c.precision != MDG_MIXED) {
+        rc = recip_nu64_setup(c);
+        if (rc) return bail(rc);
+    }
     if (c.precision == MDG_MIXED) {
         rc = recip_tc_setup(c);
         if (rc) return bail(rc);

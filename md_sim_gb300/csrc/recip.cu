@@ -25,8 +25,9 @@
 //                rows are dealt to as many grid rows as give every SM work when atoms are few.
 // 2,048-water slab (6,144 atoms, 4,338 k): k_sfac 586 -> 204 us, k_kforce 1,778 -> 290 us against the
 // form with complex products, items of 8 n, 256-thread blocks and one thread per atom over all rows;
-// a force call at 32,768 waters (29,038 k) 115.7 -> 48.6 ms, of which k_kforce 27 ms, its FMAs at
-// the 0.5 TFMA/s that a loop of independent FP64 FMAs reaches on this part.
+// 32,768 waters (29,038 k) 112 -> 44 ms, of which k_kforce 27 ms, its FMAs at the 0.5 TFMA/s that a loop of
+// independent FP64 FMAs reaches on this part.  From 5e6 (atom, k) on contexts take the gridded sum of
+// recip_nu64.cu instead; mdg_recip_forces_noalloc always runs these.
 #include <algorithm>
 #include <cmath>
 #include <complex>
@@ -504,6 +505,10 @@ void recip_fp64(Ctx& c) {
     const View& v = c.v;
     KSet& ks = c.ks;
     if (ks.nk == 0 || v.nmove == 0) return;
+    if (c.nu64.ready) {
+        recip_nu64(c);
+        return;
+    }
     KDims d{ks.klmax, ks.kmmax, ks.knmax, ks.pipix, ks.pipiy, ks.pipiz};
     const KGrid g = k_grid(d, v.nmove, ks.nrow, ks.nwork);
     cudaMemsetAsync(ks.s, 0, sizeof(double2) * ks.nk, c.stream);
