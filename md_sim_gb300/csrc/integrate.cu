@@ -8,10 +8,15 @@
 //            uconf and press of force_sum (src/forcem.f90:1055,1079,1081) and the thermostat
 //            corrector.
 //
-// One thread per ion or molecule in small blocks (the FP64 work of one molecule is a long
-// dependent chain, so the molecules are spread over as many SMs as possible); kinetic sums go
-// through block reductions into a small accumulator array that the last block reads and clears.
-// Gear coefficients are the reference's single-precision literals.
+// Systems of more than 80 molecules per SM: one thread per ion or molecule in blocks of four warps, where
+// FP64 operations bound them.  Smaller ones (k_pred_small, k_corr_small): what bounds these is the chain of
+// dependent instructions of one molecule (a warp issued one instruction per 14 clocks), so a block of five
+// warps takes 16 molecules and a thread one component of one of them (3 of the centre, 3 of the angular
+// velocity, 4 of the quaternion) through the Gear arithmetic, the forces of one site, the placing and
+// packing of one atom: 2,048 waters between walls k_pred 16.4 -> 8.1 us, k_corr 17.3 -> 9.8 us against two
+// lanes per molecule with 14 molecules per warp; 20 resident steps 1.99 -> 1.73 ms.
+// Kinetic sums go through reductions into a small accumulator array that the last block reads and
+// clears.  Gear coefficients are the reference's single-precision literals.
 #include <algorithm>
 #include <cmath>
 
@@ -24,31 +29,12 @@ namespace mdg {
 
 namespace {
 
-// A warp serves `lanes` molecules. An FP64 instruction costs the SM's FP64 pipe about the same
-// whatever the number of active lanes, so large systems pack 32 molecules per warp (blocks of four
-// warps); small ones spread one warp per SM with just enough molecules to cover the system, since
-// there the per-molecule chain of dependent FP64 operations sets the time, and with at most 16
-// molecules per warp each molecule takes a pair of lanes (centre and angular velocity on one,
-// orientation on the other) to shorten that chain.
 constexpr int kSM = 152;
 
-// unit served by this thread in sweep `r` of the grid-stride loop over the first `nb` blocks, or -1
+// unit served by this thread in sweep `r` of the grid-stride loop over the first `nb` blocks
 template <int NT>
-__device__ __forceinline__ int unit_of(int lanes, int r, int nb) {
-    const int lane = threadIdx.x & 31;
-    if (lane >= lanes) return -1;
-    const int gw = blockIdx.x * (NT / 32) + (threadIdx.x >> 5);
-    return (r * nb * (NT / 32) + gw) * lanes + lane;
-}
-
-// the same for lane pairs (two lanes per unit, `lanes` units per warp, lanes <= 16): role = lane & 1
-template <int NT>
-__device__ __forceinline__ int unit_of_pair(int lanes, int r, int nb, int& role) {
-    const int lane = threadIdx.x & 31, slot = lane >> 1;
-    role = lane & 1;
-    if (slot >= lanes) return -1;
-    const int gw = blockIdx.x * (NT / 32) + (threadIdx.x >> 5);
-    return (r * nb * (NT / 32) + gw) * lanes + slot;
+__device__ __forceinline__ int unit_of(int r, int nb) {
+    return (r * nb + blockIdx.x) * NT + threadIdx.x;
 }
 
 constexpr double Gf01 = F32D(0.348611111), Gf11 = 1.0, Gf21 = F32D(0.916666667), Gf31 = F32D(0.333333333),
@@ -112,9 +98,6 @@ __device__ __forceinline__ bool last_block(unsigned* done) {
     __syncthreads();
     return last;
 }
-
-// Register arithmetic of the rigid-body predictor and corrector, shared by the one-lane forms and
-// the lane-pair forms below (the same operations in the same order, so both give the same bits).
 
 // rotation matrix of the normalised predicted quaternion (src/move.f90:128-146)
 __device__ __forceinline__ void quat_rot(const double* qq, double* qn, double* a) {
@@ -226,52 +209,6 @@ __device__ __forceinline__ void pred_rigid(const View& v, const Dyn& D, int i, d
     }
 }
 
-// The same on a pair of lanes (mask: the lanes of the pairs on rigid molecules this sweep): role 0
-// predicts the centre and angular velocity, role 1 the orientation; after the exchange of the
-// centre and the rotation matrix, role 0 places sites 0 and 1, role 1 sites 0 and 2 (returned in
-// slots 0 and 1; each writes its own besides site 0, which role 0 writes).
-__device__ __forceinline__ void pred_rigid_pair(const View& v, const Dyn& D, int i, int role, unsigned mask,
-                                                double* sc, double* sw, double* cn, double* sx, double* sy,
-                                                double* sz) {
-    const int nr = v.nrig;
-    double a[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    cn[0] = cn[1] = cn[2] = 0.0;
-    if (role == 0) {
-        double C[5][3], W[5][3];
-        load_cw(D, nr, i, C, W);
-        pred_cw(D, nr, i, C, W, sc, sw, cn);
-    } else {
-        double Q[5][4];
-        load_q(D, nr, i, Q);
-        pred_q(D, nr, i, Q, a);
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const double t = __shfl_xor_sync(mask, role ? a[k] : cn[k], 1);
-        if (role) cn[k] = t;
-        else a[k] = t;
-    }
-#pragma unroll
-    for (int k = 3; k < 9; ++k) {
-        const double t = __shfl_xor_sync(mask, a[k], 1);
-        if (!role) a[k] = t;
-    }
-    const int ix = 3 * i, j1 = role ? 2 : 1;
-    site_pos(cn, a, D.body, 0, sx[0], sy[0], sz[0]);
-    site_pos(cn, a, D.body, j1, sx[1], sy[1], sz[1]);
-    if (role == 0) {
-        v.x[ix] = sx[0];
-        v.y[ix] = sy[0];
-        v.z[ix] = sz[0];
-    }
-    v.x[ix + j1] = sx[1];
-    v.y[ix + j1] = sy[1];
-    v.z[ix + j1] = sz[1];
-    v.rsx[ix + j1] = sx[1] - sx[0];
-    v.rsy[ix + j1] = sy[1] - sy[0];
-    v.rsz[ix + j1] = sz[1] - sz[0];
-}
-
 // thermostat predictor and kinetic energies from the summed isum[0..6] (one thread).  Runs in the
 // tail of a kernel, where every dependent round trip to L2 is about a microsecond: all loads are
 // issued first, into registers, then the arithmetic, then the stores.
@@ -347,78 +284,73 @@ struct PackArgs {
 // A packing predictor has no tail: block 0 clears the energy sums first (all but the displacement
 // maximum, which the blocks raise as they go), and the close of the packing and the thermostat
 // predictor run in k_step_close on the list's stream, off the path of the reciprocal sum.
-template <int NT, bool PACK, bool PAIR>
-__global__ void __launch_bounds__(NT) k_pred(View v, Dyn D, int lanes, Clear z, PackArgs P) {
+//
+// First block of a predictor: the sums that the step adds to.
+template <bool PACK>
+__device__ __forceinline__ void pred_clear(const View& v, const Clear& z, const PackArgs& P) {
+    for (int j = 0; j < 2; ++j)
+        for (int k = threadIdx.x; k < z.n[j]; k += blockDim.x) z.p[j][k] = 0.0;
+    if constexpr (PACK) {
+        const int na = 2 * v.nijt + ACC_NSLOT, kmax = 2 * v.nijt + ACC_MAXD;
+        for (int k = threadIdx.x; k < na; k += blockDim.x)
+            if (k != kmax) v.acc[k] = 0.0;
+        if (P.pk.cmax && threadIdx.x == 0) *P.pk.cmax = 0.f;
+    }
+}
+
+// ion u with its record; its share of kp, the dipole and the displacement maximum
+template <bool PACK>
+__device__ __forceinline__ void pred_ion_pack(const View& v, const Dyn& D, const PackArgs& P, int u, double& kp, double& mz,
+                                              double& md) {
+    double xn[3];
+    kp += pred_ion(v, D, u, xn);
+    if constexpr (PACK) {
+        const int at = v.nriga + u;
+        const double a = v.ox[u] - xn[0], b = v.oy[u] - xn[1], c = v.oz[u] - xn[2];
+        md = fmax(md, a * a + b * b + c * c);
+        mz += pack_atom(v, P.pk, at, xn[0], xn[1], xn[2], v.rsx[at], v.rsy[at], v.rsz[at], true);
+    }
+}
+
+template <bool PACK, int NT>
+__device__ __forceinline__ void pred_end(const View& v, const Dyn& D, const PackArgs& P, double mz, double md, double* red) {
+    if constexpr (PACK) {
+        pack_block(v, P.pk, mz, md, red);
+    } else if (last_block(&D.done[0]) && threadIdx.x == 0) {
+        thermo_pred(v, D, thermo_pred_load(D));
+        D.done[0] = 0u;
+    }
+}
+
+template <int NT, bool PACK>
+__global__ void __launch_bounds__(NT) k_pred(View v, Dyn D, Clear z, PackArgs P) {
     __shared__ double red[8];
     double kp = 0.0, sc[3] = {0, 0, 0}, sw[3] = {0, 0, 0};
     double mz = 0.0, md = 0.0;
     const int nu = D.nion + v.nrig;
     const int npred = PACK ? P.npred : gridDim.x;
-    if (blockIdx.x == 0) {
-        for (int j = 0; j < 2; ++j)
-            for (int k = threadIdx.x; k < z.n[j]; k += NT) z.p[j][k] = 0.0;
-        if constexpr (PACK) {
-            const int na = 2 * v.nijt + ACC_NSLOT, kmax = 2 * v.nijt + ACC_MAXD;
-            for (int k = threadIdx.x; k < na; k += NT)
-                if (k != kmax) v.acc[k] = 0.0;
-            if (P.pk.cmax && threadIdx.x == 0) *P.pk.cmax = 0.f;
-        }
-    }
+    if (blockIdx.x == 0) pred_clear<PACK>(v, z, P);
     if (blockIdx.x < npred) {
         for (int r = 0;; ++r) {
-            int u, role = 0;
-            if constexpr (PAIR) u = unit_of_pair<NT>(lanes, r, npred, role);
-            else u = unit_of<NT>(lanes, r, npred);
-            const bool act = u >= 0 && u < nu;
-            unsigned mask = 0u;
-            if constexpr (PAIR) {
-                if (!__any_sync(0xffffffffu, act)) break;
-                mask = __ballot_sync(0xffffffffu, act && u >= D.nion);
-                if (!act) continue;
-            } else {
-                if (!act) break;
-            }
+            const int u = unit_of<NT>(r, npred);
+            if (u >= nu) break;
             if (u < D.nion) {
-                if (role != 0) continue;
-                double xn[3];
-                kp += pred_ion(v, D, u, xn);
-                if constexpr (PACK) {
-                    const int at = v.nriga + u;
-                    const double a = v.ox[u] - xn[0], b = v.oy[u] - xn[1], c = v.oz[u] - xn[2];
-                    md = fmax(md, a * a + b * b + c * c);
-                    mz += pack_atom(v, P.pk, at, xn[0], xn[1], xn[2], v.rsx[at], v.rsy[at], v.rsz[at], true);
-                }
+                pred_ion_pack<PACK>(v, D, P, u, kp, mz, md);
                 continue;
             }
             const int i = u - D.nion, ix = 3 * i;
             double cn[3], px[3], py[3], pz[3];
-            if constexpr (PAIR) {
-                pred_rigid_pair(v, D, i, role, mask, sc, sw, cn, px, py, pz);
-                if constexpr (PACK) {
-                    // site 0's offset is the stored one (force_sum leaves rsx(1:3) stale), the others
-                    // the offsets just computed, as the packing kernel would read them back
-                    if (role == 0) {
-                        const double a = v.ocx[i] - cn[0], b = v.ocy[i] - cn[1], c = v.ocz[i] - cn[2];
-                        md = fmax(md, a * a + b * b + c * c);
-                        mz += pack_atom(v, P.pk, ix, px[0], py[0], pz[0], v.rsx[ix], v.rsy[ix], v.rsz[ix], true);
-                        mz += pack_atom(v, P.pk, ix + 1, px[1], py[1], pz[1], px[1] - px[0], py[1] - py[0],
-                                        pz[1] - pz[0], true);
-                    } else {
-                        mz += pack_atom(v, P.pk, ix + 2, px[1], py[1], pz[1], px[1] - px[0], py[1] - py[0],
-                                        pz[1] - pz[0], true);
-                    }
-                }
-            } else {
-                pred_rigid(v, D, i, sc, sw, cn, px, py, pz);
-                if constexpr (PACK) {
-                    const double a = v.ocx[i] - cn[0], b = v.ocy[i] - cn[1], c = v.ocz[i] - cn[2];
-                    md = fmax(md, a * a + b * b + c * c);
-                    mz += pack_atom(v, P.pk, ix, px[0], py[0], pz[0], v.rsx[ix], v.rsy[ix], v.rsz[ix], true);
+            pred_rigid(v, D, i, sc, sw, cn, px, py, pz);
+            if constexpr (PACK) {
+                // site 0's offset is the stored one (force_sum leaves rsx(1:3) stale), the others
+                // the offsets just computed, as the packing kernel would read them back
+                const double a = v.ocx[i] - cn[0], b = v.ocy[i] - cn[1], c = v.ocz[i] - cn[2];
+                md = fmax(md, a * a + b * b + c * c);
+                mz += pack_atom(v, P.pk, ix, px[0], py[0], pz[0], v.rsx[ix], v.rsy[ix], v.rsz[ix], true);
 #pragma unroll
-                    for (int j = 1; j < 3; ++j)
-                        mz += pack_atom(v, P.pk, ix + j, px[j], py[j], pz[j], px[j] - px[0], py[j] - py[0],
-                                        pz[j] - pz[0], true);
-                }
+                for (int j = 1; j < 3; ++j)
+                    mz += pack_atom(v, P.pk, ix + j, px[j], py[j], pz[j], px[j] - px[0], py[j] - py[0],
+                                    pz[j] - pz[0], true);
             }
         }
     } else if constexpr (PACK) {
@@ -431,12 +363,112 @@ __global__ void __launch_bounds__(NT) k_pred(View v, Dyn D, int lanes, Clear z, 
         for (int d = 0; d < 3; ++d) block_atomic_sum<NT>(sc[d], &D.isum[1 + d]);
         for (int d = 0; d < 3; ++d) block_atomic_sum<NT>(sw[d], &D.isum[4 + d]);
     }
-    if constexpr (PACK) {
-        pack_block(v, P.pk, mz, md, red);
-    } else if (last_block(&D.done[0]) && threadIdx.x == 0) {
-        thermo_pred(v, D, thermo_pred_load(D));
-        D.done[0] = 0u;
+    pred_end<PACK, NT>(v, D, P, mz, md, red);
+}
+
+// ---- small systems -----------------------------------------------------------------------------
+constexpr int kMol = 16, kComp = 10, kST = kMol * kComp;  // molecules, components, threads of a block
+constexpr int kFlex = 32;                                 // ions or surface atoms of a block that takes those
+
+// Component k of molecule i: its derivatives are st apart from the returned pointer on.
+__device__ __forceinline__ double* component(const Dyn& D, int nr, int i, int k, int& st) {
+    st = k < 6 ? 3 * nr : nr;
+    return (k < 3 ? D.c + (size_t)k * nr : k < 6 ? D.w + (size_t)(k - 3) * nr : D.q + (size_t)(k - 6) * 5 * nr) + i;
+}
+
+// Sum over the 16 lanes of a component.
+__device__ __forceinline__ double sum16(double x) {
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
+}
+
+// Blocks below nrb: 16 molecules each; below nrb + nfb: ions; then (PACK) wall atoms.
+template <bool PACK>
+__global__ void __launch_bounds__(kST) k_pred_small(View v, Dyn D, Clear z, PackArgs P, int nrb, int nfb) {
+    __shared__ double red[8], s_c[3][kMol], s_q[4][kMol], s_a[9][kMol];
+    double mz = 0.0, md = 0.0;
+    const int t = threadIdx.x;
+    if (blockIdx.x == 0) pred_clear<PACK>(v, z, P);
+    if (blockIdx.x < nrb) {
+        const int m = t & (kMol - 1), k = t / kMol, nr = v.nrig, i = blockIdx.x * kMol + m;
+        const bool act = i < nr;
+        int st;
+        double* b = component(D, nr, act ? i : 0, k, st);
+        double a0 = b[0], a1 = b[st], a2 = b[2 * st], a3 = b[3 * (size_t)st];
+        gpred(a0, a1, a2, a3, b[4 * (size_t)st]);
+        if (k < 3) s_c[k][m] = a0;
+        if (k >= 6) s_q[k - 6][m] = a0;
+        __syncthreads();
+        if (act) {
+            if (k < 6) b[0] = a0;
+            b[st] = a1;
+            b[2 * st] = a2;
+            b[3 * (size_t)st] = a3;
+        }
+        if (t >= kST - 32) {  // the warp with the last two quaternion components: no kinetic sums there
+            if (t < kST - kMol) {
+                double qq[4], qn[4], a[9];
+#pragma unroll
+                for (int cc = 0; cc < 4; ++cc) qq[cc] = s_q[cc][m];
+                quat_rot(qq, qn, a);
+#pragma unroll
+                for (int e = 0; e < 9; ++e) s_a[e][m] = a[e];
+                if (act)
+#pragma unroll
+                    for (int cc = 0; cc < 4; ++cc) D.q[(size_t)(cc * 5) * nr + i] = qn[cc];
+            }
+        } else {
+            const double x = k < 3 ? a1 : a0;  // d/dt of the centre, angular velocity
+            const double s = sum16(act && k < 6 ? x * x : 0.0);
+            if (m == 0 && k < 6) atomicAdd(&D.isum[1 + k], s);
+        }
+        __syncthreads();
+        if (act && k < 9) D.a[(size_t)k * nr + i] = s_a[k][m];
+        if (act && k < 3) {
+            double cn[3], a[9], p0[3], p[3];
+#pragma unroll
+            for (int d = 0; d < 3; ++d) cn[d] = s_c[d][m];
+#pragma unroll
+            for (int e = 0; e < 9; ++e) a[e] = s_a[e][m];
+            const int ix = 3 * i;
+            site_pos(cn, a, D.body, 0, p0[0], p0[1], p0[2]);
+            site_pos(cn, a, D.body, k, p[0], p[1], p[2]);
+            v.x[ix + k] = p[0];
+            v.y[ix + k] = p[1];
+            v.z[ix + k] = p[2];
+            double rx = 0.0, ry = 0.0, rz = 0.0;
+            if (k > 0) {
+                v.rsx[ix + k] = rx = p[0] - p0[0];
+                v.rsy[ix + k] = ry = p[1] - p0[1];
+                v.rsz[ix + k] = rz = p[2] - p0[2];
+            }
+            if constexpr (PACK) {
+                if (k == 0) {
+                    // site 0's offset is the stored one (force_sum leaves rsx(1:3) stale)
+                    rx = v.rsx[ix];
+                    ry = v.rsy[ix];
+                    rz = v.rsz[ix];
+                    const double dx = v.ocx[i] - cn[0], dy = v.ocy[i] - cn[1], dz = v.ocz[i] - cn[2];
+                    md = dx * dx + dy * dy + dz * dz;
+                }
+                mz = pack_atom(v, P.pk, ix + k, p[0], p[1], p[2], rx, ry, rz, true);
+            }
+        }
+    } else if (blockIdx.x < nrb + nfb) {
+        const int u = (blockIdx.x - nrb) * kFlex + t;
+        double kp = 0.0;
+        if (t < kFlex && u < D.nion) pred_ion_pack<PACK>(v, D, P, u, kp, mz, md);
+        if (t < kFlex) {
+            kp = warp_sum(kp);
+            if (t == 0) atomicAdd(&D.isum[0], kp);
+        }
+    } else if constexpr (PACK) {
+        const int b0 = nrb + nfb, nw = gridDim.x - b0;
+        for (int a = v.nmove + (blockIdx.x - b0) * kST + t; a < v.ntota; a += nw * kST)
+            pack_atom(v, P.pk, a, v.x[a], v.y[a], v.z[a], 0.0, 0.0, 0.0, false);
     }
+    pred_end<PACK, kST>(v, D, P, mz, md, red);
 }
 
 // After a packing predictor (one block of two warps): the close of its packing (slab dipole from
@@ -558,33 +590,6 @@ __device__ __forceinline__ void corr_rigid(const View& v, const Dyn& D, int i) {
     corr_cw(D, nr, i, C, W, a, fc, tq, s0i, rs0i);
 }
 
-// The same on a pair of lanes: role 0 corrects the centre and angular velocity (with fc, tq),
-// role 1 the orientation, with the predicted angular velocity passed over from role 0.
-__device__ __forceinline__ void corr_rigid_pair(const View& v, const Dyn& D, int i, int role, unsigned mask,
-                                                const double* fc, const double* tq) {
-    const int nr = v.nrig;
-    const double s0i = D.th[TH_S], rs0i = D.th[TH_RS];
-    double C[5][3], W[5][3], Q[5][4], a[9];
-    double w0[3] = {0.0, 0.0, 0.0};
-    if (role == 0) {
-        load_cw(D, nr, i, C, W);
-#pragma unroll
-        for (int k = 0; k < 9; ++k) a[k] = D.a[k * nr + i];
-        w0[0] = W[0][0];
-        w0[1] = W[0][1];
-        w0[2] = W[0][2];
-    } else {
-        load_q(D, nr, i, Q);
-    }
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const double t = __shfl_xor_sync(mask, w0[d], 1);
-        if (role) w0[d] = t;
-    }
-    if (role == 0) corr_cw(D, nr, i, C, W, a, fc, tq, s0i, rs0i);
-    else corr_q(D, nr, i, Q, w0);
-}
-
 constexpr int kTailAcc = 512;  // energy sums staged in shared memory by the corrector's tail
 
 // The corrector's tail, in the block that finished last, as two independent parts on two warps:
@@ -654,82 +659,175 @@ __device__ void corr_thermo(const View& v, const Dyn& D) {
     if (reb) th[TH_REBUILDS] = nreb + 1.0;
 }
 
-// Blocks of one-warp correctors carry a second warp for the tail (as the predictor's).
-template <int NT>
-struct CorrBlock {
-    static constexpr int kThreads = NT == 32 ? 64 : NT;
-};
+// The block that finished last adds uconf/press and corrects the thermostat.
+__device__ __forceinline__ void corr_end(const View& v, const Dyn& D, int slab, double* sh) {
+    if (!last_block(&D.done[1])) return;
+    if (threadIdx.x < 32) {
+        if (threadIdx.x == 0) D.done[1] = 0u;
+        corr_energy(v, D, slab, sh);
+    } else if (threadIdx.x == 32) {
+        corr_thermo(v, D);
+    }
+}
 
-// The correctors read the thermostat values of the predictor; the block that finishes last then
-// adds uconf/press and corrects the thermostat.  MERGE: the mixed force form's final merge and
+// The correctors read the thermostat values of the predictor.  MERGE: the mixed force form's final merge and
 // force_sum (merge.cuh) run here, each unit's just before its corrector, instead of in a kernel
 // of their own; units past the molecules and ions are the surface atoms, whose forces SHAKE's
 // Verlet step reads next.
-template <int NT, bool MERGE, bool PAIR>
-__global__ void __launch_bounds__(CorrBlock<NT>::kThreads) k_corr(View v, Dyn D, int slab, int lanes, MergeArgs A) {
-    constexpr bool kTailWarp = CorrBlock<NT>::kThreads > NT;
+template <int NT, bool MERGE>
+__global__ void __launch_bounds__(NT) k_corr(View v, Dyn D, int slab, MergeArgs A) {
     const int nsurf = MERGE ? v.nmove - v.nliqa : 0;
     const int nu = D.nion + v.nrig + nsurf;
     MergeArgs M;
     if constexpr (MERGE) M = merge_begin(v, A);
     double sx = 0.0, sy = 0.0, sz = 0.0;
-    for (int r = 0; !kTailWarp || threadIdx.x < NT; ++r) {
-        int u, role = 0;
-        if constexpr (PAIR) u = unit_of_pair<NT>(lanes, r, gridDim.x, role);
-        else u = unit_of<NT>(lanes, r, gridDim.x);
-        const bool act = u >= 0 && u < nu;
-        const bool rigid = act && u >= D.nion && u < D.nion + v.nrig;
-        unsigned mask = 0u;
-        if constexpr (PAIR) {
-            if (!__any_sync(0xffffffffu, act)) break;
-            mask = __ballot_sync(0xffffffffu, rigid);
-            if (!act) continue;
-        } else {
-            if (!act) break;
-        }
-        if (rigid) {
+    for (int r = 0;; ++r) {
+        const int u = unit_of<NT>(r, gridDim.x);
+        if (u >= nu) break;
+        if (u < D.nion) {
+            if constexpr (MERGE) merge_flex(v, M, u, sx, sy, sz);
+            corr_ion(v, D, u);
+        } else if (u < D.nion + v.nrig) {
             const int i = u - D.nion;
-            if constexpr (PAIR) {
-                double fc[3] = {0, 0, 0}, tq[3] = {0, 0, 0};
-                if constexpr (MERGE) {
-                    merge_rigid_pair(v, M, i, role, mask, sx, sy, sz, fc, tq);
-                } else if (role == 0) {
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        fc[d] = D.fc[d * v.nrig + i];
-                        tq[d] = D.tq[d * v.nrig + i];
-                    }
-                }
-                corr_rigid_pair(v, D, i, role, mask, fc, tq);
-            } else {
-                if constexpr (MERGE) merge_rigid(v, M, i, sx, sy, sz);
-                corr_rigid(v, D, i);
-            }
-        } else if (role == 0) {
-            if (u < D.nion) {
-                if constexpr (MERGE) merge_flex(v, M, u, sx, sy, sz);
-                corr_ion(v, D, u);
-            } else if constexpr (MERGE) {
-                merge_flex(v, M, u - v.nrig, sx, sy, sz);  // surface atom: flexible index nion + s
-            }
+            if constexpr (MERGE) merge_rigid(v, M, i, sx, sy, sz);
+            corr_rigid(v, D, i);
+        } else if constexpr (MERGE) {
+            merge_flex(v, M, u - v.nrig, sx, sy, sz);  // surface atom: flexible index nion + s
         }
     }
     if constexpr (MERGE) {
-        if (!kTailWarp || threadIdx.x < NT) {
-            block_atomic_sum<NT>(sx, &v.acc[2 * v.nijt + ACC_FWS0 + 0]);
-            block_atomic_sum<NT>(sy, &v.acc[2 * v.nijt + ACC_FWS0 + 1]);
-            block_atomic_sum<NT>(sz, &v.acc[2 * v.nijt + ACC_FWS0 + 2]);
+        block_atomic_sum<NT>(sx, &v.acc[2 * v.nijt + ACC_FWS0 + 0]);
+        block_atomic_sum<NT>(sy, &v.acc[2 * v.nijt + ACC_FWS0 + 1]);
+        block_atomic_sum<NT>(sz, &v.acc[2 * v.nijt + ACC_FWS0 + 2]);
+    }
+    __shared__ double sh_acc[kTailAcc];
+    corr_end(v, D, slab, sh_acc);
+}
+
+// The same for small systems: blocks below nrb 16 molecules each, the others ions and surface atoms.
+template <bool MERGE>
+__global__ void __launch_bounds__(kST) k_corr_small(View v, Dyn D, int slab, MergeArgs A, int nrb) {
+    __shared__ double s_w[3][kMol], s_q[4][kMol], s_f[3][3][kMol], s_t[3][3][kMol];
+    const int t = threadIdx.x;
+    MergeArgs M;
+    if constexpr (MERGE) M = merge_begin(v, A);
+    if (blockIdx.x < nrb) {
+        const int m = t & (kMol - 1), k = t / kMol, nr = v.nrig;
+        const bool act = blockIdx.x * kMol + m < nr;
+        const int i = act ? blockIdx.x * kMol + m : 0;
+        const mdg_rigid& body = D.body;
+        int st;
+        double* b = component(D, nr, i, k, st);
+        double a0 = b[0], a1 = b[st], a2 = b[2 * st], a3 = b[3 * (size_t)st], a4 = b[4 * (size_t)st];
+        const double s0i = D.th[TH_S], rs0i = D.th[TH_RS];
+        double rot[3] = {0, 0, 0};
+        if (k >= 3 && k < 6)
+#pragma unroll
+            for (int e = 0; e < 3; ++e) rot[e] = D.a[(size_t)(3 * (k - 3) + e) * nr + i];
+        if (k >= 3 && k < 6) s_w[k - 3][m] = a0;
+        if (k >= 6) s_q[k - 6][m] = a0;
+        if constexpr (MERGE) {
+            if (act && k < 3) {  // site k
+                const int j = 3 * i + k;
+                double fx, fy, fz;
+                merged_force(v, M, j, fx, fy, fz);
+                const double rx = v.x[j] - v.cx[i], ry = v.y[j] - v.cy[i], rz = v.z[j] - v.cz[i];
+                s_f[k][0][m] = fx;
+                s_f[k][1][m] = fy;
+                s_f[k][2][m] = fz;
+                s_t[k][0][m] = ry * fz - rz * fy;
+                s_t[k][1][m] = rz * fx - rx * fz;
+                s_t[k][2][m] = rx * fy - ry * fx;
+                if (i == nr - 1) {
+                    v.rsx[k] = rx;
+                    v.rsy[k] = ry;
+                    v.rsz[k] = rz;
+                }
+            }
+        }
+        __syncthreads();
+        double fsum = 0.0;
+        if (act && k < 3) {
+            double fc;
+            if constexpr (MERGE) {
+                fc = s_f[0][k][m] + s_f[1][k][m] + s_f[2][k][m];
+                fsum = fc;
+                M.fc[(size_t)k * nr + i] = fc;
+            } else {
+                fc = D.fc[(size_t)k * nr + i];
+            }
+            const double co = (0.5 / body.mw) * fc - a1 * s0i - a2;
+            a0 = a0 + Gf02 * co;
+            a1 = a1 + Gf12 * co;
+            a2 = a2 + Gf22 * co;
+            a3 = a3 + Gf32 * co;
+            a4 = a4 + Gf42 * co;
+        } else if (act) {
+            const double wx = s_w[0][m], wy = s_w[1][m], wz = s_w[2][m];
+            double co;
+            if (k < 6) {
+                double tq[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    if constexpr (MERGE) tq[d] = s_t[0][d][m] + s_t[1][d][m] + s_t[2][d][m];
+                    else tq[d] = D.tq[(size_t)d * nr + i];
+                }
+                if constexpr (MERGE) M.tq[(size_t)(k - 3) * nr + i] = k == 3 ? tq[0] : k == 4 ? tq[1] : tq[2];
+                const double dI = k == 3 ? body.inyy - body.inzz : k == 4 ? body.inzz - body.inxx : body.inxx - body.inyy;
+                const double ww = k == 3 ? wy * wz : k == 4 ? wz * wx : wx * wy;
+                const double inv = 1.0 / (k == 3 ? body.inxx : k == 4 ? body.inyy : body.inzz);
+                const double c = rot[0] * tq[0] + rot[1] * tq[1] + rot[2] * tq[2];
+                co = (c + ww * dI) * inv - a1 - rs0i * a0;
+            } else {
+                const double q1 = s_q[0][m], q2 = s_q[1][m], q3 = s_q[2][m], q4 = s_q[3][m];
+                double cq;
+                if (k == 6) cq = 0.5 * (-q3 * wx - q4 * wy + q2 * wz);
+                else if (k == 7) cq = 0.5 * (q4 * wx - q3 * wy - q1 * wz);
+                else if (k == 8) cq = 0.5 * (q1 * wx + q2 * wy + q4 * wz);
+                else cq = 0.5 * (-q2 * wx + q1 * wy - q3 * wz);
+                co = cq - a1;
+            }
+            a0 = a0 + Gf01 * co;
+            a1 = a1 + Gf11 * co;
+            a2 = a2 + Gf21 * co;
+            a3 = a3 + Gf31 * co;
+            a4 = a4 + Gf41 * co;
+        }
+        if (act) {
+            b[0] = a0;
+            b[st] = a1;
+            b[2 * st] = a2;
+            b[3 * (size_t)st] = a3;
+            b[4 * (size_t)st] = a4;
+        }
+        if constexpr (MERGE) {
+            if (t < 2 * 32) {
+                fsum = sum16(fsum);
+                if (m == 0 && k < 3) atomicAdd(&v.acc[2 * v.nijt + ACC_FWS0 + k], fsum);
+            }
+        }
+    } else {
+        const int nflex = D.nion + (MERGE ? v.nmove - v.nliqa : 0), u = (blockIdx.x - nrb) * kFlex + t;
+        if (t < kFlex) {
+            double sx = 0.0, sy = 0.0, sz = 0.0;
+            if constexpr (MERGE) {
+                if (u < nflex) merge_flex(v, M, u, sx, sy, sz);
+            }
+            if (u < D.nion) corr_ion(v, D, u);
+            if constexpr (MERGE) {
+                sx = warp_sum(sx);
+                sy = warp_sum(sy);
+                sz = warp_sum(sz);
+                if (t == 0) {
+                    atomicAdd(&v.acc[2 * v.nijt + ACC_FWS0 + 0], sx);
+                    atomicAdd(&v.acc[2 * v.nijt + ACC_FWS0 + 1], sy);
+                    atomicAdd(&v.acc[2 * v.nijt + ACC_FWS0 + 2], sz);
+                }
+            }
         }
     }
     __shared__ double sh_acc[kTailAcc];
-    if (last_block(&D.done[1])) {
-        if (threadIdx.x < 32) {
-            if (threadIdx.x == 0) D.done[1] = 0u;
-            corr_energy(v, D, slab, sh_acc);
-        } else if (threadIdx.x == 32) {
-            corr_thermo(v, D);
-        }
-    }
+    corr_end(v, D, slab, sh_acc);
 }
 
 Dyn dyn_of(Ctx& c) {
@@ -750,20 +848,19 @@ Dyn dyn_of(Ctx& c) {
     return D;
 }
 
-// molecules per warp, and the block size: one warp per block while a warp per SM covers the
-// system, else full warps in blocks of four
-int lanes_of(int n) { return std::max(1, std::min(32, (n + kSM - 1) / kSM)); }
-int nblk(int n, int nt) {
-    const int lanes = lanes_of(n), warps = (n + lanes - 1) / lanes;
-    return std::max(1, std::min((warps + nt / 32 - 1) / (nt / 32), kSM * 8));
-}
+// Units up to which the forms for small systems are the faster ones: with more the FP64 pipe is the limit and
+// their half-filled warps cost (bulk water, k_pred and k_corr, one thread per molecule | component): 1,000
+// 17 and 17 | 8 and 11 us, 4,913 19 and 17 | 11 and 13, 8,000 19 and 18 | 12 and 15, 15,625 19 and 19 | 19
+// and 20, 32,768 28 and 25 | 37 and 33.
+bool small(int nu) { return nu <= 80 * kSM; }
+int nblk(int n) { return std::max(1, std::min((n + 127) / 128, kSM * 8)); }
 
 }  // namespace
 
 void predict_launch(Ctx& c, bool clear_acc, bool clear_kps, bool pack) {
     const View& v = c.v;
     Dyn D = dyn_of(c);
-    const int nu = D.nion + v.nrig, lanes = lanes_of(nu);
+    const int nu = D.nion + v.nrig;
     Clear z{{v.acc, c.d_kps}, {clear_acc ? 2 * v.nijt + ACC_NSLOT : 0, clear_kps && c.d_kps ? v.nit : 0}};
     PackArgs P{};
     if (pack) {
@@ -771,25 +868,19 @@ void predict_launch(Ctx& c, bool clear_acc, bool clear_kps, bool pack) {
         P.dip = c.variant == MDG_SLAB ? 1 : 0;
     }
     const int nwall = v.ntota - v.nmove;
-    if (lanes < 32) {
-        const int nb = nblk(nu, 32);
-        P.npred = nb;
-        const int nwb = pack ? std::min((nwall + 31) / 32, kSM * 8) : 0;
+    if (small(nu)) {
+        const int nrb = (v.nrig + kMol - 1) / kMol, nfb = (D.nion + kFlex - 1) / kFlex;
+        const int nb = std::max(1, nrb + nfb), nwb = pack ? std::min((nwall + kST - 1) / kST, kSM * 8) : 0;
         c.pred_parts = nb + nwb;
-        if (lanes <= 16) {  // two lanes per molecule
-            if (pack) k_pred<32, true, true><<<nb + nwb, 32, 0, c.stream>>>(v, D, lanes, z, P);
-            else k_pred<32, false, true><<<nb, 32, 0, c.stream>>>(v, D, lanes, z, P);
-        } else {
-            if (pack) k_pred<32, true, false><<<nb + nwb, 32, 0, c.stream>>>(v, D, lanes, z, P);
-            else k_pred<32, false, false><<<nb, 32, 0, c.stream>>>(v, D, lanes, z, P);
-        }
+        if (pack) k_pred_small<true><<<nb + nwb, kST, 0, c.stream>>>(v, D, z, P, nrb, nb - nrb);
+        else k_pred_small<false><<<nb, kST, 0, c.stream>>>(v, D, z, P, nrb, nb - nrb);
     } else {
-        const int nb = nblk(nu, 128);
+        const int nb = nblk(nu);
         P.npred = nb;
         const int nwb = pack ? std::min((nwall + 127) / 128, kSM * 8) : 0;
         c.pred_parts = nb + nwb;
-        if (pack) k_pred<128, true, false><<<nb + nwb, 128, 0, c.stream>>>(v, D, lanes, z, P);
-        else k_pred<128, false, false><<<nb, 128, 0, c.stream>>>(v, D, lanes, z, P);
+        if (pack) k_pred<128, true><<<nb + nwb, 128, 0, c.stream>>>(v, D, z, P);
+        else k_pred<128, false><<<nb, 128, 0, c.stream>>>(v, D, z, P);
     }
 }
 
@@ -800,19 +891,16 @@ void step_close_launch(Ctx& c) {
 void correct_launch(Ctx& c, bool merge) {
     const View& v = c.v;
     Dyn D = dyn_of(c);
-    const int nu = D.nion + v.nrig + (merge ? v.nmove - v.nliqa : 0), lanes = lanes_of(nu);
+    const int nu = D.nion + v.nrig + (merge ? v.nmove - v.nliqa : 0);
     const int slab = c.variant == MDG_SLAB ? 1 : 0;
     const MergeArgs A = merge ? merge_args(c, c.d_frc) : MergeArgs{};
-    constexpr int kCT = CorrBlock<32>::kThreads;
-    if (lanes <= 16) {
-        if (merge) k_corr<32, true, true><<<nblk(nu, 32), kCT, 0, c.stream>>>(v, D, slab, lanes, A);
-        else k_corr<32, false, true><<<nblk(nu, 32), kCT, 0, c.stream>>>(v, D, slab, lanes, A);
-    } else if (lanes < 32) {
-        if (merge) k_corr<32, true, false><<<nblk(nu, 32), kCT, 0, c.stream>>>(v, D, slab, lanes, A);
-        else k_corr<32, false, false><<<nblk(nu, 32), kCT, 0, c.stream>>>(v, D, slab, lanes, A);
+    if (small(nu)) {
+        const int nrb = (v.nrig + kMol - 1) / kMol, nb = std::max(1, nrb + (nu - v.nrig + kFlex - 1) / kFlex);
+        if (merge) k_corr_small<true><<<nb, kST, 0, c.stream>>>(v, D, slab, A, nrb);
+        else k_corr_small<false><<<nb, kST, 0, c.stream>>>(v, D, slab, A, nrb);
     } else {
-        if (merge) k_corr<128, true, false><<<nblk(nu, 128), 128, 0, c.stream>>>(v, D, slab, lanes, A);
-        else k_corr<128, false, false><<<nblk(nu, 128), 128, 0, c.stream>>>(v, D, slab, lanes, A);
+        if (merge) k_corr<128, true><<<nblk(nu), 128, 0, c.stream>>>(v, D, slab, A);
+        else k_corr<128, false><<<nblk(nu), 128, 0, c.stream>>>(v, D, slab, A);
     }
 }
 
