@@ -100,4 +100,15 @@ inline cudaError_t allow_max_smem(F* f) {
     return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, mx - (int)fa.sharedSizeBytes);
 }
 
+// the system of block b: the largest r with first[r] <= b (first[0] = 0 <= b < first[nrep])
+__device__ __forceinline__ int rep_of_block(const int* __restrict__ first, int nrep, int b) {
+    int lo = 0, hi = nrep - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (first[mid] <= b) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
 }  // namespace mdg

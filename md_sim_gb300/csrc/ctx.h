@@ -339,6 +339,21 @@ struct LsBatch {
 int ls_batch_setup(LsBatch& lb, const std::vector<Ctx*>& cs, std::string& err);
 void ls_batch_launch(const LsBatch& lb, cudaStream_t st);
 void ls_batch_free(LsBatch& lb);
+// integrate.cu: predictor, close of the packing, wall tail and corrector of several systems
+struct IntBatch {
+    void* d_buf = nullptr;                           // descriptors, then first blocks
+    size_t cap = 0;
+    int* first[3] = {nullptr, nullptr, nullptr};     // predictor, corrector, wall tail
+    int nblk[3] = {0, 0, 0};
+    int nrep = 0;
+};
+bool int_batchable(const Ctx& c);
+int int_batch_setup(IntBatch& ib, const std::vector<Ctx*>& cs, std::string& err);
+void int_batch_pred(const IntBatch& ib, cudaStream_t st);
+void int_batch_close(const IntBatch& ib, cudaStream_t st);
+void int_batch_lr(const IntBatch& ib, cudaStream_t st);
+void int_batch_correct(const IntBatch& ib, cudaStream_t st);
+void int_batch_free(IntBatch& ib);
 // pair.cu
 int pair_setup(Ctx& c);
 void pair_forces_fp64(Ctx& c);

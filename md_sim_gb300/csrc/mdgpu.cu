@@ -1451,21 +1451,23 @@ int mdg_mlp_train(const float* x, const float* y, int64_t n, int epochs, int bat
 // Replica batches: independent contexts stepped by one graph launch.  Two graph forms:
 //   MDG_BATCH_GRAPHS  every replica's step graph is a parallel child graph of one graph, so the
 //                     kernels of small systems fill the GPU together;
-//   MDG_BATCH_PHASES  phase order: every replica's predictor, packing close (rebuild decision),
-//                     wall tail and reciprocal branch as in its own step, then, for the replicas
-//                     in the concurrent mixed form (walls, no surface atoms), the list build as
-//                     five launches in all and the head-head and head-wall loops as one persistent
-//                     kernel each over all their heads, then every replica's merge, corrector and
-//                     SHAKE.  Other replicas keep their whole step in the graph.
+//   MDG_BATCH_PHASES  phase order for the replicas in the concurrent mixed form (walls, no surface
+//                     atoms): predictor, packing close (rebuild decision) and wall tail in one
+//                     launch each for all of them, every replica's reciprocal branch, the list build
+//                     as four launches in all, the head-head and head-wall loops as one persistent
+//                     kernel each over all heads, then merge and corrector in one launch (large
+//                     replicas, and those whose site forces are needed apart, have launches of their
+//                     own instead).  Other replicas keep their whole step in the graph.
 // ---------------------------------------------------------------------------------------------
 struct mdg_batch {
     std::vector<mdg_ctx*> ctx;
     cudaStream_t stream = nullptr;      // stream the batch graph is launched on
     cudaStream_t own_stream = nullptr;  // the batch's own stream (the only one it destroys)
     cudaStream_t cs = nullptr, cs2 = nullptr;  // capture streams of the phase-ordered graph
-    std::vector<cudaEvent_t> ev;        // its fork and join events: 4 + 2 per replica
+    std::vector<cudaEvent_t> ev;        // its fork and join events: 4 + 2 per replica + 2
     RsBatch rb;                         // descriptors of the batched real-space loops
-    LsBatch lb;                         // and of the batched list build
+    LsBatch lb;                         // of the batched list build
+    IntBatch ib;                        // and of the batched predictor, close, wall tail and corrector
     int mode = MDG_BATCH_PHASES;
     int phased = 0;                     // replicas in the batched loops (last graph build)
     cudaGraphExec_t exec = nullptr;
@@ -1489,25 +1491,30 @@ static int batch_graph_phases(mdg_batch* b) {
             cudaStreamCreateWithPriority(&b->cs2, cudaStreamNonBlocking, prio_hi) != cudaSuccess)
             return batch_err(b, MDG_E_CUDA, "batch: capture streams");
     }
-    while (b->ev.size() < 4 + 2 * n) {
+    while (b->ev.size() < 6 + 2 * n) {
         cudaEvent_t e;
         if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
             return batch_err(b, MDG_E_CUDA, "batch: events");
         b->ev.push_back(e);
     }
-    std::vector<Ctx*> ph;
-    std::vector<char> is_ph(n, 0);
+    std::vector<Ctx*> ph, in;
+    std::vector<char> is_ph(n, 0), is_in(n, 0);
     for (size_t i = 0; i < n; ++i)
         if (batch_phased(*b->ctx[i])) {
             ph.push_back(b->ctx[i]);
             is_ph[i] = 1;
+            if (merge_fusable(*b->ctx[i]) && int_batchable(*b->ctx[i])) {
+                in.push_back(b->ctx[i]);
+                is_in[i] = 1;
+            }
         }
     std::string err;
     int rc = rs_batch_setup(b->rb, ph, err);
     if (!rc) rc = ls_batch_setup(b->lb, ph, err);
+    if (!rc) rc = int_batch_setup(b->ib, in, err);
     if (rc) return batch_err(b, rc, err);
     b->phased = (int)ph.size();
-    cudaEvent_t ev0 = b->ev[0], evf = b->ev[1], evw = b->ev[2], evrs = b->ev[3];
+    cudaEvent_t ev0 = b->ev[0], evf = b->ev[1], evw = b->ev[2], evrs = b->ev[3], evp = b->ev[4 + 2 * n], evc = b->ev[5 + 2 * n];
     auto ev_pre = [&](size_t i) { return b->ev[4 + 2 * i]; };
     auto ev_post = [&](size_t i) { return b->ev[5 + 2 * i]; };
     if (cudaStreamBeginCapture(b->cs, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
@@ -1521,7 +1528,25 @@ static int batch_graph_phases(mdg_batch* b) {
         return batch_err(b, code, m);
     };
     bool ok = cudaEventRecord(ev0, b->cs) == cudaSuccess;
+    if (ok && !in.empty()) {
+        // the replicas with batched integrator kernels: predictor, then each one's reciprocal branch and the
+        // wall tail beside the close of the packing
+        int_batch_pred(b->ib, b->cs);
+        ok = cudaEventRecord(evp, b->cs) == cudaSuccess && cudaStreamWaitEvent(b->cs2, evp, 0) == cudaSuccess;
+        for (Ctx* c : in) {
+            if (!ok) break;
+            ok = cudaStreamWaitEvent(c->side, evp, 0) == cudaSuccess;
+            const cudaStream_t s0 = c->stream;
+            c->stream = c->side;
+            recip_tc(*c);
+            c->stream = s0;
+            ok = ok && cudaEventRecord(c->ev_join, c->side) == cudaSuccess;
+        }
+        int_batch_lr(b->ib, b->cs2);
+        int_batch_close(b->ib, b->cs);
+    }
     for (size_t i = 0; i < n && ok; ++i) {
+        if (is_in[i]) continue;
         Ctx& c = *b->ctx[i];
         ok = cudaStreamWaitEvent(c.stream, ev0, 0) == cudaSuccess;
         c.batch_stage = is_ph[i] ? 1 : 0;
@@ -1532,15 +1557,27 @@ static int batch_graph_phases(mdg_batch* b) {
     }
     if (ok && !ph.empty()) {
         for (size_t i = 0; i < n && ok; ++i)
-            if (is_ph[i]) ok = cudaStreamWaitEvent(b->cs, ev_pre(i), 0) == cudaSuccess;
+            if (is_ph[i] && !is_in[i]) ok = cudaStreamWaitEvent(b->cs, ev_pre(i), 0) == cudaSuccess;
         if (ok) ls_batch_launch(b->lb, b->cs);
         ok = ok && cudaEventRecord(evf, b->cs) == cudaSuccess && cudaStreamWaitEvent(b->cs2, evf, 0) == cudaSuccess;
         if (ok) rs_batch_launch(b->rb, b->cs, b->cs2);
         ok = ok && cudaEventRecord(evw, b->cs2) == cudaSuccess && cudaStreamWaitEvent(b->cs, evw, 0) == cudaSuccess &&
              cudaEventRecord(evrs, b->cs) == cudaSuccess;
+        if (ok && !in.empty()) {
+            for (Ctx* c : in) ok = ok && cudaStreamWaitEvent(b->cs, c->ev_join, 0) == cudaSuccess;
+            if (ok) int_batch_correct(b->ib, b->cs);
+            ok = ok && cudaEventRecord(evc, b->cs) == cudaSuccess;
+        }
         for (size_t i = 0; i < n && ok; ++i) {
             if (!is_ph[i]) continue;
             Ctx& c = *b->ctx[i];
+            if (is_in[i]) {
+                if (!(c.meas.init && c.meas.profiles)) continue;
+                ok = cudaStreamWaitEvent(c.stream, evc, 0) == cudaSuccess;
+                measure_do_launch(c, c.v.x, c.v.y, c.v.z);
+                ok = ok && cudaEventRecord(ev_post(i), c.stream) == cudaSuccess;
+                continue;
+            }
             ok = cudaStreamWaitEvent(c.stream, evrs, 0) == cudaSuccess;
             c.batch_stage = 2;
             rc = step_launch(c);
@@ -1549,8 +1586,11 @@ static int batch_graph_phases(mdg_batch* b) {
             ok = ok && cudaEventRecord(ev_post(i), c.stream) == cudaSuccess;
         }
     }
-    for (size_t i = 0; i < n && ok; ++i)
+    for (size_t i = 0; i < n && ok; ++i) {
+        const Ctx& c = *b->ctx[i];
+        if (is_in[i] && !(c.meas.init && c.meas.profiles)) continue;  // its last kernel is on cs
         ok = cudaStreamWaitEvent(b->cs, is_ph[i] ? ev_post(i) : ev_pre(i), 0) == cudaSuccess;
+    }
     if (!ok) return fail(MDG_E_CUDA, std::string("batch capture: ") + cudaGetErrorString(cudaGetLastError()));
     cudaGraph_t g = nullptr;
     const cudaError_t ce = cudaStreamEndCapture(b->cs, &g);
@@ -1636,6 +1676,7 @@ void mdg_batch_destroy(mdg_batch* b) {
     for (cudaEvent_t e : b->ev) cudaEventDestroy(e);
     rs_batch_free(b->rb);
     ls_batch_free(b->lb);
+    int_batch_free(b->ib);
     delete b;
 }
 

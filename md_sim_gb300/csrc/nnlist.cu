@@ -344,17 +344,6 @@ struct alignas(16) LsRep {
     float4 *cpos, *wpos;
 };
 
-// the system of block b: the largest r with first[r] <= b (first[0] = 0 <= b < first[nrep])
-__device__ __forceinline__ int rep_of_block(const int* __restrict__ first, int nrep, int b) {
-    int lo = 0, hi = nrep - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (first[mid] <= b) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
 __global__ void __launch_bounds__(kNT) k_bin_heads_b(const LsRep* __restrict__ reps, const int* __restrict__ first,
                                                      int nrep) {
     const int r = rep_of_block(first, nrep, blockIdx.x);

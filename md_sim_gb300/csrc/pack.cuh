@@ -63,9 +63,10 @@ __device__ __forceinline__ double pack_atom(const View& v, const Pk& pk, int a, 
     return mz;
 }
 
-// Every thread of the block: its dipole share to pk.part[blockIdx.x], its maximum displacement
+// Every thread of the block: its dipole share to pk.part[bid], its maximum displacement
 // into the accumulator slot (atomic max).  red: 8 doubles of shared memory.
-__device__ __forceinline__ void pack_block(const View& v, const Pk& pk, double mz, double md, double* red) {
+__device__ __forceinline__ void pack_block(const View& v, const Pk& pk, double mz, double md, double* red,
+                                           int bid) {
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
     mz = warp_sum(mz);
     for (int o = 16; o > 0; o >>= 1) md = fmax(md, __shfl_xor_sync(0xffffffffu, md, o));
@@ -77,7 +78,7 @@ __device__ __forceinline__ void pack_block(const View& v, const Pk& pk, double m
     if (threadIdx.x == 0) {
         double b = 0.0;
         for (int k = 0; k < nw; ++k) b += red[k];
-        pk.part[blockIdx.x] = b;
+        pk.part[bid] = b;
     }
     __syncthreads();
 }

@@ -185,7 +185,7 @@ __global__ void k_pack(View v, Pk pk, int dip, int force, int reset_status, int 
         mz += pack_atom(v, pk, a, v.x[a], v.y[a], v.z[a], mv ? v.rsx[a] : 0.0, mv ? v.rsy[a] : 0.0,
                         mv ? v.rsz[a] : 0.0, mv);
     }
-    pack_block(v, pk, mz, md, red);
+    pack_block(v, pk, mz, md, red, blockIdx.x);
     if (defer_close) return;
     __threadfence();
     if (threadIdx.x == 0) last = atomicAdd(&v.status[ST_PACK_DONE], 1) == (int)gridDim.x - 1;
