@@ -79,21 +79,46 @@ __device__ __forceinline__ void e_flush(EAcc& e, double* s_e, int nijt) {
     e.qq = Kahan();
 }
 
-// All lanes of a warp: lanes holding the warp's (largest) pair type reduce with shuffles in FP64 (a
-// warp's total grows with the heads it took, and an FP32 reduction of it would round at that
-// size), one shared atomic per warp; lanes left with another type flush one by one.  Leaves e empty.
-__device__ __forceinline__ void e_final(EAcc& e, double* s_e, int nijt) {
-    const int ij0 = __reduce_max_sync(0xffffffffu, e.ijt);
-    if (ij0 < 0) return;
-    const bool mine = e.ijt == ij0;
-    const double lj = warp_sum(mine ? e.lj.value() : 0.0);
-    const double qq = warp_sum(mine ? e.qq.value() : 0.0);
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&s_e[ij0], lj);
-        atomicAdd(&s_e[nijt + ij0], qq);
+// Sums of N values over the warp (FP64): lane 32 / N k gets that of v[k].  Each step halves the values a lane still carries, so that a sum takes 9 FP64 additions for 8 values
+// where one butterfly after the other takes 40: at the end of a block all its warps queue for the FP64 pipe.
+template <int N>
+__device__ __forceinline__ double warp_sums(double (&v)[N]) {
+    const int lane = threadIdx.x & 31;
+    int o = 16;
+#pragma unroll
+    for (int n = N / 2; n > 0; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int k = 0; k < n; ++k) {
+            const double keep = up ? v[k + n] : v[k], send = up ? v[k] : v[k + n];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
     }
-    if (!mine) e_flush(e, s_e, nijt);
-    e = EAcc();
+    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+
+// All lanes of a warp: lanes holding the warp's (largest) pair type of an accumulator reduce with shuffles in
+// FP64 (a warp's total grows with the heads it took, and an FP32 reduction of it would round at that
+// size), one shared atomic per sum; lanes left with another type flush one by one.  Leaves e empty.
+__device__ __forceinline__ void e_final(EAcc (&e)[2], double* s_e, int nijt) {
+    const int ij[2] = {__reduce_max_sync(0xffffffffu, e[0].ijt), __reduce_max_sync(0xffffffffu, e[1].ijt)};
+    if (ij[0] < 0 && ij[1] < 0) return;
+    double v[4];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        const bool mine = e[k].ijt >= 0 && e[k].ijt == ij[k];
+        v[2 * k] = mine ? e[k].lj.value() : 0.0;
+        v[2 * k + 1] = mine ? e[k].qq.value() : 0.0;
+    }
+    const double sum = warp_sums(v);
+    const int lane = threadIdx.x & 31, k = lane >> 3, t = k > 1 ? ij[1] : ij[0];
+    if ((lane & 7) == 0 && t >= 0) atomicAdd(&s_e[(k & 1) * nijt + t], sum);
+#pragma unroll
+    for (int a = 0; a < 2; ++a) {
+        if (e[a].ijt != ij[a]) e_flush(e[a], s_e, nijt);
+        e[a] = EAcc();
+    }
 }
 
 __device__ __forceinline__ void e_add(EAcc& e, int ijt, float lj, float qq, double* s_e, int nijt) {
@@ -326,7 +351,7 @@ struct Queue {
 // The head-head loop of one warp over the heads h0, h0 + hs, ... below v.nheads; e: energies with
 // partners of the first site type and of the others.
 template <int ZPER>
-__device__ __forceinline__ void pair_heads(const View& v, const Pk& pk, const Tables& T, int h0, int hs, EAcc e[2],
+__device__ __forceinline__ void pair_heads(const View& v, const Pk& pk, const Tables& T, int h0, int hs, EAcc (&e)[2],
                                            double* s_e, QueueMem* queue) {
     const int lane = threadIdx.x & 31;
     const float alfa = pk.alfa, spii = pk.spii, facq = pk.facq, rcutsq = pk.rcutsq;
@@ -349,8 +374,7 @@ __device__ __forceinline__ void pair_heads(const View& v, const Pk& pk, const Ta
         const int it = (int)(pi.w & 0x7fffffffu);
         const int nsi_i = T.nsi[it];
         if (it != it_last && it_last >= 0) {
-            e_final(e[0], s_e, v.nijt);
-            e_final(e[1], s_e, v.nijt);
+            e_final(e, s_e, v.nijt);
         }
         it_last = it;
         const float zli = ZPER ? 0.f : pk.zlo[i];
@@ -450,9 +474,8 @@ __device__ __forceinline__ void pair_heads(const View& v, const Pk& pk, const Ta
 
 // The block's energy sums into the system's accumulators (all threads; the shared sums are free
 // for the next system's tables afterwards).
-__device__ __forceinline__ void pair_flush(const View& v, EAcc e[2], double* s_e) {
-    e_final(e[0], s_e, v.nijt);
-    e_final(e[1], s_e, v.nijt);
+__device__ __forceinline__ void pair_flush(const View& v, EAcc (&e)[2], double* s_e) {
+    e_final(e, s_e, v.nijt);
     __syncthreads();
     for (int k = threadIdx.x; k < 2 * v.nijt; k += blockDim.x)
         if (s_e[k] != 0.0) atomicAdd(&v.acc[k], s_e[k]);
@@ -515,8 +538,7 @@ __device__ __forceinline__ void wall_heads(const View& v, const Pk& pk, const Ta
         const int it = (int)(pi.w & 0x7fffffffu);
         const int nsi_i = T.nsi[it];
         if (it != it_last && it_last >= 0) {
-            e_final(w.ew[0], w.s_e, v.nijt);
-            e_final(w.ew[1], w.s_e, v.nijt);
+            e_final(w.ew, w.s_e, v.nijt);
         }
         it_last = it;
         const bool book = (it + 1) <= v.nltype;
@@ -602,14 +624,13 @@ __device__ __forceinline__ void wall_heads(const View& v, const Pk& pk, const Ta
 // The block's energy and wall reaction sums into the system's accumulators (all threads).
 __device__ __forceinline__ void wall_flush(const View& v, WAcc& w) {
     double* s_e = w.s_e;
-    e_final(w.ew[0], s_e, v.nijt);
-    e_final(w.ew[1], s_e, v.nijt);
+    e_final(w.ew, s_e, v.nijt);
+    double ws[8] = {w.ws[0], w.ws[1], w.ws[2], w.ws[3], w.ws[4], w.ws[5], 0.0, 0.0};
+    const double s = warp_sums(ws);
+    const int lane = threadIdx.x & 31;
+    if ((lane & 3) == 0 && lane < 24 && s != 0.0) atomicAdd(&s_e[2 * v.nijt + (lane >> 2)], s);
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        const double s = warp_sum(w.ws[k]);
-        if ((threadIdx.x & 31) == 0 && s != 0.0) atomicAdd(&s_e[2 * v.nijt + k], s);
-        w.ws[k] = 0.0;
-    }
+    for (int k = 0; k < 6; ++k) w.ws[k] = 0.0;
     __syncthreads();
     for (int k = threadIdx.x; k < 2 * v.nijt; k += blockDim.x)
         if (s_e[k] != 0.0) atomicAdd(&v.acc[k], s_e[k]);
