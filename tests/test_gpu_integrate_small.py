@@ -56,3 +56,19 @@ def test_line(n_side, gpulib, oracle):
     b, rb = _run(oracle, s, prm, 2)
     a, ra = _run(gpulib, s, prm, 2)
     _close(a, ra, b, rb, 1e-9, 1e-9, True)
+
+
+@pytest.mark.parametrize("fn", [lambda: configs.bulk_water(7, "sc"), lambda: configs.slab_electrolyte()])
+def test_merge_blocks(fn, gpulib):
+    """Site forces, centre forces and torques of a mixed force call from the merge by sites, against the FP64
+    form: a last block of 23 molecules, and 24 ions beside full blocks.  Bar: the mixed forces' 1e-5 of the norm."""
+    s, prm = fn()
+    out = []
+    for p in (abi.MDG_FP64, abi.MDG_MIXED):
+        c = abi.Context(gpulib, s.copy(), abi.RunParams(**{**prm.__dict__, "precision": p}))
+        out.append(c.force_get(s.copy()))
+        c.close()
+    a, b = out
+    for key in ("f", "ft", "fc", "torque"):
+        if a[key].size:
+            assert np.linalg.norm(b[key] - a[key]) <= 1e-5 * np.linalg.norm(a[key]), key
