@@ -16,7 +16,7 @@ __device__ __forceinline__ void lr_tail_block(const View& v, const double* lr, i
     for (int i = bid * kLrNT + threadIdx.x; i < v.nmove; i += nblk * kLrNT) {
         const int it = v.type[i];
         if (fabs(v.q[i]) < F32D(0.7)) continue;
-        double fz = v.fz[i];
+        double fz = 0.0;
         for (int j = -1; j <= 1; j += 2) {
             double aux = 0.0;
             const double sgn = (double)j;
@@ -40,7 +40,7 @@ __device__ __forceinline__ void lr_tail_block(const View& v, const double* lr, i
             fz -= aux;
             if (it + 1 <= v.nltype) fw[(j + 1) / 2] += aux;
         }
-        v.fz[i] = fz;
+        atomicAdd(&v.fz[i], fz);  // the reciprocal sum of the FP64 form may be adding too
     }
     block_atomic_sum<kLrNT>(ulr, &v.acc[2 * v.nijt + ACC_ULR]);
     block_atomic_sum<kLrNT>(fw[0], &v.acc[2 * v.nijt + ACC_FWS + 6 + 0]);

@@ -249,15 +249,9 @@ __global__ void __launch_bounds__(kForceNT) k_kforce(View v, KDims d, int nrow, 
     fx *= d.px;
     fy *= d.py;
     fz *= d.pz;
-    if (gridDim.y > 1) {
-        atomicAdd(&v.fx[j], fx);
-        atomicAdd(&v.fy[j], fy);
-        atomicAdd(&v.fz[j], fz);
-    } else {
-        v.fx[j] += fx;
-        v.fy[j] += fy;
-        v.fz[j] += fz;
-    }
+    atomicAdd(&v.fx[j], fx);  // other grid rows add to it too, and the real-space loops may be running
+    atomicAdd(&v.fy[j], fy);
+    atomicAdd(&v.fz[j], fz);
 }
 
 // Widom insertion: P and M of every entry (two double2), from S and the walls' sums as they stand.

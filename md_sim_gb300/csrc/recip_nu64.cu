@@ -189,12 +189,13 @@ __global__ void __launch_bounds__(kNT) k_nu64_force(View v, NuViewT<double> g, c
     __shared__ double wts[kFA][3][kW], dwts[kFA][3][kW], charge[kFA];
     __shared__ int cell[kFA][4];
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5, nblk = g.nblk;
+    // (atomics: the real-space loops may be running)
     auto add = [&](int id, double q, double2 s) {
         if (lane == 0) {
-            v.fx[id] -= q * g.scale[0] * s.x;
-            v.fz[id] -= q * g.scale[2] * s.y;
+            atomicAdd(&v.fx[id], -q * g.scale[0] * s.x);
+            atomicAdd(&v.fz[id], -q * g.scale[2] * s.y);
         }
-        if (lane == 16) v.fy[id] -= q * g.scale[1] * s.x;
+        if (lane == 16) atomicAdd(&v.fy[id], -q * g.scale[1] * s.x);
     };
     const int z = lane & 15, h = lane >> 4;
     if (blockIdx.x == nblk) {
