@@ -208,13 +208,34 @@ def fp32_nominal_tflops():
     return 152 * 128 * 2 * mhz * 1e6 / 1e12
 
 
+def gridded(s, nk, precision):
+    """Whether the library takes the gridded reciprocal sum: atoms times k vectors from its lines on
+    (kGridWork in recip_tc.cu, kGridWork64 in recip_nu64.cu)."""
+    from md_sim_gb300.abi import MDG_MIXED
+
+    return s.nmove * nk >= (8.0e7 if precision == MDG_MIXED else 5.0e6)
+
+
+def grid_flops(s, prm, mixed):
+    """Operations of one gridded reciprocal sum: w^3 points per atom once for the charges and 2.4 times for the
+    forces (a window of w points per direction), and the folded separable Fourier sums, both ways."""
+    w = 8 if mixed else 16
+    lmin = min(s.lx, s.ly, s.lz)
+    K = [round(prm.kmax * x / lmin) for x in (s.lx, s.ly, s.lz)]
+    M = [max(16, 4 * k + 8) if mixed else max(24, (9 * k // 2 + 4 + 7) // 8 * 8) for k in K]
+    h, n = [m // 2 + 1 for m in M], K[2] + 1
+    fourier = 2 * M[0] * M[1] * n * h[2] + 4 * n * M[0] * (K[1] + 1) * h[1] + 4 * n * (2 * K[1] + 1) * (K[0] + 1) * h[0]
+    return 2.0 * (3.4 * w ** 3 * s.nmove + 2.0 * fourier)
+
+
 def roofline(ctx, s, prm, precision, pk, config_name="", fp64_peak=None):
     """Roofline of the dominant force phase (and of the reciprocal and pair phases), from CUDA-event
     phase times of mdg_phase_times and the algorithmic work per unit:
       pair phases   45 flops per accepted site pair (FP64 pipe, or FP32 + MUFU when mixed)
       reciprocal    18 flops per (atom, valid k) in FP64; 24 flops per (atom, valid k) for the
                     three complex products of the tensor-core form, whose ceiling is the dense
-                    16-bit tensor peak / 3 (hi*hi + hi*lo + lo*hi).
+                    16-bit tensor peak / 3 (hi*hi + hi*lo + lo*hi); where the library takes the
+                    gridded sum, that sum's own operations (grid_flops) on the FP32 or FP64 pipe.
     FP64 phases are set against the measured DGEMM rate (fp64_peak)."""
     from md_sim_gb300.abi import MDG_MIXED
 
@@ -230,7 +251,13 @@ def roofline(ctx, s, prm, precision, pk, config_name="", fp64_peak=None):
         t = ph[kind] * 1e-3
         if kind == "reciprocal":
             units = s.nmove * nk
-            if mixed:
+            if gridded(s, nk, precision):
+                flops = grid_flops(s, prm, mixed)
+                if mixed:
+                    bound, peak, src = "fp32", fp32_nominal_tflops(), "nominal FP32 (152 SM x 128 lanes x 2 x max clock)"
+                else:
+                    bound, peak, src = "fp64", fp64_peak, fp64_src
+            elif mixed:
                 flops, bound, peak, src = 24.0 * units, "tensor", pk["bf16_tflops"] / 3.0, pk["source"] + " bf16 burst /3"
             else:
                 flops, bound, peak, src = 18.0 * units, "fp64", fp64_peak, fp64_src
@@ -539,6 +566,7 @@ def run_workload(lib, name, args, torch, stream, flush, pk, fp64_peak, headline=
     kps = ctx.kernels_per_step()
     ctx.get_state(s)
     roof, roof_recip, roof_pairs = roofline(ctx, s, prm, precision, pk, name, fp64_peak)
+    on_grid = gridded(s, len(ctx.kvectors()[0]), precision)
     learned_rep, shake_model = None, None
     if s.ncons > 0 and args.learned and precision == MDG_MIXED:
         learned_rep, per_seed, shake_model = learned_arm(lib, ctx, s_start, args, K, stream, flush, torch, value,
@@ -555,7 +583,8 @@ def run_workload(lib, name, args, torch, stream, flush, pk, fp64_peak, headline=
     out = {
         "metric": METRIC, "value": value, "unit": UNIT, "n_gpus": 1, "steps": K, "warmup": args.warmup,
         "ms_per_step": t_step * 1e3, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "f64" if precision == MDG_FP64 else "f32 pairs + f16x3 tensor reciprocal (f64 state)",
+        "dtype": "f64" if precision == MDG_FP64 else "f32 pairs + f32 gridded reciprocal (f64 state)" if on_grid
+        else "f32 pairs + f16x3 tensor reciprocal (f64 state)",
         "data": "synthetic (seeded)",
         "config": config_dict(name, desc, args.precision, args, s),
         "e2e": e2e,

@@ -44,7 +44,7 @@ extern "C" {
 
 /* arithmetic of the force phases */
 #define MDG_FP64 0  /* every phase in FP64 (reproduces the reference) */
-#define MDG_MIXED 1 /* FP32 pairs with compensated sums, tensor-core reciprocal sum, FP64 state */
+#define MDG_MIXED 1 /* FP32 pairs with compensated sums, tensor-core or gridded FP32 reciprocal sum, FP64 state */
 
 /* quirk switches (mdg_params.quirks); default 0 reproduces the reference */
 #define MDG_QUIRK_CLEAN_SHAKE_DONE 1u /* SHAKE stops when no molecule moved (global test) instead of
@@ -353,10 +353,11 @@ int mdg_batch_run_async(mdg_batch* b, int64_t nsteps);
  * 1024 atoms, pass 2 whole atom tiles) instead of spreading each replica over every SM;
  * mdg_batch_destroy restores each replica's own plan.
  * Graph form of the batch (the next run builds it):
- *   MDG_BATCH_PHASES (default)  phase order: the head-head and head-wall loops of all replicas in
- *       the mixed form with walls and no surface atoms run as one persistent kernel each over all
- *       their heads (pair_blocks / wall_blocks blocks; 0 = 1216), between the replicas' own list
- *       builds and their merge, corrector and SHAKE; other replicas step as in their own graphs;
+ *   MDG_BATCH_PHASES (default)  phase order: the predictor, packing close, wall tail, list build,
+ *       merge and corrector of all replicas in the mixed form with walls and no surface atoms run as
+ *       one launch per kernel, their head-head and head-wall loops as one persistent kernel each
+ *       over all heads (pair_blocks / wall_blocks blocks; 0 = 1216), beside every replica's own
+ *       reciprocal sum; other replicas step as in their own graphs;
  *   MDG_BATCH_GRAPHS  every replica's own step graph as a parallel child graph. */
 #define MDG_BATCH_GRAPHS 0
 #define MDG_BATCH_PHASES 1

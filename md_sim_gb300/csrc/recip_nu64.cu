@@ -15,7 +15,7 @@
 //
 // FP64 operations bound spread and force: 1 and 2.4 per point and atom, 4,096 points.
 // 98,304 atoms, 29,038 k vectors (M = 112): spread 0.98 ms, zy 0.17, x 0.07, yz 0.11, force 1.98 = 3.3 ms where
-// the direct sums take 44; a force call 46.1 -> 5.4 ms.  6,144 atoms, 4,338 k in a slab: 0.40 ms for 0.49.
+// the direct sums take 44; a force call 46.1 -> 5.4 ms.  6,144 atoms, 4,338 k in a slab: 0.39 ms for 0.49.
 #include <algorithm>
 #include <cmath>
 #include <vector>
@@ -329,9 +329,9 @@ constexpr int kSmem = kTile * (int)sizeof(double);
 }  // namespace
 
 // Atoms times k vectors from which the grid is faster: below, its six kernels and the points of mostly empty
-// blocks cost more than the products.  Whole force calls, direct | grid: 1,000 waters (3.2e6) 367 | 374 us, 1,331
-// (6.1e6) 488 | 437, 1,728 (1.1e7) 591 | 536; slabs of 700 (3.0e6) 351 | 419, 1,000 (6.4e6) 493 | 442 and 2,048
-// waters (2.6e7) 867 | 727.
+// blocks cost more than the products.  Whole force calls, direct | grid: 1,000 waters (3.2e6) 325 | 343 us, 1,331
+// (6.1e6) 435 | 399, 1,728 (1.1e7) 550 | 476; slabs of 700 (3.0e6) 313 | 343, 1,000 (6.4e6) 435 | 376 and 2,048
+// waters (2.6e7) 821 | 615.
 constexpr double kGridWork64 = 5.0e6;
 
 // Takes the gridded sum where the rule asks for it and its tables and arrays have room; the direct sums
