@@ -457,6 +457,7 @@ struct IoBatch {
 // Queues the move of nwords 8-byte words host -> device (h2d) or back: into the batch when the
 // host side is pinned, else as a cudaMemcpyAsync on the context's stream.
 cudaError_t io_add(Ctx& c, IoBatch& b, void* dst, const void* src, long nwords, bool h2d);
+void io_add_device(IoBatch& b, void* dst, const void* src, long nwords);  // device to device, b not full
 void io_flush(Ctx& c, IoBatch& b);  // launches the batch's copy kernel and empties it
 cudaError_t pin_host_range(void* p, size_t bytes);  // cudaHostRegister + the registry of io_add
 cudaError_t unpin_host_range(void* p);

@@ -71,6 +71,14 @@ cudaError_t io_add(Ctx& c, IoBatch& b, void* dst, const void* src, long nwords, 
                            h2d ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost, c.stream);
 }
 
+void io_add_device(IoBatch& b, void* dst, const void* src, long nwords) {
+    b.src[b.nseg] = static_cast<const unsigned long long*>(src);
+    b.dst[b.nseg] = static_cast<unsigned long long*>(dst);
+    b.n[b.nseg] = nwords;
+    b.nmax = std::max(b.nmax, nwords);
+    ++b.nseg;
+}
+
 cudaError_t pin_host_range(void* p, size_t bytes) {
     cudaError_t e = cudaHostRegister(p, bytes, cudaHostRegisterMapped | cudaHostRegisterPortable);
     if (e != cudaSuccess) return e;
