@@ -283,6 +283,7 @@ struct Ctx {
     int64_t widom_cap = 0;        // Widom insertion scratch (widom.cu)
     double *d_widom_draw = nullptr, *d_widom_rot = nullptr, *d_widom_res = nullptr;
     double* h_widom_draw = nullptr;  // pinned, two chunks
+    double* h_thermo = nullptr;      // pinned copy of d_thermo, as of the last read_status
     cudaEvent_t widom_read[2] = {nullptr, nullptr};
     double* d_widom_u = nullptr;     // FP64 form: real-space energies, points, their potentials and counts
     float4* d_widom_atoms = nullptr; // FP64 form: sites the probe's O is tested against

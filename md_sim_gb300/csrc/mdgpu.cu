@@ -179,8 +179,15 @@ int sync_check(Ctx& c, const char* where) {
     return MDG_OK;
 }
 
-int read_status(Ctx& c) {
+// The status words, and the thermostat's of a resident context, queued to pinned memory.
+static int queue_status(Ctx& c) {
     MDG_CUDA(cudaMemcpyAsync(c.h_status, c.v.status, sizeof(int) * ST_NWORDS, cudaMemcpyDeviceToHost, c.stream));
+    if (c.d_thermo)
+        MDG_CUDA(cudaMemcpyAsync(c.h_thermo, c.d_thermo, sizeof(double) * TH_N, cudaMemcpyDeviceToHost, c.stream));
+    return MDG_OK;
+}
+
+static int await_status(Ctx& c) {
     int rc = sync_check(c, "status");
     if (rc) return rc;
     if (c.h_status[ST_TC_TIMEOUT]) {
@@ -189,6 +196,11 @@ int read_status(Ctx& c) {
         return set_err(&c, MDG_E_CUDA, b);
     }
     return MDG_OK;
+}
+
+int read_status(Ctx& c) {
+    const int rc = queue_status(c);
+    return rc ? rc : await_status(c);
 }
 
 // Debug runs (MDG_DEBUG_SYNC=1 in the environment at mdg_create): synchronise after every
@@ -384,6 +396,7 @@ void mdg_destroy(mdg_ctx* c) {
     if (c->h_acc) cudaFreeHost(c->h_acc);
     if (c->h_status) cudaFreeHost(c->h_status);
     if (c->h_small) cudaFreeHost(c->h_small);
+    if (c->h_thermo) cudaFreeHost(c->h_thermo);
     if (c->h_widom_draw) cudaFreeHost(c->h_widom_draw);
     for (cudaEvent_t e : c->widom_read)
         if (e) cudaEventDestroy(e);
@@ -1013,6 +1026,7 @@ int mdg_unpin_host(void* p) {
 // Resident mode
 // ---------------------------------------------------------------------------------------------
 static int resident_alloc_impl(Ctx& c) {
+    if (!c.h_thermo) MDG_CUDA(cudaMallocHost(&c.h_thermo, sizeof(double) * TH_N));
     if (c.d_thermo) return MDG_OK;
     View& v = c.v;
     const int nion = std::max(v.nliqa - v.nriga, 1), nr = std::max(v.nrig, 1);
@@ -1136,7 +1150,8 @@ int mdg_get_state(mdg_ctx* cp, mdg_state* st) {
     MDG_CUDA(cudaStreamSynchronize(c.stream));
     const int nm = v.nmove, nr = v.nrig, nion = v.nliqa - v.nriga, nold = v.ntota - v.nliqa;
     // about 60 arrays: the pinned ones leave in a kernel per IoBatch::kMax of them (one copy each took 5 us apiece:
-    // 20 steps of 2,048 waters and a frame of 16 arrays 1.64 ms, 1.46 with this and the snapshot by a kernel), the others as copies, with one wait for all
+    // 20 steps of 2,048 waters and a frame of 16 arrays 1.64 ms, 1.43 with this, the snapshot
+    // by a kernel and the status words and thermostat read together), the others as copies, with one wait for all
     IoBatch io;
     auto get = [&](double* dst, const double* src, size_t n) -> cudaError_t {
         if (io.nseg == IoBatch::kMax) io_flush(c, io);
@@ -1165,10 +1180,10 @@ int mdg_get_state(mdg_ctx* cp, mdg_state* st) {
     MDG_CUDA(get(st->rsx, v.rsx, nm));
     MDG_CUDA(get(st->rsy, v.rsy, nm));
     MDG_CUDA(get(st->rsz, v.rsz, nm));
-    double th[TH_N];
+    MDG_CUDA(get(c.h_thermo, c.d_thermo, TH_N));
     io_flush(c, io);
-    MDG_CUDA(cudaMemcpyAsync(th, c.d_thermo, sizeof(th), cudaMemcpyDeviceToHost, c.stream));
     MDG_CUDA(cudaStreamSynchronize(c.stream));
+    const double* th = c.h_thermo;
     for (int k = 0; k < 5; ++k) {
         st->s[k] = th[TH_S + k];
         st->rs[k] = th[TH_RS + k];
@@ -1261,8 +1276,7 @@ int mdg_check(mdg_ctx* cp, mdg_report* rep) {
     if (c.h_status[ST_SHAKE_RPTOL]) return set_err(&c, MDG_E_SHAKE_RPTOL, "Constraint failure");
     if (c.h_status[ST_SHAKE_MAXIT]) return set_err(&c, MDG_E_SHAKE_MAXIT, "shake(): Too many constraint iterations!");
     if (c.resident) {
-        double th[TH_N];
-        MDG_CUDA(cudaMemcpy(th, c.d_thermo, sizeof(th), cudaMemcpyDeviceToHost));
+        const double* th = c.h_thermo;
         if (!std::isfinite(th[TH_HTOT]) || !std::isfinite(th[TH_UCONF]))
             return set_err(&c, MDG_E_NAN, "non-finite energy");
         if (rep) fill_report(c, th, rep);
@@ -1314,8 +1328,11 @@ int mdg_run(mdg_ctx* cp, int64_t nsteps, mdg_report* rep) {
         if (c.h_status[ST_SHAKE_MAXIT]) return set_err(&c, MDG_E_SHAKE_MAXIT, "shake(): Too many constraint iterations!");
         done += chunk;
     }
-    double th[TH_N];
-    MDG_CUDA(cudaMemcpy(th, c.d_thermo, sizeof(th), cudaMemcpyDeviceToHost));
+    if (nsteps <= 0) {  // no chunk has read them
+        const int rc = read_status(c);
+        if (rc) return rc;
+    }
+    const double* th = c.h_thermo;
     if (!std::isfinite(th[TH_HTOT]) || !std::isfinite(th[TH_UCONF])) return set_err(&c, MDG_E_NAN, "non-finite energy");
     if (rep) fill_report(c, th, rep);
     return MDG_OK;
@@ -1759,9 +1776,11 @@ int mdg_batch_run(mdg_batch* b, int64_t nsteps, mdg_report* reps) {
         if (rc) return rc;
         if (cudaStreamSynchronize(b->stream) != cudaSuccess) return batch_err(b, MDG_E_CUDA, "batch step failed");
         bool rebuild = false;
+        for (auto* cp : b->ctx)
+            if ((rc = queue_status(*cp))) return batch_err(b, rc, cp->err);
         for (size_t i = 0; i < b->ctx.size(); ++i) {
             Ctx& c = *b->ctx[i];
-            rc = read_status(c);
+            rc = await_status(c);
             if (rc) return batch_err(b, rc, "replica " + std::to_string(i) + ": " + c.err);
             const int ovf = c.h_status[ST_LIST_OVF], wovf = c.h_status[ST_WLIST_OVF];
             if (ovf || wovf) {
@@ -1790,10 +1809,8 @@ int mdg_batch_run(mdg_batch* b, int64_t nsteps, mdg_report* reps) {
     if (reps) {
         for (size_t i = 0; i < b->ctx.size(); ++i) {
             Ctx& c = *b->ctx[i];
-            double th[TH_N];
-            if (cudaMemcpy(th, c.d_thermo, sizeof(th), cudaMemcpyDeviceToHost) != cudaSuccess)
-                return batch_err(b, MDG_E_CUDA, "batch report");
-            fill_report(c, th, &reps[i]);
+            if (nsteps <= 0 && read_status(c)) return batch_err(b, MDG_E_CUDA, "batch report");
+            fill_report(c, c.h_thermo, &reps[i]);
         }
     }
     return MDG_OK;
