@@ -11,9 +11,9 @@
 //   f_j  = -q_j grad Phi(r_j),  Phi(r) = Re sum_k C(k) e^{ik.r},  C = Ak conj(S + S_wall),
 //          Phi on the grid from C / phi^, between grid points by the window, its gradient by the
 //          window's derivative.
-// With b = 6 pi the window and its aliases leave a relative error of about 1e-6 in the reciprocal
-// forces (1e-7 in S(k)); everything between the fixed-point positions and C(k) is FP32, C(k) and
-// the energies are FP64 as in the direct form.
+// With b = 20 for spreading and 21.5 for the forces the window and its aliases leave a relative error of about
+// 3e-7 in the reciprocal forces (4e-8 in S(k)); everything between the fixed-point positions and C(k) is
+// FP32, C(k) and the energies are FP64 as in the direct form.  The Fourier sums are in nu_fourier.cuh.
 //
 // The packing of the atom records (pack.cuh) also drops each moving atom's index into the bucket of
 // its block of 8 x 8 x 8 cells.  Then, all on one stream:
