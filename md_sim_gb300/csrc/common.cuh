@@ -55,6 +55,25 @@ __device__ __forceinline__ T warp_sum(T v) {
     return v;
 }
 
+// Sums of N values over the warp (FP64): lane 32 / N k gets that of v[k].  Each step halves the values a lane still carries, so that a sum takes 9 FP64 additions for 8 values
+// where one butterfly after the other takes 40: at the end of a block all its warps queue for the FP64 pipe.
+template <int N>
+__device__ __forceinline__ double warp_sums(double (&v)[N]) {
+    const int lane = threadIdx.x & 31;
+    int o = 16;
+#pragma unroll
+    for (int n = N / 2; n > 0; n >>= 1, o >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int k = 0; k < n; ++k) {
+            const double keep = up ? v[k + n] : v[k], send = up ? v[k] : v[k + n];
+            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    return v[0];
+}
+
 // Block-wide sum into *dst with one atomic per block; all threads must call.  Blocks smaller than
 // a warp (used to spread FP64-heavy per-molecule work over more SMs) reduce within their lanes.
 template <int NT>

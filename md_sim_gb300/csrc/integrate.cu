@@ -363,9 +363,10 @@ __global__ void __launch_bounds__(NT) k_pred(View v, Dyn D, Clear z, PackArgs P)
             pack_atom(v, P.pk, a, v.x[a], v.y[a], v.z[a], 0.0, 0.0, 0.0, false);
     }
     if (blockIdx.x < npred) {
-        block_atomic_sum<NT>(kp, &D.isum[0]);
-        for (int d = 0; d < 3; ++d) block_atomic_sum<NT>(sc[d], &D.isum[1 + d]);
-        for (int d = 0; d < 3; ++d) block_atomic_sum<NT>(sw[d], &D.isum[4 + d]);
+        double t[8] = {kp, sc[0], sc[1], sc[2], sw[0], sw[1], sw[2], 0.0};
+        const double sum = warp_sums(t);
+        const int lane = threadIdx.x & 31;
+        if ((lane & 3) == 0 && lane < 28) atomicAdd(&D.isum[lane >> 2], sum);
     }
     pred_end<PACK>(v, D, P, mz, md, red, blockIdx.x, gridDim.x);
 }
@@ -710,9 +711,10 @@ __global__ void __launch_bounds__(NT) k_corr(View v, Dyn D, int slab, MergeArgs 
         }
     }
     if constexpr (MERGE) {
-        block_atomic_sum<NT>(sx, &v.acc[2 * v.nijt + ACC_FWS0 + 0]);
-        block_atomic_sum<NT>(sy, &v.acc[2 * v.nijt + ACC_FWS0 + 1]);
-        block_atomic_sum<NT>(sz, &v.acc[2 * v.nijt + ACC_FWS0 + 2]);
+        double t[4] = {sx, sy, sz, 0.0};
+        const double sum = warp_sums(t);
+        const int lane = threadIdx.x & 31;
+        if ((lane & 7) == 0 && lane < 24) atomicAdd(&v.acc[2 * v.nijt + ACC_FWS0 + (lane >> 3)], sum);
     }
     __shared__ double sh_acc[kTailAcc];
     corr_end(v, D, slab, sh_acc, gridDim.x);
@@ -927,7 +929,8 @@ Dyn dyn_of(Ctx& c) {
 // Units up to which the forms for small systems are the faster ones: with more the FP64 pipe is the limit and
 // their half-filled warps cost (bulk water, k_pred and k_corr, one thread per molecule | component): 1,000
 // 17 and 17 | 8 and 11 us, 4,913 19 and 17 | 11 and 13, 8,000 19 and 18 | 12 and 15, 15,625 19 and 19 | 19
-// and 20, 32,768 28 and 25 | 37 and 33.
+// and 20, 32,768 28 and 25 (24 and
+// 24 since a warp's sums share their steps) | 37 and 33.
 bool small(int nu) { return nu <= 80 * kSM; }
 int nblk(int n) { return std::max(1, std::min((n + 127) / 128, kSM * 8)); }
 

@@ -79,25 +79,6 @@ __device__ __forceinline__ void e_flush(EAcc& e, double* s_e, int nijt) {
     e.qq = Kahan();
 }
 
-// Sums of N values over the warp (FP64): lane 32 / N k gets that of v[k].  Each step halves the values a lane still carries, so that a sum takes 9 FP64 additions for 8 values
-// where one butterfly after the other takes 40: at the end of a block all its warps queue for the FP64 pipe.
-template <int N>
-__device__ __forceinline__ double warp_sums(double (&v)[N]) {
-    const int lane = threadIdx.x & 31;
-    int o = 16;
-#pragma unroll
-    for (int n = N / 2; n > 0; n >>= 1, o >>= 1) {
-        const bool up = lane & o;
-#pragma unroll
-        for (int k = 0; k < n; ++k) {
-            const double keep = up ? v[k + n] : v[k], send = up ? v[k] : v[k + n];
-            v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
-        }
-    }
-    for (; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-    return v[0];
-}
-
 // All lanes of a warp: lanes holding the warp's (largest) pair type of an accumulator reduce with shuffles in
 // FP64 (a warp's total grows with the heads it took, and an FP32 reduction of it would round at that
 // size), one shared atomic per sum; lanes left with another type flush one by one.  Leaves e empty.
