@@ -397,12 +397,16 @@ int pair_blocks(int units) { return std::max(1, std::min((units + kWarps - 1) / 
 
 }  // namespace
 
+// The table lives in a static device array: one per GPU, the same bytes for every context.
+static __device__ __align__(128) double g_etab[kEtRows * 16];
+
 int pair_setup(Ctx& c) {
+    if (c.precision == MDG_MIXED) return MDG_OK;
     static const std::vector<double> table = ewald_table(c.v.spii);  // of the functions, no system's own
-    double2* d = (double2*)dalloc(c, sizeof(double) * table.size());
-    if (c.alloc_failed) return set_err(&c, MDG_E_CUDA, "out of device memory");
-    MDG_CUDA(cudaMemcpy(d, table.data(), sizeof(double) * table.size(), cudaMemcpyHostToDevice));
-    c.v.etab = d;
+    void* p = nullptr;
+    MDG_CUDA(cudaGetSymbolAddress(&p, g_etab));
+    MDG_CUDA(cudaMemcpy(p, table.data(), sizeof(double) * table.size(), cudaMemcpyHostToDevice));
+    c.v.etab = static_cast<const double2*>(p);
     return MDG_OK;
 }
 
