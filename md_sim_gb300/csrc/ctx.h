@@ -300,7 +300,8 @@ struct Ctx {
     double *d_ang_kt = nullptr, *d_ang_th = nullptr;
     std::vector<double> h_qs_wall;  // wall charges (for the static structure factor)
     double *d_ft = nullptr, *d_fc = nullptr, *d_tq = nullptr;  // force_sum outputs
-    bool alloc_failed = false;
+    bool alloc_failed = false;    // since creation began, or since the mark of the arrays being taken
+    int fail_alloc = 0;           // debug: this allocation from now on fails (MDG_DEBUG_FAIL_ALLOC at creation)
     int batch_stage = 0;          // captures of a phase-ordered replica batch: 1 up to the list, 2 after the loops
     bool debug_sync = false;
     // resident mode
@@ -474,7 +475,17 @@ void step_close_launch(Ctx& c);
 void correct_launch(Ctx& c, bool merge = false);
 
 int set_err(Ctx* c, int code, const std::string& msg);
-void* dalloc(Ctx& c, size_t bytes);
+void* dalloc(Ctx& c, size_t bytes);  // zeroed device memory, the context's own; nullptr: alloc_failed is set
+template <typename T>
+bool halloc(Ctx& c, T** p, size_t bytes) {  // pinned host memory; false: alloc_failed is set, *p null
+    *p = nullptr;
+    if (!(c.fail_alloc > 0 && --c.fail_alloc == 0) && cudaMallocHost((void**)p, bytes) == cudaSuccess) return true;
+    *p = nullptr;
+    c.alloc_failed = true;
+    return false;
+}
+// Arrays taken by dalloc since owned.size() was `mark` are given back, and the failure among them is forgotten.
+void drop_owned(Ctx& c, size_t mark);
 
 }  // namespace mdg
 

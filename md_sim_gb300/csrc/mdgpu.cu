@@ -28,13 +28,19 @@ int set_err(Ctx* c, int code, const std::string& msg) {
 void* dalloc(Ctx& c, size_t bytes) {
     void* p = nullptr;
     bytes = std::max<size_t>(bytes, 16);
-    if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    if ((c.fail_alloc > 0 && --c.fail_alloc == 0) || cudaMalloc(&p, bytes) != cudaSuccess) {
         c.alloc_failed = true;
         return nullptr;
     }
     cudaMemset(p, 0, bytes);
     c.owned.push_back(p);
     return p;
+}
+
+void drop_owned(Ctx& c, size_t mark) {
+    for (; c.owned.size() > mark; c.owned.pop_back()) cudaFree(c.owned.back());
+    cudaGetLastError();  // the allocation's error, which the caller reports or lives with
+    c.alloc_failed = false;
 }
 
 static void dfree(Ctx& c, void* p) {
@@ -443,12 +449,15 @@ int mdg_create(const mdg_sysdesc* s, const mdg_params* p, const double* x0, cons
     {
         const char* dbg = getenv("MDG_DEBUG_SYNC");
         c.debug_sync = dbg && dbg[0] == '1';
+        dbg = getenv("MDG_DEBUG_FAIL_ALLOC");  // tests: the n-th allocation of this context fails
+        c.fail_alloc = dbg ? std::atoi(dbg) : 0;
     }
     c.variant = p->variant;
     c.quirks = p->quirks;
     auto bail = [&](int code) {
         std::string m = c.err;
         mdg_destroy(cp);
+        cudaGetLastError();  // reported here, and not the next call's
         return set_err(nullptr, code, m.empty() ? "mdg_create failed" : m);
     };
     // The reciprocal branch is the longest of a force evaluation: its stream gets the highest
@@ -590,10 +599,9 @@ int mdg_create(const mdg_sysdesc* s, const mdg_params* p, const double* x0, cons
     c.d_ft = (double*)dalloc(c, sizeof(double) * 3 * std::max(nflex, 1));
     c.d_fc = (double*)dalloc(c, sizeof(double) * 3 * std::max(v.nrig, 1));
     c.d_tq = (double*)dalloc(c, sizeof(double) * 3 * std::max(v.nrig, 1));
-    if (cudaMallocHost(&c.h_acc, sizeof(double) * (2 * nijt + ACC_NSLOT)) != cudaSuccess ||
-        cudaMallocHost(&c.h_status, sizeof(int) * ST_NWORDS) != cudaSuccess ||
-        cudaMallocHost(&c.h_small, sizeof(double) * (std::max(v.nit, 1) + 1)) != cudaSuccess)
-        c.alloc_failed = true;
+    halloc(c, &c.h_acc, sizeof(double) * (2 * nijt + ACC_NSLOT));
+    halloc(c, &c.h_status, sizeof(int) * ST_NWORDS);
+    halloc(c, &c.h_small, sizeof(double) * (std::max(v.nit, 1) + 1));
     if (c.alloc_failed) {
         c.err = "out of device memory";
         return bail(MDG_E_CUDA);
@@ -668,6 +676,10 @@ int mdg_create(const mdg_sysdesc* s, const mdg_params* p, const double* x0, cons
         c.d_ang = reinterpret_cast<int*>(upload(c, terms));
         c.d_ang_kt = upload(c, kt);
         c.d_ang_th = upload(c, th);
+    }
+    if (c.alloc_failed) {  // of the arrays since the test above; no kernel has run yet
+        c.err = "out of device memory";
+        return bail(MDG_E_CUDA);
     }
     c.nfreed = 3 * (s->nmove - s->nliqa);
     for (int64_t it = s->nltype; it < s->ntype; ++it)

@@ -340,17 +340,17 @@ int recip_nu64_setup(Ctx& c) {
     const View& v = c.v;
     if (c.ks.nk == 0 || (double)v.nmove * c.ks.nk < kGridWork64) return MDG_OK;
     NuPlanT<double>& plan = c.nu64;
-    const size_t owned = c.owned.size();
+    // what is forgiven below is what this function asks for
+    if (c.alloc_failed) return set_err(&c, MDG_E_CUDA, "out of device memory for the reciprocal sum");
+    const size_t mark = c.owned.size();
     const int rc = nu_setup<double>(
         c, plan, [](int K) { return std::max(24, (9 * K / 2 + 4 + 7) / 8 * 8); },
         [](int, int k, int M) { return inverse_transform(k, M); });
     if (rc == MDG_OK) plan.rec = (double2*)dalloc(c, 2 * sizeof(double2) * ((size_t)plan.g.nblk * plan.g.cap + v.nmove));
     if (rc != MDG_OK || c.alloc_failed) {
-        for (; c.owned.size() > owned; c.owned.pop_back()) cudaFree(c.owned.back());
+        drop_owned(c, mark);
         plan = NuPlanT<double>();
-        c.alloc_failed = false;
         c.err.clear();
-        cudaGetLastError();
         return MDG_OK;
     }
     static const NuPoly64 P = window_poly();

@@ -1,0 +1,49 @@
+"""Allocations that fail, one after the other (MDG_DEBUG_FAIL_ALLOC: the n-th of a context, on the host): a call that
+does without one of its arrays says so, and nothing runs on an array that is not there."""
+import numpy as np
+import pytest
+
+from md_sim_gb300 import abi, configs
+
+pytestmark = pytest.mark.gpu
+
+SYSTEMS = {
+    "fp64 direct": (abi.MDG_FP64, lambda: configs.slab_water(96, 6, kmax=6, placement="lattice")),
+    "fp64 gridded": (abi.MDG_FP64, lambda: configs.slab_water(700, 7, kmax=12, placement="lattice")),
+    "mixed": (abi.MDG_MIXED, lambda: configs.slab_water(96, 6, kmax=6, placement="lattice")),
+    "mixed gridded": (abi.MDG_MIXED, lambda: configs.slab_water(64, 6, kmax=6, lz=6 * 4.21 * 5.6, placement="lattice")),
+}
+MOST = 130  # more than a context's creation asks for
+
+
+def _system(name):
+    precision, make = SYSTEMS[name]
+    s, prm = make()
+    prm.precision = precision
+    return s, prm
+
+
+@pytest.mark.parametrize("name", list(SYSTEMS))
+def test_creation(name, gpulib, monkeypatch):
+    """Every allocation of mdg_create in turn: no context, or (where the direct FP64 sums take the place of the
+    gridded one) a context that works."""
+    s, prm = _system(name)
+    ref = abi.Context(gpulib, s.copy(), prm)
+    a = ref.force_get(s.copy())["f"]
+    ref.close()
+    refused = []
+    for n in range(1, MOST):
+        monkeypatch.setenv("MDG_DEBUG_FAIL_ALLOC", str(n))
+        try:
+            ctx = abi.Context(gpulib, s.copy(), prm)
+        except abi.MdgError as e:
+            assert abi.ERRORS[e.code] == "MDG_E_CUDA", e
+            refused.append(n)
+            continue
+        # the bars of the two forms against the oracle, of either sum
+        bar = 1e-5 if prm.precision == abi.MDG_MIXED else 2e-12
+        b = ctx.force_get(s.copy())["f"]
+        assert np.linalg.norm(b - a) <= bar * np.linalg.norm(a), n
+        ctx.close()
+    assert len(refused) > 60 and refused[-1] < MOST - 5
+    assert name == "fp64 gridded" or refused == list(range(1, len(refused) + 1))
