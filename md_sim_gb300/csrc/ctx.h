@@ -280,7 +280,8 @@ struct Ctx {
     bool pack_force = false;
     Meas meas;                    // measurement histograms (measure.cu)
     std::vector<int64_t> h_moltypen, h_nt, h_ns, h_itype;  // molecule types and site types (cfgio.cu)
-    int64_t widom_cap = 0;        // Widom insertion scratch (widom.cu)
+    int64_t widom_cap = 0;        // Widom insertion scratch (widom.cu): positions d_widom_res holds
+    bool widom_ready = false;     // all of the rest is there
     double *d_widom_draw = nullptr, *d_widom_rot = nullptr, *d_widom_res = nullptr;
     double* h_widom_draw = nullptr;  // pinned, two chunks
     double* h_thermo = nullptr;      // pinned copy of d_thermo, as of the last read_status

@@ -349,10 +349,14 @@ int measure_init(Ctx& c, const mdg_measure_params* p, mdg_measure_dims* d) {
     // doubles: efipos 2L | tefipos 2L | ndip 4L | mu 3L | ftot 9 | pos 3 nmove
     const size_t o_tef = 2 * L, o_ndip = 4 * L, o_mu = 8 * L, o_ftot = 11 * L, o_pos = 11 * L + 9;
     const size_t nd = o_pos + 3 * (size_t)std::max(v.nmove, 1);
+    const size_t mark = c.owned.size();
     auto* u = static_cast<unsigned long long*>(dalloc(c, sizeof(unsigned long long) * nu));
     auto* dd = static_cast<double*>(dalloc(c, sizeof(double) * nd));
     int* amt = c.h_ang_mt.empty() ? nullptr : static_cast<int*>(dalloc(c, sizeof(int) * c.h_ang_mt.size()));
-    if (!u || !dd || (!c.h_ang_mt.empty() && !amt)) return set_err(&c, MDG_E_CUDA, "measure: out of device memory");
+    if (c.alloc_failed) {
+        drop_owned(c, mark);
+        return set_err(&c, MDG_E_CUDA, "measure: out of device memory");
+    }
     if (amt) MDG_CUDA(cudaMemcpy(amt, c.h_ang_mt.data(), sizeof(int) * c.h_ang_mt.size(), cudaMemcpyHostToDevice));
     m.ngc = u;
     m.nefipos = m.ngc + (size_t)v.nijt * L;

@@ -538,6 +538,59 @@ __global__ void __launch_bounds__(kWT) k_widom(View v, WArgs w) {
     if (t == 0) w.res[ins] = make_double2(acc, 0.0);
 }
 
+// Scratch of the calls: results grow on demand, the rest is sized for one chunk and taken whole or not at all, so
+// that the call after one that found no memory starts over.
+int widom_scratch(Ctx& c, int64_t nins) {
+    const KSet& ks = c.ks;
+    const View& v = c.v;
+    const size_t mark = c.owned.size();
+    const char* oom = "Widom insertion: out of memory";
+    if (c.widom_cap < nins) {
+        const int64_t cap = std::max<int64_t>(nins, 256);
+        double* res = (double*)dalloc(c, sizeof(double) * 2 * cap);
+        if (!res) {
+            drop_owned(c, mark);
+            return set_err(&c, MDG_E_CUDA, oom);
+        }
+        c.d_widom_res = res;
+        c.widom_cap = cap;
+    }
+    if (c.widom_ready) return MDG_OK;
+    const size_t rest = c.owned.size();
+    c.d_widom_rot = (double*)dalloc(c, sizeof(double) * kIns * kMaxRot * 6);
+    c.d_widom_draw = (double*)dalloc(c, sizeof(double) * kIns * kDraw);
+    if (c.precision != MDG_MIXED) {
+        // real-space energies, points, potentials (doubles), first points and two counts (int)
+        c.d_widom_u = (double*)dalloc(c, (sizeof(double) * (kMaxRot + 4 * kPts) + sizeof(int)) * kIns + 2 * sizeof(int));
+        c.d_widom_pm = (double2*)dalloc(c, 2 * sizeof(double2) * std::max(ks.nent, 1));
+        c.d_widom_atoms = (float4*)dalloc(c, sizeof(float4) * std::max(v.ntota, 1));
+    } else {
+        const int nk = std::max(ks.nk, 1);
+        c.d_widom_akf = (float*)dalloc(c, sizeof(float) * nk);
+        c.d_widom_qsf = (float2*)dalloc(c, sizeof(float2) * nk);
+        c.d_widom_rsf = (float4*)dalloc(c, sizeof(float4) * std::max(v.ntota, 1));
+    }
+    if (!c.h_widom_draw) halloc(c, &c.h_widom_draw, sizeof(double) * 2 * kIns * kDraw);
+    for (cudaEvent_t& e : c.widom_read)
+        if (!e && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) {
+            e = nullptr;
+            c.alloc_failed = true;
+        }
+    if (c.alloc_failed) {
+        drop_owned(c, rest);
+        return set_err(&c, MDG_E_CUDA, oom);
+    }
+    if (c.precision == MDG_MIXED && ks.nk > 0) {
+        std::vector<double> ak(ks.nk);
+        std::vector<float> akf(ks.nk);
+        MDG_CUDA(cudaMemcpy(ak.data(), ks.ak, sizeof(double) * ks.nk, cudaMemcpyDeviceToHost));
+        for (int k = 0; k < ks.nk; ++k) akf[k] = (float)ak[k];
+        MDG_CUDA(cudaMemcpy(c.d_widom_akf, akf.data(), sizeof(float) * ks.nk, cudaMemcpyHostToDevice));
+    }
+    c.widom_ready = true;
+    return MDG_OK;
+}
+
 }  // namespace
 
 int widom(Ctx& c, const mdg_widom_params* p, double* seed, double* pave, int64_t* inave, int64_t* done) {
@@ -556,28 +609,7 @@ int widom(Ctx& c, const mdg_widom_params* p, double* seed, double* pave, int64_t
     const double chtemper = p->temper > 0.0 ? p->temper : 300.0;
     const double beta = 1000.0 / ((double)8.31441f * chtemper);
     const double M_PI_R = (double)3.1415926535898f;
-    // scratch: results grow on demand, the rest is sized for one chunk
-    if (c.widom_cap < nins) {
-        const int64_t cap = std::max<int64_t>(nins, 256);
-        c.d_widom_res = (double*)dalloc(c, sizeof(double) * 2 * cap);
-        if (c.alloc_failed) return set_err(&c, MDG_E_CUDA, "Widom insertion: out of device memory");
-        c.widom_cap = cap;
-    }
-    if (!c.d_widom_draw) {
-        c.d_widom_rot = (double*)dalloc(c, sizeof(double) * kIns * kMaxRot * 6);
-        if (c.precision != MDG_MIXED) {
-            // real-space energies, points, potentials (doubles), first points and two counts (int)
-            c.d_widom_u = (double*)dalloc(c, (sizeof(double) * (kMaxRot + 4 * kPts) + sizeof(int)) * kIns + 2 * sizeof(int));
-            c.d_widom_pm = (double2*)dalloc(c, 2 * sizeof(double2) * std::max(ks.nent, 1));
-            c.d_widom_atoms = (float4*)dalloc(c, sizeof(float4) * std::max(v.ntota, 1));
-        }
-        c.d_widom_draw = (double*)dalloc(c, sizeof(double) * kIns * kDraw);
-        if (!c.alloc_failed && (cudaMallocHost(&c.h_widom_draw, sizeof(double) * 2 * kIns * kDraw) != cudaSuccess ||
-                                cudaEventCreateWithFlags(&c.widom_read[0], cudaEventDisableTiming) != cudaSuccess ||
-                                cudaEventCreateWithFlags(&c.widom_read[1], cudaEventDisableTiming) != cudaSuccess))
-            c.alloc_failed = true;
-        if (c.alloc_failed) return set_err(&c, MDG_E_CUDA, "Widom insertion: out of memory");
-    }
+    if (const int rc = widom_scratch(c, nins)) return rc;
     double dipz = 0.0;
     if (p->flags & MDG_WIDOM_EW3DC)
         MDG_CUDA(cudaMemcpy(&dipz, v.acc + 2 * v.nijt + ACC_DIPZ, sizeof(double), cudaMemcpyDeviceToHost));
@@ -612,17 +644,6 @@ int widom(Ctx& c, const mdg_widom_params* p, double* seed, double* pave, int64_t
     w.rsf = nullptr;
     W64 s{};
     if (mx) {
-        if (!c.d_widom_akf) {
-            std::vector<float> akf(std::max(ks.nk, 1));
-            std::vector<double> ak(ks.nk);
-            if (ks.nk) MDG_CUDA(cudaMemcpy(ak.data(), ks.ak, sizeof(double) * ks.nk, cudaMemcpyDeviceToHost));
-            for (int k = 0; k < ks.nk; ++k) akf[k] = (float)ak[k];
-            c.d_widom_akf = (float*)dalloc(c, sizeof(float) * akf.size());
-            c.d_widom_qsf = (float2*)dalloc(c, sizeof(float2) * akf.size());
-            c.d_widom_rsf = (float4*)dalloc(c, sizeof(float4) * std::max(v.ntota, 1));
-            if (c.alloc_failed) return set_err(&c, MDG_E_CUDA, "Widom insertion: out of device memory");
-            MDG_CUDA(cudaMemcpy(c.d_widom_akf, akf.data(), sizeof(float) * akf.size(), cudaMemcpyHostToDevice));
-        }
         const int np = std::max(std::max(ks.nk, v.ntota), 1);
         k_widom_prep<<<std::min((np + 255) / 256, 152 * 4), 256, 0, c.stream>>>(v, ks.s, ks.qw, c.d_widom_qsf, ks.nk,
                                                                              c.d_widom_rsf);

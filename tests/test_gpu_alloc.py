@@ -47,3 +47,38 @@ def test_creation(name, gpulib, monkeypatch):
         ctx.close()
     assert len(refused) > 60 and refused[-1] < MOST - 5
     assert name == "fp64 gridded" or refused == list(range(1, len(refused) + 1))
+
+
+@pytest.mark.parametrize("name", ["fp64 direct", "mixed"])
+def test_widom(name, gpulib, monkeypatch):
+    """Every allocation of the first insertion call in turn: it reports the failure, and the next call inserts as
+    if nothing had been."""
+    s, prm = _system(name)
+
+    def insert(ctx):
+        return ctx.widom(20, 1.0, 4.0, 8, 0, 14135621772.0, flags=abi.MDG_WIDOM_SKIP_OVERLAP)
+
+    ctx = abi.Context(gpulib, s.copy(), prm)
+    ctx.force_get(s.copy())
+    want = insert(ctx)
+    ctx.close()
+    failed = 0
+    for n in range(1, MOST):
+        monkeypatch.setenv("MDG_DEBUG_FAIL_ALLOC", str(n))
+        try:
+            ctx = abi.Context(gpulib, s.copy(), prm)
+        except abi.MdgError:
+            continue
+        ctx.force_get(s.copy())
+        try:
+            got = insert(ctx)
+        except abi.MdgError as e:
+            assert "out of memory" in str(e)
+            failed += 1
+            got = insert(ctx)
+        assert got["seed"] == want["seed"] and got["done"] == want["done"]
+        np.testing.assert_array_equal(got["inave"], want["inave"])
+        # sums in another order, of energies with atomically added terms
+        assert np.abs(got["pave"] - want["pave"]).max() <= (1e-4 if name == "mixed" else 1e-9) * want["pave"].max()
+        ctx.close()
+    assert failed == 7  # six arrays and the pinned staging
