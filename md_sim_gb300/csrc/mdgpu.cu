@@ -1038,10 +1038,11 @@ int mdg_unpin_host(void* p) {
 // Resident mode
 // ---------------------------------------------------------------------------------------------
 static int resident_alloc_impl(Ctx& c) {
-    if (!c.h_thermo) MDG_CUDA(cudaMallocHost(&c.h_thermo, sizeof(double) * TH_N));
-    if (c.d_thermo) return MDG_OK;
+    if (c.d_snap) return MDG_OK;  // the last of them
     View& v = c.v;
+    const size_t mark = c.owned.size();
     const int nion = std::max(v.nliqa - v.nriga, 1), nr = std::max(v.nrig, 1);
+    if (!c.h_thermo) halloc(c, &c.h_thermo, sizeof(double) * TH_N);
     c.d_xd = (double*)dalloc(c, sizeof(double) * 12 * nion);
     c.d_c = (double*)dalloc(c, sizeof(double) * 15 * nr);
     c.d_q = (double*)dalloc(c, sizeof(double) * 20 * nr);
@@ -1050,13 +1051,9 @@ static int resident_alloc_impl(Ctx& c) {
     c.d_thermo = (double*)dalloc(c, sizeof(double) * TH_N);
     c.d_isum = (double*)dalloc(c, sizeof(double) * 8);
     c.d_done = (unsigned*)dalloc(c, sizeof(unsigned) * 4);
-    if (c.alloc_failed) return set_err(&c, MDG_E_CUDA, "out of device memory for the integrator state");
-    // the centres of mass of the force phases become the first Gear slice
-    v.cx = c.d_c;
-    v.cy = c.d_c + nr;
-    v.cz = c.d_c + 2 * nr;
     // regions saved before each chunk of steps (restored when the list must grow)
     const int nold = v.ntota - v.nliqa, nflex = v.nmove - v.nriga;
+    c.snap_regions.clear();
     auto add = [&](void* p, size_t b) {
         if (p && b) c.snap_regions.push_back({p, b});
     };
@@ -1073,7 +1070,16 @@ static int resident_alloc_impl(Ctx& c) {
     size_t tot = 0;
     for (auto& r : c.snap_regions) tot += (r.second + 255) / 256 * 256;
     c.d_snap = (char*)dalloc(c, tot);
-    if (c.alloc_failed) return set_err(&c, MDG_E_CUDA, "out of device memory for the step snapshot");
+    if (c.alloc_failed) {  // all of them or none: the next call starts over
+        drop_owned(c, mark);
+        c.d_thermo = nullptr;
+        c.d_snap = nullptr;
+        return set_err(&c, MDG_E_CUDA, "out of device memory for the integrator state");
+    }
+    // the centres of mass of the force phases become the first Gear slice
+    v.cx = c.d_c;
+    v.cy = c.d_c + nr;
+    v.cz = c.d_c + 2 * nr;
     return MDG_OK;
 }
 

@@ -82,3 +82,36 @@ def test_widom(name, gpulib, monkeypatch):
         assert np.abs(got["pave"] - want["pave"]).max() <= (1e-4 if name == "mixed" else 1e-9) * want["pave"].max()
         ctx.close()
     assert failed == 7  # six arrays and the pinned staging
+
+
+@pytest.mark.parametrize("name", ["fp64 direct", "mixed"])
+def test_resident_state(name, gpulib, monkeypatch):
+    """Every allocation of the first mdg_set_state in turn: it reports the failure, and the next one starts a run like
+    any other."""
+    s, prm = _system(name)
+    ctx = abi.Context(gpulib, s.copy(), prm)
+    ctx.set_state(ctx.sys)
+    ctx.run(2)
+    ctx.get_state()
+    want = ctx.sys.x0.copy()
+    ctx.close()
+    failed = 0
+    for n in range(1, MOST):
+        monkeypatch.setenv("MDG_DEBUG_FAIL_ALLOC", str(n))
+        try:
+            ctx = abi.Context(gpulib, s.copy(), prm)
+        except abi.MdgError:
+            continue
+        try:
+            ctx.set_state(ctx.sys)
+        except abi.MdgError as e:
+            assert "out of device memory" in str(e)
+            failed += 1
+            ctx.force_get(ctx.sys.copy())  # the drop-in call goes on as before
+            ctx.set_state(ctx.sys)
+        ctx.run(2)
+        ctx.get_state()
+        # atomically added forces: rounding of FP64, of FP32 in the mixed form
+        assert np.abs(ctx.sys.x0 - want).max() <= (1e-7 if name == "mixed" else 1e-11) * s.lx
+        ctx.close()
+    assert failed == 10  # the pinned thermostat values, eight arrays and the snapshot
