@@ -445,7 +445,7 @@ __device__ __forceinline__ void pair_heads(const View& v, const Pk& pk, const Ta
                 if (k + 64 < n) j2 = nb[k + 64];
                 float dx, dy, dz;
                 head_vec<ZPER>(pi, zli, pj, pk, j, dx, dy, dz);
-                Q.push(k < n && dx * dx + dy * dy + dz * dz <= rcutsq, dx, dy, dz, j, pj.w);
+                Q.push(k < n && !(dx * dx + dy * dy + dz * dz > rcutsq), dx, dy, dz, j, pj.w);  // NaN too
             }
             if (Q.n > 0) evaluate(min(Q.n, 32));
         }
@@ -590,7 +590,7 @@ __device__ __forceinline__ void wall_heads(const View& v, const Pk& pk, const Ta
                 if (k + 64 < n) j2 = nb[k + 64];
                 float dx, dy, dz;
                 head_vec<ZPER>(pi, zli, pj, pk, j, dx, dy, dz);
-                Q.push(k < n && dx * dx + dy * dy + dz * dz <= rcutsq, dx, dy, dz, j, pj.w);
+                Q.push(k < n && !(dx * dx + dy * dy + dz * dz > rcutsq), dx, dy, dz, j, pj.w);
             }
             if (Q.n > 0) evaluate(min(Q.n, 32));
         }
