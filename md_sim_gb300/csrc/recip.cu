@@ -45,7 +45,7 @@ namespace {
 constexpr int kChunk = 13;    // most entries per work item in k_sfac (4 sums each, in registers)
 constexpr int kSfacNT = 128;
 constexpr int kForceNT = 64;
-constexpr int kSfacTile = 32;   // atoms per phase table of k_sfac
+constexpr int kSfacTile = 32;   // most atoms per phase table of k_sfac (fewer where one atom's factors are many)
 constexpr int kMaxSplit = 64;   // most grid rows of k_kforce
 
 // Entries of a row: n = 0..nmax, whose (n, -n) are the row's k vectors ((0, 0, n > 0) for the first).
@@ -79,7 +79,7 @@ __device__ void phase_table(double a, int K, double2* t, int stride) {
 // rows: (l, m, n_first, k_first); witem_n: first entry | entries << 16 of each work item
 __global__ void __launch_bounds__(kSfacNT) k_sfac(View v, KDims d, int nrow, const int4* __restrict__ rows,
                                                   const int* __restrict__ witem_row, const int* __restrict__ witem_n,
-                                                  int nwork, int atoms_per_split, double2* S, int nk_total) {
+                                                  int nwork, int tile, int atoms_per_split, double2* S, int nk_total) {
     extern __shared__ double2 sm[];
     // per atom: q e^{i l tx} (l = 0..KL), e^{i m ty} (m = 0..KM), e^{i n tz} (n = 0..KN)
     const int per = d.KL + 1 + d.KM + 1 + d.KN + 1;
@@ -103,13 +103,13 @@ __global__ void __launch_bounds__(kSfacNT) k_sfac(View v, KDims d, int nrow, con
     for (int c = 0; c < kChunk; ++c) x1[c] = x2[c] = x3[c] = x4[c] = 0.0;
     const int a_begin = blockIdx.y * atoms_per_split;
     const int a_end = min(v.nmove, a_begin + atoms_per_split);
-    for (int t0 = a_begin; t0 < a_end; t0 += kSfacTile) {
-        const int nt = min(kSfacTile, a_end - t0);
+    for (int t0 = a_begin; t0 < a_end; t0 += tile) {
+        const int nt = min(tile, a_end - t0);
         __syncthreads();
         for (int s = threadIdx.x; s < nt * 3; s += blockDim.x) {
             const int a = s % nt, which = s / nt;
             const int at = CK(t0 + a, v.nmove, 202);
-            double2* base = sm + (size_t)CK(a, kSfacTile, 203) * per;
+            double2* base = sm + (size_t)CK(a, tile, 203) * per;
             if (which == 0) {
                 phase_table(d.px * v.x[at], d.KL, base, 1);
                 const double q = v.q[at];
@@ -354,8 +354,14 @@ int sfac_items(const int4* rows, const int* nlen, int nrow, int* ent, int* wr, i
 // (both kernels keep the FP64 pipe busy with four warps per SM), at least 4 atoms and 4 rows each.
 struct KGrid {
     dim3 sfac, force;
-    int atoms_per_split, smem_sfac, smem_force;
+    int tile, atoms_per_split, smem_sfac, smem_force;
 };
+constexpr int kTableRoom = 200 * 1024;  // shared memory for phase tables
+// Whether the phase tables fit: 8 atoms of k_sfac, and (the limit set by a block of 128 atoms) k_kforce's.
+bool tables_fit(const KDims& d) {
+    const int per = (d.KL + 1 + d.KM + 1 + d.KN + 1) * (int)sizeof(double2) + (int)sizeof(double);
+    return 128 * (d.KM + 1 + d.KN + 1) * (int)sizeof(double2) <= kTableRoom && 8 * per <= kTableRoom;
+}
 KGrid k_grid(const KDims& d, int natom, int nrow, int nwork) {
     KGrid g;
     const int kb = std::max(1, (nwork + kSfacNT - 1) / kSfacNT), fb = std::max(1, (natom + kForceNT - 1) / kForceNT);
@@ -364,7 +370,9 @@ KGrid k_grid(const KDims& d, int natom, int nrow, int nwork) {
     splits = (natom + g.atoms_per_split - 1) / g.atoms_per_split;
     g.sfac = dim3(kb, splits);
     g.force = dim3(fb, std::max(1, std::min({(152 * 16 + fb - 1) / fb, kMaxSplit, nrow / 4})));
-    g.smem_sfac = kSfacTile * (d.KL + 1 + d.KM + 1 + d.KN + 1) * (int)sizeof(double2);
+    const int per = (d.KL + 1 + d.KM + 1 + d.KN + 1) * (int)sizeof(double2);
+    g.tile = std::min(kSfacTile, kTableRoom / per);  // (at least 8: tables_fit)
+    g.smem_sfac = g.tile * per;
     g.smem_force = kForceNT * (d.KM + 1 + d.KN + 1) * (int)sizeof(double2);
     return g;
 }
@@ -487,10 +495,7 @@ int recip_setup(Ctx& c, int64_t kmax, const double* x0, const double* y0, const 
     MDG_CUDA(allow_max_smem(k_kforce));
     MDG_CUDA(allow_max_smem(k_pot));
     ks.nent = nent;
-    // (the limits that earlier tile sizes set: what they refused stays refused)
-    const int per = (KL + 1 + KM + 1 + KN + 1) * (int)sizeof(double2) + (int)sizeof(double);
-    if (128 * (KM + 1 + KN + 1) * (int)sizeof(double2) > 200 * 1024 ||
-        std::max(8, std::min(64, (96 * 1024) / per)) * per > 200 * 1024)
+    if (!tables_fit(KDims{KL, KM, KN, ks.pipix, ks.pipiy, ks.pipiz}))
         return set_err(&c, MDG_E_UNSUPPORTED, "kmax too large for the shared-memory phase tables");
     return MDG_OK;
 }
@@ -507,7 +512,7 @@ void recip_fp64(Ctx& c) {
     const KGrid g = k_grid(d, v.nmove, ks.nrow, ks.nwork);
     cudaMemsetAsync(ks.s, 0, sizeof(double2) * ks.nk, c.stream);
     k_sfac<<<g.sfac, kSfacNT, g.smem_sfac, c.stream>>>(v, d, ks.nrow, ks.row, ks.witem_row, ks.witem_n, ks.nwork,
-                                                       g.atoms_per_split, ks.s, ks.nk);
+                                                       g.tile, g.atoms_per_split, ks.s, ks.nk);
     k_kenergy<<<std::min((ks.nrow + 7) / 8, 256), 256, 0, c.stream>>>(v, ks.nrow, ks.row, ks.row_nlen, ks.ent, ks.ak,
                                                                      ks.s, ks.qw, ks.c4);
     k_kforce<<<g.force, kForceNT, g.smem_force, c.stream>>>(v, d, ks.nrow, ks.row, ks.row_nlen, ks.ent, ks.c4);
@@ -651,10 +656,8 @@ int recip_forces_noalloc(const double* x, const double* y, const double* z, cons
         kmmin = -KM;
     }
     if (nk == 0) return na_fail(MDG_E_ARG, "mdg_recip_forces_noalloc: empty k set");
-    const int per = (KL + 1 + KM + 1 + KN + 1) * (int)sizeof(double2) + (int)sizeof(double);
-    const int smem1 = std::max(8, std::min(64, (96 * 1024) / per)) * per;
-    const int smem2 = 128 * (KM + 1 + KN + 1) * (int)sizeof(double2);
-    if (smem1 > 200 * 1024 || smem2 > 200 * 1024)
+    const KDims d{KL, KM, KN, pipix, pipiy, pipiz};
+    if (!tables_fit(d))
         return na_fail(MDG_E_UNSUPPORTED, "mdg_recip_forces_noalloc: kmax too large for the phase tables");
     if (sfac_items(g_na_rows, g_na_nlen, nrow, g_na_ent, g_na_wr, g_na_wn, nwork) > kNaMaxEnt)
         return na_fail(MDG_E_UNSUPPORTED, "mdg_recip_forces_noalloc: too many k rows");
@@ -698,9 +701,8 @@ int recip_forces_noalloc(const double* x, const double* y, const double* z, cons
     v.fz = fz;
     v.acc = acc;
     v.status = status;
-    KDims d{KL, KM, KN, pipix, pipiy, pipiz};
     const KGrid g = k_grid(d, (int)n, nrow, nwork);
-    k_sfac<<<g.sfac, kSfacNT, g.smem_sfac, st>>>(v, d, nrow, rows, wr, wn, nwork, g.atoms_per_split, S, nk);
+    k_sfac<<<g.sfac, kSfacNT, g.smem_sfac, st>>>(v, d, nrow, rows, wr, wn, nwork, g.tile, g.atoms_per_split, S, nk);
     k_kenergy<<<std::min((nrow + 7) / 8, 256), 256, 0, st>>>(v, nrow, rows, nlen, ent, Ak, S, nullptr, C);
     k_kforce<<<g.force, kForceNT, g.smem_force, st>>>(v, d, nrow, rows, nlen, ent, C);
     k_noalloc_energy<<<1, 32, 0, st>>>(acc, uewa);
