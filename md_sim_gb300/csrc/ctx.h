@@ -364,7 +364,7 @@ void wall_forces_fp64(Ctx& c);
 void surf_partition(Ctx& c);
 void lr_tail(Ctx& c);
 // pair_mx.cu
-void pack_setup(Ctx& c);
+int pack_setup(Ctx& c);
 // per-evaluation records of the real-space loops and the reciprocal sum; clears the FP64 forces
 // and sums the slab dipole M_z
 // reset_status: also clear the list overflow words; the energy sums are always cleared.

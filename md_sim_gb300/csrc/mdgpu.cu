@@ -622,7 +622,8 @@ int mdg_create(const mdg_sysdesc* s, const mdg_params* p, const double* x0, cons
     if (c.precision == MDG_MIXED) {
         rc = recip_tc_setup(c);
         if (rc) return bail(rc);
-        pack_setup(c);
+        rc = pack_setup(c);
+        if (rc) return bail(rc);
         if (c.nu.ready) {
             const NuView& g = c.nu.g;
             c.pk.nu_cnt = g.cnt;

@@ -407,6 +407,11 @@ int pair_setup(Ctx& c) {
     MDG_CUDA(cudaGetSymbolAddress(&p, g_etab));
     MDG_CUDA(cudaMemcpy(p, table.data(), sizeof(double) * table.size(), cudaMemcpyHostToDevice));
     c.v.etab = static_cast<const double2*>(p);
+    // the energy sums share a block's 48 KB with the queues (7 KB); a kernel takes more only where allowed
+    if (sizeof(double) * (2 * c.v.nijt + 6) > 32 * 1024) {
+        MDG_CUDA(allow_max_smem(k_pair_fp64));
+        MDG_CUDA(allow_max_smem(k_wall_fp64));
+    }
     return MDG_OK;
 }
 

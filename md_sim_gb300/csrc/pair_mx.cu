@@ -768,8 +768,19 @@ size_t table_smem(const View& v, int nextra) {
 
 }  // namespace
 
-void pack_setup(Ctx& c) {
+int pack_setup(Ctx& c) {
     const View& v = c.v;
+    // the type tables share a block's 48 KB with the queues (10 KB); a kernel takes more only where allowed
+    if (table_smem(v, 6) > 32 * 1024) {
+        MDG_CUDA(allow_max_smem(k_pair_mx<0>));
+        MDG_CUDA(allow_max_smem(k_pair_mx<1>));
+        MDG_CUDA(allow_max_smem(k_wall_mx<0>));
+        MDG_CUDA(allow_max_smem(k_wall_mx<1>));
+        MDG_CUDA(allow_max_smem(k_pair_mx_batch<0>));
+        MDG_CUDA(allow_max_smem(k_pair_mx_batch<1>));
+        MDG_CUDA(allow_max_smem(k_wall_mx_batch<0>));
+        MDG_CUDA(allow_max_smem(k_wall_mx_batch<1>));
+    }
     const int n = std::max(v.ntota, 1);
     c.pk.P = (uint4*)dalloc(c, sizeof(uint4) * n);
     c.pk.Q = (float4*)dalloc(c, sizeof(float4) * n);
@@ -784,6 +795,7 @@ void pack_setup(Ctx& c) {
     c.pk.spii = (float)v.spii;
     c.pk.facq = (float)v.facq;
     c.pk.rcutsq = (float)v.rcutsq;
+    return MDG_OK;
 }
 
 double slab_crf0(const Ctx& c) {
