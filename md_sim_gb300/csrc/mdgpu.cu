@@ -1077,7 +1077,8 @@ static int resident_alloc_impl(Ctx& c) {
         c.d_snap = nullptr;
         return set_err(&c, MDG_E_CUDA, "out of device memory for the integrator state");
     }
-    // the centres of mass of the force phases become the first Gear slice
+    // the centres of mass of the force phases become the first Gear slice (graphs captured before read the old ones)
+    drop_graphs(c);
     v.cx = c.d_c;
     v.cy = c.d_c + nr;
     v.cz = c.d_c + 2 * nr;
