@@ -174,8 +174,19 @@ int alloc_lists(Ctx& c, int maxnb, int maxwnb) {
     v.maxwnb = std::max(maxwnb, 8);
     v.nb = (int*)dalloc(c, sizeof(int) * (size_t)std::max(v.nheads, 1) * v.maxnb);
     v.wnb = (int*)dalloc(c, sizeof(int) * (size_t)std::max(v.nheads, 1) * (v.nwall > 0 ? v.maxwnb : 1));
-    if (!v.nb || !v.wnb) return set_err(&c, MDG_E_CUDA, "out of device memory for the neighbour lists");
-    return MDG_OK;
+    if (v.nb && v.wnb) return MDG_OK;
+    // empty lists: the next evaluation rebuilds them, finds no room and comes back here
+    dfree(c, v.nb);
+    dfree(c, v.wnb);
+    v.nb = v.wnb = nullptr;
+    v.maxnb = v.maxwnb = 0;
+    c.alloc_failed = false;
+    cudaGetLastError();
+    const int one = 1;
+    cudaMemset(v.nbcnt, 0, sizeof(int) * std::max(v.nheads, 1));
+    cudaMemset(v.wnbcnt, 0, sizeof(int) * std::max(v.nheads, 1));
+    cudaMemcpy(v.status + ST_FORCE_RB, &one, sizeof(int), cudaMemcpyHostToDevice);
+    return set_err(&c, MDG_E_CUDA, "out of device memory for the neighbour lists");
 }
 
 int sync_check(Ctx& c, const char* where) {
@@ -1336,9 +1347,9 @@ int mdg_run(mdg_ctx* cp, int64_t nsteps, mdg_report* rep) {
         const int ovf = c.h_status[ST_LIST_OVF], wovf = c.h_status[ST_WLIST_OVF];
         if (ovf || wovf) {
             if (++retries > 4) return set_err(&c, MDG_E_LIST_OVERFLOW, "nnlist_make(): nnlist too big!");
+            snapshot(c, true);
             rc = alloc_lists(c, ovf ? ovf + ovf / 4 + 32 : v.maxnb, wovf ? wovf + wovf / 4 + 32 : v.maxwnb);
             if (rc) return rc;
-            snapshot(c, true);
             const int one = 1;
             MDG_CUDA(cudaMemcpyAsync(v.status + ST_FORCE_RB, &one, sizeof(int), cudaMemcpyHostToDevice, c.stream));
             MDG_CUDA(cudaStreamSynchronize(c.stream));
@@ -1804,9 +1815,13 @@ int mdg_batch_run(mdg_batch* b, int64_t nsteps, mdg_report* reps) {
             if (rc) return batch_err(b, rc, "replica " + std::to_string(i) + ": " + c.err);
             const int ovf = c.h_status[ST_LIST_OVF], wovf = c.h_status[ST_WLIST_OVF];
             if (ovf || wovf) {
-                rc = alloc_lists(c, ovf ? ovf + ovf / 4 + 32 : c.v.maxnb, wovf ? wovf + wovf / 4 + 32 : c.v.maxwnb);
-                if (rc) return batch_err(b, rc, "replica " + std::to_string(i) + ": " + c.err);
                 snapshot(c, true);
+                rc = alloc_lists(c, ovf ? ovf + ovf / 4 + 32 : c.v.maxnb, wovf ? wovf + wovf / 4 + 32 : c.v.maxwnb);
+                if (rc) {
+                    if (b->exec) cudaGraphExecDestroy(b->exec);  // it holds the lists that are gone
+                    b->exec = nullptr;
+                    return batch_err(b, rc, "replica " + std::to_string(i) + ": " + c.err);
+                }
                 const int one = 1;
                 cudaMemcpyAsync(c.v.status + ST_FORCE_RB, &one, sizeof(int), cudaMemcpyHostToDevice, c.stream);
                 cudaStreamSynchronize(c.stream);

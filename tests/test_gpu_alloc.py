@@ -115,3 +115,32 @@ def test_resident_state(name, gpulib, monkeypatch):
         assert np.abs(ctx.sys.x0 - want).max() <= (1e-7 if name == "mixed" else 1e-11) * s.lx
         ctx.close()
     assert failed == 10  # the pinned thermostat values, eight arrays and the snapshot
+
+
+@pytest.mark.parametrize("precision", [abi.MDG_FP64, abi.MDG_MIXED])
+def test_list_growth(precision, gpulib, monkeypatch):
+    """A force call whose lists outgrow their room and find no memory: it says so, and the next call has them."""
+    s, prm = configs.ion_lattice(6, rcut=3.5, shuffle=True)
+    prm.precision, prm.list_capacity = precision, 1
+    near = s.copy()
+    for a in (near.x0, near.y0, near.z0):
+        a[:s.nmove] *= 0.4
+    ctx = abi.Context(gpulib, s.copy(), prm)
+    want = ctx.force_get(near.copy())["f"]
+    ctx.close()
+    failed = 0
+    for n in range(1, MOST):
+        monkeypatch.setenv("MDG_DEBUG_FAIL_ALLOC", str(n))
+        try:
+            ctx = abi.Context(gpulib, s.copy(), prm)
+        except abi.MdgError:
+            continue
+        try:
+            got = ctx.force_get(near.copy())
+        except abi.MdgError as e:
+            assert "out of device memory" in str(e)
+            failed += 1
+            got = ctx.force_get(near.copy())
+        assert np.linalg.norm(got["f"] - want) <= (1e-5 if precision else 1e-12) * np.linalg.norm(want)
+        ctx.close()
+    assert failed == 2
