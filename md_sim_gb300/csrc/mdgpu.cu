@@ -1131,6 +1131,7 @@ int mdg_set_state(mdg_ctx* cp, const mdg_rigid* b, const mdg_state* st) {
     MDG_CUDA(cudaStreamSynchronize(c.stream));
     int rc = resident_alloc_impl(c);
     if (rc) return rc;
+    if (std::memcmp(&c.body, b, sizeof(*b)) != 0) drop_graphs(c);  // a captured step holds it by value
     c.body = *b;
     const int nm = v.nmove, nr = v.nrig, nion = v.nliqa - v.nriga, nold = v.ntota - v.nliqa;
     MDG_CUDA(cudaMemcpy(v.x, st->x0, sizeof(double) * nm, cudaMemcpyHostToDevice));
