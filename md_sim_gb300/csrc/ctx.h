@@ -316,6 +316,7 @@ struct Ctx {
     cudaGraphExec_t graph_exec = nullptr;   // resident step
     cudaGraphExec_t force_exec = nullptr;   // force evaluation of the drop-in path
     int graph_steps = 0;
+    uint64_t graph_gen = 0;                 // times they were dropped: a batch's graph holds the same arguments
     int64_t kernels_per_step = 0;
     // host staging (pinned)
     double* h_acc = nullptr;
@@ -498,6 +499,7 @@ inline void drop_graphs(Ctx& c) {
     if (c.force_exec) cudaGraphExecDestroy(c.force_exec);
     c.graph_exec = nullptr;
     c.force_exec = nullptr;
+    ++c.graph_gen;
 }
 }  // namespace mdg
 

@@ -1544,6 +1544,7 @@ struct mdg_batch {
     int mode = MDG_BATCH_PHASES;
     int phased = 0;                     // replicas in the batched loops (last graph build)
     cudaGraphExec_t exec = nullptr;
+    uint64_t gen = 0;                   // sum of the contexts' graph_gen when exec was built
     int device = 0;
     std::string err;
 };
@@ -1686,10 +1687,15 @@ static int batch_plans(mdg_batch* b, bool on) {
     return MDG_OK;
 }
 
-static int batch_graph(mdg_batch* b) {
-    if (b->exec) return MDG_OK;
-    const int prc = batch_plans(b, true);
-    if (prc) return prc;
+// The contexts' graph generations: they grow whenever an argument that the batch's graph holds by value changes
+// (grown lists, another thermostat, measurement switches).
+static uint64_t batch_gen(const mdg_batch* b) {
+    uint64_t g = 0;
+    for (const mdg_ctx* c : b->ctx) g += c->graph_gen;
+    return g;
+}
+
+static int batch_build(mdg_batch* b) {
     if (b->mode == MDG_BATCH_PHASES) return batch_graph_phases(b);
     b->phased = 0;
     cudaGraph_t g;
@@ -1714,6 +1720,20 @@ static int batch_graph(mdg_batch* b) {
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return batch_err(b, MDG_E_CUDA, std::string("batch instantiate: ") + cudaGetErrorString(e));
     return MDG_OK;
+}
+
+// The batch's graph, built again when an argument changed since.
+static int batch_graph(mdg_batch* b) {
+    if (b->exec && b->gen == batch_gen(b)) return MDG_OK;
+    if (b->exec) {
+        cudaStreamSynchronize(b->stream);  // its kernels read the descriptors that the next one overwrites
+        cudaGraphExecDestroy(b->exec);
+        b->exec = nullptr;
+    }
+    int rc = batch_plans(b, true);
+    if (!rc) rc = batch_build(b);
+    b->gen = batch_gen(b);
+    return rc;
 }
 
 int mdg_batch_create(mdg_ctx* const* ctxs, int n, mdg_batch** out) {
@@ -1807,7 +1827,6 @@ int mdg_batch_run(mdg_batch* b, int64_t nsteps, mdg_report* reps) {
         int rc = mdg_batch_run_async(b, chunk);
         if (rc) return rc;
         if (cudaStreamSynchronize(b->stream) != cudaSuccess) return batch_err(b, MDG_E_CUDA, "batch step failed");
-        bool rebuild = false;
         for (auto* cp : b->ctx)
             if ((rc = queue_status(*cp))) return batch_err(b, rc, cp->err);
         for (size_t i = 0; i < b->ctx.size(); ++i) {
@@ -1818,27 +1837,18 @@ int mdg_batch_run(mdg_batch* b, int64_t nsteps, mdg_report* reps) {
             if (ovf || wovf) {
                 snapshot(c, true);
                 rc = alloc_lists(c, ovf ? ovf + ovf / 4 + 32 : c.v.maxnb, wovf ? wovf + wovf / 4 + 32 : c.v.maxwnb);
-                if (rc) {
-                    if (b->exec) cudaGraphExecDestroy(b->exec);  // it holds the lists that are gone
-                    b->exec = nullptr;
-                    return batch_err(b, rc, "replica " + std::to_string(i) + ": " + c.err);
-                }
+                if (rc) return batch_err(b, rc, "replica " + std::to_string(i) + ": " + c.err);
                 const int one = 1;
                 cudaMemcpyAsync(c.v.status + ST_FORCE_RB, &one, sizeof(int), cudaMemcpyHostToDevice, c.stream);
                 cudaStreamSynchronize(c.stream);
                 rc = mdg_run(b->ctx[i], chunk, nullptr);
                 if (rc) return batch_err(b, rc, "replica " + std::to_string(i) + ": " + c.err);
-                rebuild = true;
                 continue;
             }
             if (c.h_status[ST_SHAKE_RPTOL])
                 return batch_err(b, MDG_E_SHAKE_RPTOL, "replica " + std::to_string(i) + ": Constraint failure");
             if (c.h_status[ST_SHAKE_MAXIT])
                 return batch_err(b, MDG_E_SHAKE_MAXIT, "replica " + std::to_string(i) + ": shake(): Too many constraint iterations!");
-        }
-        if (rebuild && b->exec) {
-            cudaGraphExecDestroy(b->exec);
-            b->exec = nullptr;
         }
         done += chunk;
     }
