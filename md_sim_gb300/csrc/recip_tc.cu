@@ -513,7 +513,8 @@ __global__ void k_tc_prep_c(const float2* __restrict__ Cf, const int4* __restric
                 // each row's C scaled by its own max |n C|: under one scale for all rows the
                 // large-k rows' C would fall below FP16's normal range
                 const float sr = rowsc[rorig[row]];
-                const float inv = sr > 0.f ? 1.0f / sr : 1.0f;
+                // (where the reciprocal of the maximum could overflow the row stays as it is, zero in FP16)
+                const float inv = sr > 1e-37f ? 1.0f / sr : 1.0f;
                 const float2 cv = Cf[rw.w + n - rw.z];
                 const float sc = (tt ? (float)n : 1.0f) * inv;
                 const float cr = cv.x * sc, ci = cv.y * sc;
