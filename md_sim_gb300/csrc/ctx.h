@@ -413,6 +413,7 @@ int recip_tc_throughput(Ctx& c, bool on);
 void recip_tc(Ctx& c);  // (or the gridded sum, by the size of the system)
 // recip_nu.cu
 int recip_nu_setup(Ctx& c);
+int recip_nu_points(int K);  // grid points of an edge with frequencies up to K
 int recip_nu64_setup(Ctx& c);
 void recip_nu64(Ctx& c);
 void recip_nu(Ctx& c);

@@ -392,12 +392,12 @@ struct WindowTable {
 
 }  // namespace
 
+int recip_nu_points(int K) { return std::max(16, 4 * K + 8); }  // 2.1 to 2.5 (2K + 1), a multiple of 4
+
 int recip_nu_setup(Ctx& c) {
     if (c.ks.nk == 0 || c.v.nmove == 0) return MDG_OK;
     static const WindowTable spread(kBetaSpread), force(kBetaForce);
-    return nu_setup<float>(
-        c, c.nu, [](int K) { return std::max(16, 4 * K + 8); },  // 2.1 to 2.5 (2K + 1), a multiple of 4
-        [](int h, int k, int M) { return (h ? force : spread).inverse(k, M); });
+    return nu_setup<float>(c, c.nu, recip_nu_points, [](int h, int k, int M) { return (h ? force : spread).inverse(k, M); });
 }
 
 void recip_nu(Ctx& c) {

@@ -963,7 +963,15 @@ int recip_tc_throughput(Ctx& c, bool on) {
 // GPU, tensor cores against grid: 17,496 atoms x 5,876 k (1.0e8) 98.9 and 93.6 us, 9,000 x 7,404
 // with walls (6.7e7) 116.7 and 99.0, 14,739 x 4,717 (7.0e7) 89.0 and 98.6, 12,288 x 3,720 (4.6e7)
 // 80.7 and 81.0, 6,144 x 4,338 (2.7e7) 84.8 and 89.2; 98,304 x 29,038 (2.9e9) 462 and 240.
-constexpr double kGridWork = 8e7;
+// The grid's Fourier sums grow with its points, about 30 per k vector: where a few atoms have very many k vectors
+// the products are the cheaper part.  Force calls at 262 points per atom (6,591 x 46,174) 110 and 119 us, at 103
+// (6,591 x 16,916) 82 and 85, at 21 (14,739 x 7,181) 90 and 89.
+constexpr double kGridWork = 8e7, kGridPoints = 150.0;
+static bool grid_pays(const Ctx& c) {
+    double points = 1.0;
+    for (int K : {c.ks.klmax, c.ks.kmmax, c.ks.knmax}) points *= recip_nu_points(K);
+    return (double)c.v.nmove * c.ks.nk >= kGridWork && points <= kGridPoints * c.v.nmove;
+}
 
 int recip_tc_setup(Ctx& c) {
     View& v = c.v;
@@ -989,7 +997,7 @@ int recip_tc_setup(Ctx& c) {
     c.d_tc_atoms = (uint4*)dalloc(c, sizeof(uint4) * std::max(v.nmove, 1));
     c.d_frc = (double*)dalloc(c, sizeof(double) * 3 * std::max(v.nmove, 1));
     if (c.alloc_failed) return set_err(&c, MDG_E_CUDA, "out of device memory for the tensor-core reciprocal sum");
-    if (2 * p.NN > 128 || (double)v.nmove * ks.nk >= kGridWork) return recip_nu_setup(c);
+    if (2 * p.NN > 128 || grid_pays(c)) return recip_nu_setup(c);
     tc_plan_pass1(c, 2);
     // the partial-sum buffer is sized for the largest split the autotuner may choose
     size_t part_max = 0;
