@@ -392,7 +392,12 @@ int nu_setup(Ctx& c, NuPlanT<T>& plan, Rule rule, Inverse inverse) {
     const double want = 3.0 * std::max((double)v.nmove / (double)nblk, 0.11 * cell) + 16.0;
     g.cap = (int)std::min<double>(want, v.nmove);
     g.nblk = (int)nblk;
-    g.split = std::max(1, std::min(64, std::max((int)(v.nmove / nblk / kSplit) + 1, (int)(912 / nblk))));
+    // CTAs per block: for kSplit atoms each, for 912 in all, and where most of the box is empty for 340 over the blocks
+    // that a liquid would fill (with no more than 4,096 in all, most of which have nothing to do).  Slabs of 4,000 and 1,400 waters in boxes 4.5 and 9 edges tall (mixed, a force call):
+    // by the box's mean density 118 and 83 us, this 98 and 81 (912 over the filled blocks 104 and 97).
+    const double dense = std::max((double)v.nmove / (double)nblk, 0.1 * cell), full = std::max(v.nmove / dense, 1.0);
+    g.split = std::max({(int)(dense / kSplit) + 1, (int)(912 / nblk), std::min((int)(340.0 / full), (int)(4096 / nblk))});
+    g.split = std::min(g.split, 64);
     const int nm = 2 * K[1] + 1, nl = 2 * K[0] + 1;
     std::vector<int> kmap((size_t)(K[2] + 1) * nm * nl, -1);
     for (int r = 0; r < ks.nrow; ++r)
