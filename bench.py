@@ -208,12 +208,20 @@ def fp32_nominal_tflops():
     return 152 * 128 * 2 * mhz * 1e6 / 1e12
 
 
-def gridded(s, nk, precision):
-    """Whether the library takes the gridded reciprocal sum: atoms times k vectors from its lines on
-    (kGridWork in recip_tc.cu, kGridWork64 in recip_nu64.cu)."""
+def gridded(s, prm, nk, precision):
+    """Whether the library takes the gridded reciprocal sum: atoms times k vectors from its lines on; in the
+    mixed form not with more than 150 grid points per atom, and always with 2 (2 knmax + 1) > 128
+    (recip_tc_setup in recip_tc.cu, recip_nu64_setup in recip_nu64.cu)."""
     from md_sim_gb300.abi import MDG_MIXED
 
-    return s.nmove * nk >= (8.0e7 if precision == MDG_MIXED else 5.0e6)
+    if precision != MDG_MIXED:
+        return s.nmove * nk >= 5.0e6
+    lmin = min(s.lx, s.ly, s.lz)
+    K = [round(prm.kmax * x / lmin) for x in (s.lx, s.ly, s.lz)]
+    points = 1.0
+    for k in K:
+        points *= max(16, 4 * k + 8)
+    return 2 * (2 * K[2] + 1) > 128 or (s.nmove * nk >= 8.0e7 and points <= 150.0 * s.nmove)
 
 
 def grid_flops(s, prm, mixed):
@@ -251,7 +259,7 @@ def roofline(ctx, s, prm, precision, pk, config_name="", fp64_peak=None):
         t = ph[kind] * 1e-3
         if kind == "reciprocal":
             units = s.nmove * nk
-            if gridded(s, nk, precision):
+            if gridded(s, prm, nk, precision):
                 flops = grid_flops(s, prm, mixed)
                 if mixed:
                     bound, peak, src = "fp32", fp32_nominal_tflops(), "nominal FP32 (152 SM x 128 lanes x 2 x max clock)"
@@ -525,7 +533,7 @@ def learned_arm(lib, ctx, s_start, args, K, stream, flush, torch, value, t_step)
 
 def widom_arm(ctx, s, args):
     """Widom insertions (chempot) on the context's last force evaluation: wall time per call on the
-    GPU (host clock around mdg_widom: generator on the host, one kernel, results back)."""
+    GPU (host clock around mdg_widom: generator on the host beside the device's kernels, results back)."""
     from md_sim_gb300 import abi
 
     seed0 = 14135621772.0
@@ -566,7 +574,7 @@ def run_workload(lib, name, args, torch, stream, flush, pk, fp64_peak, headline=
     kps = ctx.kernels_per_step()
     ctx.get_state(s)
     roof, roof_recip, roof_pairs = roofline(ctx, s, prm, precision, pk, name, fp64_peak)
-    on_grid = gridded(s, len(ctx.kvectors()[0]), precision)
+    on_grid = gridded(s, prm, len(ctx.kvectors()[0]), precision)
     learned_rep, shake_model = None, None
     if s.ncons > 0 and args.learned and precision == MDG_MIXED:
         learned_rep, per_seed, shake_model = learned_arm(lib, ctx, s_start, args, K, stream, flush, torch, value,

@@ -323,9 +323,9 @@ int mdg_phase_times(mdg_ctx* ctx, int reps, double* ms);
  * tiles per CTA and atom splits) and keeps the fastest.  reps evaluations per candidate.
  * ------------------------------------------------------------------------------------------- */
 typedef struct mdg_tuning {
-    int32_t pair_blocks;      /* real-space blocks (0: one warp per head) */
-    int32_t tc_rows_per_cta;  /* structure-factor (l, m) rows per CTA (mixed precision) */
-    int32_t tc_atom_splits;   /* structure-factor atom chunks */
+    int32_t pair_blocks;      /* real-space blocks (0: one warp per head, one block per SM beside walls, else two) */
+    int32_t tc_rows_per_cta;  /* tensor-core structure factor: (l, m) rows per CTA (256 also where it does not run) */
+    int32_t tc_atom_splits;   /* its atom chunks (1 where the gridded or the FP64 sum runs) */
     float ms_before, ms_after;
 } mdg_tuning;
 int mdg_autotune(mdg_ctx* ctx, int32_t reps, mdg_tuning* out);

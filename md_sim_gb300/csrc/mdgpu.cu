@@ -1911,7 +1911,7 @@ int mdg_autotune(mdg_ctx* cp, int32_t reps, mdg_tuning* out) {
     cudaSetDevice(c.device);
     reps = std::max(reps, 1);
     const float t0 = time_force(c, reps);
-    // real-space grid (blocks of 8 warps; 0 = one warp per head up to 16 blocks per SM)
+    // real-space grid (blocks of 8 warps; 0: one warp per head in at most 152 blocks beside walls, 304 otherwise)
     int best_pb = c.pair_blocks;
     float best = t0;
     for (int pb : {0, 152 * 2, 152 * 4, 152 * 8}) {
@@ -1948,8 +1948,8 @@ int mdg_autotune(mdg_ctx* cp, int32_t reps, mdg_tuning* out) {
     if (rc) return rc;
     if (out) {
         out->pair_blocks = best_pb;
-        out->tc_rows_per_cta = 256;
-        out->tc_atom_splits = std::max(c.tcp.nsplit1, 1);  // 1: the gridded sum has no such split
+        out->tc_rows_per_cta = 256;  // (both are the tensor-core sum's; the gridded sum has neither)
+        out->tc_atom_splits = std::max(c.tcp.nsplit1, 1);
         out->ms_before = t0;
         out->ms_after = t1;
     }

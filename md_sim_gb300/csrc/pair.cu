@@ -391,7 +391,9 @@ __global__ void __launch_bounds__(kLrNT) k_lr_tail(View v, const double* lr) { l
 
 // Parts of a head's list: enough warps for every SM where heads are few; more parts leave queues that
 // end less than half full.  1, 2, 3, 4, 8 parts: 256 heads 50, 34, 38, 27, 41 us; 2,048 heads 146, 123,
-// 135, 138, 146 us (walls 77, 70, 78, 73, 80); one part is enough from 152 * 27 heads on.
+// 135, 138, 146 us (walls 77, 70, 78, 73, 80).  One part from 2,049 heads on: with 1 and 2 parts 2,197 bulk heads
+// 170 and 154 us but whole force calls, beside the reciprocal sum, 458 and 463; 2,744 heads 207 and 180, calls 524
+// and 532; slabs of 2,600 heads 141 and 155, calls 536 and 555, of 6,000 heads 300 and 330, calls 1,081 and 1,125.
 int list_parts(int nheads) { return std::max(1, std::min(4, 4096 / nheads)); }
 int pair_blocks(int units) { return std::max(1, std::min((units + kWarps - 1) / kWarps, 152 * 64)); }
 

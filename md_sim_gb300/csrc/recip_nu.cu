@@ -28,8 +28,8 @@
 // multiply-adds of the plain complex sums: 95 M FMAs forward and back at M = 104.
 //
 // 98,304 atoms, 29,038 k vectors (M = 104): spread 32 us, zy 12, x 13, yz 11, force 30 = 98 us where the
-// tensor-core passes take 310 (143 + 11 + 5 + 156); resident step 0.496 -> 0.276 ms, forces of the
-// whole evaluation 6.2e-7 off FP64 (tensor cores 1.1e-6), reciprocal energy 2e-7 (1.9e-6).  Spread and
+// tensor-core passes take 310 (143 + 11 + 5 + 156); forces of the whole evaluation 6.2e-7 off FP64 (tensor
+// cores 1.1e-6), reciprocal energy 2e-7 (1.9e-6).  Spread and
 // force are bound by shared-memory wavefronts (79 and 82 % of the L1 pipe), the Fourier sums by them
 // and by the few CTAs.
 #include <algorithm>

@@ -959,7 +959,8 @@ int recip_tc_throughput(Ctx& c, bool on) {
     return MDG_OK;
 }
 
-// (atom, k) products from which the gridded sum (recip_nu.cu) is taken.  Resident step, alone on the
+// (atom, k) products from which the gridded sum (recip_nu.cu) is taken (it also takes every set of k vectors with
+// 2 (2 KN + 1) > 128, which the passes here do not hold).  Resident step, alone on the
 // GPU, tensor cores against grid: 17,496 atoms x 5,876 k (1.0e8) 98.9 and 93.6 us, 9,000 x 7,404
 // with walls (6.7e7) 116.7 and 99.0, 14,739 x 4,717 (7.0e7) 89.0 and 98.6, 12,288 x 3,720 (4.6e7)
 // 80.7 and 81.0, 6,144 x 4,338 (2.7e7) 84.8 and 89.2; 98,304 x 29,038 (2.9e9) 462 and 240.
